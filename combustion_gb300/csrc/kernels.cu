@@ -10,6 +10,7 @@
 #include "device_common.cuh"
 #include "device_math.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "rates_core.cuh"
 #include "tables.h"
 
@@ -530,52 +531,6 @@ __global__ void __launch_bounds__(32 * kWarpCellWarps) transport_warp_kernel(con
 }
 
 // ---------------------------------------------------------------------------------------------------
-namespace {
-int sm_count() {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 1;
-    }
-    return sms;
-}
-
-template <class Args>
-bool gathered(const Args&) { return false; }
-template <int KMAX>
-bool gathered(const TransportArgs<KMAX>& io) { return io.index != nullptr; }
-
-// Persistent grid: as many blocks as fit on the GPU at once (each stages the tables once), never more
-// than the cells need. Tables go to shared memory when they fit, else they are read through L1/L2.
-template <int BLOCK, class Args, class KS, class KG>
-cudaError_t launch_table_kernel(KS ksmem, KG kglobal, const uint8_t* tab, uint32_t tab_bytes, const Args& io,
-                                size_t n, cudaStream_t st, int* status) {
-    const bool smem = (int)tab_bytes <= max_table_smem();
-    // Gathered cells are few (a trust gate's fallback or audit): one warp per block spreads them over
-    // every SM instead of filling a few blocks.
-    const int block = gathered(io) ? 32 : BLOCK;
-    int per_sm = 1;
-    const size_t want = (n + block - 1) / block;
-    cudaError_t e = table_kernel_occupancy(ksmem, kglobal, block, tab_bytes, kMathBytes, smem, &per_sm);
-    if (e != cudaSuccess) return e;
-    size_t grid = (size_t)sm_count() * per_sm;
-    if (want < grid) grid = want ? want : 1;
-    if (smem) ksmem<<<(unsigned)grid, block, tab_bytes, st>>>(tab, tab_bytes, io, n, status);
-    else kglobal<<<(unsigned)grid, block, kMathBytes, st>>>(tab, tab_bytes, io, n, status);
-    return cudaGetLastError();
-}
-template <int BLOCK, class KS, class KG>
-size_t wave_of(KS ksmem, KG kglobal, uint32_t tab_bytes) {
-    int per_sm = 1;
-    if (table_kernel_occupancy(ksmem, kglobal, BLOCK, tab_bytes, kMathBytes, (int)tab_bytes <= max_table_smem(),
-                               &per_sm) != cudaSuccess)
-        return 0;
-    return (size_t)sm_count() * per_sm * BLOCK;
-}
-}  // namespace
-
 // Non-finite values by exponent bits (all ones): integer instructions only.
 __global__ void count_nonfinite_kernel(const __grid_constant__ CountArgs args, size_t n, unsigned long long* count) {
     unsigned long long c = 0;
@@ -631,36 +586,12 @@ int max_table_smem() {
     return v;
 }
 
-#define CB_DISPATCH(FN, KERNEL, ARGS, BLOCK)                                                               \
-    cudaError_t FN(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,            \
-                   cudaStream_t st, int* status) {                                                         \
-        switch (kmax) {                                                                                    \
-        case 16: return launch_table_kernel<BLOCK>(KERNEL<16, true>, KERNEL<16, false>, tab, tab_bytes,    \
-                                                   *static_cast<const ARGS<16>*>(args), n, st, status);    \
-        case 64: return launch_table_kernel<BLOCK>(KERNEL<64, true>, KERNEL<64, false>, tab, tab_bytes,    \
-                                                   *static_cast<const ARGS<64>*>(args), n, st, status);    \
-        case 256: return launch_table_kernel<BLOCK>(KERNEL<256, true>, KERNEL<256, false>, tab, tab_bytes, \
-                                                    *static_cast<const ARGS<256>*>(args), n, st, status);  \
-        default: return cudaErrorInvalidValue;                                                             \
-        }                                                                                                  \
-    }
-CB_DISPATCH(launch_rates, rates_kernel, RatesArgs, kBlock)
-CB_DISPATCH(launch_reaction_rates, reaction_rates_kernel, ReactionRatesArgs, kBlock)
-#undef CB_DISPATCH
+CB_DISPATCH(launch_rates, rates_kernel, RatesArgs, kBlock, kMathBytes, true)
+CB_DISPATCH(launch_reaction_rates, reaction_rates_kernel, ReactionRatesArgs, kBlock, kMathBytes, true)
 
-#define CB_WAVE(FN, KERNEL, BLOCK)                                                     \
-    size_t FN(int kmax, uint32_t tab_bytes) {                                          \
-        switch (kmax) {                                                                \
-        case 16: return wave_of<BLOCK>(KERNEL<16, true>, KERNEL<16, false>, tab_bytes);    \
-        case 64: return wave_of<BLOCK>(KERNEL<64, true>, KERNEL<64, false>, tab_bytes);    \
-        case 256: return wave_of<BLOCK>(KERNEL<256, true>, KERNEL<256, false>, tab_bytes); \
-        default: return 0;                                                             \
-        }                                                                              \
-    }
-CB_WAVE(wave_rates, rates_kernel, kBlock)
-CB_WAVE(wave_reaction_rates, reaction_rates_kernel, kBlock)
-CB_WAVE(wave_transport, transport_kernel, kTransportBlock)
-#undef CB_WAVE
+CB_WAVE(wave_rates, rates_kernel, kBlock, kMathBytes)
+CB_WAVE(wave_reaction_rates, reaction_rates_kernel, kBlock, kMathBytes)
+CB_WAVE(wave_transport, transport_kernel, kTransportBlock, kMathBytes)
 
 namespace {
 // Gathered launches of up to this many cells per SM go warp-per-cell (above 16 species): one cell per
@@ -690,7 +621,7 @@ cudaError_t launch_transport_k(const uint8_t* tab, uint32_t tab_bytes, const Tra
         }
     }
     return launch_table_kernel<kTransportBlock>(transport_kernel<KMAX, true>, transport_kernel<KMAX, false>, tab,
-                                                tab_bytes, io, n, st, status);
+                                                tab_bytes, io, n, kMathBytes, true, st, status);
 }
 }  // namespace
 

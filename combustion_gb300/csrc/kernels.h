@@ -89,6 +89,15 @@ cudaError_t table_kernel_occupancy(KS ksmem, KG kglobal, int block, uint32_t tab
     return cudaSuccess;
 }
 
+// Shared memory (of an SM's 256 KB, shared with L1) for `per_sm` resident blocks of a table kernel, whatever
+// block size a launch takes.
+template <class K>
+cudaError_t set_carveout(K kernel, int per_sm, uint32_t bytes) {
+    const int most = max_table_smem() + 1024, want = per_sm * (int)(bytes + 2048);
+    const int percent = want >= most ? 100 : (int)((100ll * want + most - 1) / most);
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+}
+
 // Cells one wave of a kernel's persistent grid covers (its threads resident on the whole GPU): every
 // thread of a launch over a multiple of it gets the same number of cells. Host arrays go through the
 // GPU in chunks of whole waves.

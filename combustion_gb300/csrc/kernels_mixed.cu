@@ -13,6 +13,7 @@
 #include "device_common.cuh"
 #include "device_math.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "rates_mixed_core.cuh"
 #include "tables_mixed.h"
 
@@ -273,79 +274,9 @@ __global__ void __launch_bounds__(kTransportMixedBlock) transport_mixed_kernel(c
 }
 
 // ---------------------------------------------------------------------------------------------------
-namespace {
-int sm_count_m() {
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 1;
-}
-
-template <int BLOCK, class KS, class KG>
-size_t wave_of_m(KS ksmem, KG kglobal, uint32_t tab_bytes) {
-    int per_sm = 1;
-    if (table_kernel_occupancy(ksmem, kglobal, BLOCK, tab_bytes, kMathBytes, (int)tab_bytes <= max_table_smem(),
-                               &per_sm) != cudaSuccess)
-        return 0;
-    return (size_t)sm_count_m() * per_sm * BLOCK;
-}
-
-template <class Args>
-bool gathered_m(const Args&) { return false; }
-template <int KMAX>
-bool gathered_m(const TransportArgs<KMAX>& io) { return io.index != nullptr; }
-
-template <int BLOCK, class Args, class KS, class KG>
-cudaError_t launch_mixed(KS ksmem, KG kglobal, const uint8_t* tab, uint32_t tab_bytes, const Args& io, size_t n,
-                         cudaStream_t st, int* status) {
-    const bool smem = (int)tab_bytes <= max_table_smem();
-    // A gathered launch of fewer cells than one wave of full blocks (a trust gate's fallback) spreads
-    // them over every SM in one-warp blocks.
-    int block = BLOCK, per_sm = 1;
-    cudaError_t e = table_kernel_occupancy(ksmem, kglobal, BLOCK, tab_bytes, kMathBytes, smem, &per_sm);
-    if (e != cudaSuccess) return e;
-    if (gathered_m(io) && n < (size_t)sm_count_m() * per_sm * BLOCK) {
-        block = 32;
-        e = table_kernel_occupancy(ksmem, kglobal, block, tab_bytes, kMathBytes, smem, &per_sm);
-        if (e != cudaSuccess) return e;
-    }
-    const size_t want = (n + block - 1) / block;
-    size_t grid = (size_t)sm_count_m() * per_sm;
-    if (want < grid) grid = want ? want : 1;
-    if (smem) ksmem<<<(unsigned)grid, block, tab_bytes, st>>>(tab, tab_bytes, io, n, status);
-    else kglobal<<<(unsigned)grid, block, kMathBytes, st>>>(tab, tab_bytes, io, n, status);
-    return cudaGetLastError();
-}
-}  // namespace
-
-#define CB_DISPATCH_M(FN, KERNEL, ARGS, BLOCK)                                                             \
-    cudaError_t FN(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,            \
-                   cudaStream_t st, int* status) {                                                         \
-        switch (kmax) {                                                                                    \
-        case 16: return launch_mixed<BLOCK>(KERNEL<16, true>, KERNEL<16, false>, tab, tab_bytes,           \
-                                            *static_cast<const ARGS<16>*>(args), n, st, status);           \
-        case 64: return launch_mixed<BLOCK>(KERNEL<64, true>, KERNEL<64, false>, tab, tab_bytes,           \
-                                            *static_cast<const ARGS<64>*>(args), n, st, status);           \
-        case 256: return launch_mixed<BLOCK>(KERNEL<256, true>, KERNEL<256, false>, tab, tab_bytes,        \
-                                             *static_cast<const ARGS<256>*>(args), n, st, status);         \
-        default: return cudaErrorInvalidValue;                                                             \
-        }                                                                                                  \
-    }
-CB_DISPATCH_M(launch_rates_mixed, rates_mixed_kernel, RatesArgs, kBlock)
-CB_DISPATCH_M(launch_transport_mixed, transport_mixed_kernel, TransportArgs, kTransportMixedBlock)
-#undef CB_DISPATCH_M
-
-#define CB_WAVE_M(FN, KERNEL, BLOCK)                                                        \
-    size_t FN(int kmax, uint32_t tab_bytes) {                                               \
-        switch (kmax) {                                                                     \
-        case 16: return wave_of_m<BLOCK>(KERNEL<16, true>, KERNEL<16, false>, tab_bytes);    \
-        case 64: return wave_of_m<BLOCK>(KERNEL<64, true>, KERNEL<64, false>, tab_bytes);    \
-        case 256: return wave_of_m<BLOCK>(KERNEL<256, true>, KERNEL<256, false>, tab_bytes); \
-        default: return 0;                                                                  \
-        }                                                                                   \
-    }
-CB_WAVE_M(wave_rates_mixed, rates_mixed_kernel, kBlock)
-CB_WAVE_M(wave_transport_mixed, transport_mixed_kernel, kTransportMixedBlock)
-#undef CB_WAVE_M
+CB_DISPATCH(launch_rates_mixed, rates_mixed_kernel, RatesArgs, kBlock, kMathBytes, false)
+CB_DISPATCH(launch_transport_mixed, transport_mixed_kernel, TransportArgs, kTransportMixedBlock, kMathBytes, false)
+CB_WAVE(wave_rates_mixed, rates_mixed_kernel, kBlock, kMathBytes)
+CB_WAVE(wave_transport_mixed, transport_mixed_kernel, kTransportMixedBlock, kMathBytes)
 
 }  // namespace cbg
