@@ -20,6 +20,7 @@ struct cb_mech {
     int device = 0;
     int kmax = 0;
     uint8_t* d_rates = nullptr;      // rates table blob
+    uint8_t* d_rates_fixed = nullptr;  // the same in fixed point (null: the mechanism is out of its range)
     uint8_t* d_transport = nullptr;  // transport table blob
     uint8_t* d_rates_mixed = nullptr;      // tables of the mixed-precision form
     uint8_t* d_transport_mixed = nullptr;
@@ -62,6 +63,11 @@ int check_status(cb_mech* m) {
 
 enum class Path { Rates, ReactionRates, Transport, Fused, RatesMixed, TransportMixed, FusedMixed };
 
+template <class Args>
+auto set_f64_tables(Args& a, const uint8_t* tab) -> decltype((void)(a.f64_tab = tab)) { a.f64_tab = tab; }
+template <int KM>
+void set_f64_tables(cbg::TransportArgs<KM>&, const uint8_t*) {}
+
 template <template <int> class Args, int KM>
 int fill_and_launch(cb_mech* m, size_t n, const double* const* in, int ni, double* const* out, int no,
                     uint32_t flags, cudaStream_t st,
@@ -72,6 +78,7 @@ int fill_and_launch(cb_mech* m, size_t n, const double* const* in, int ni, doubl
     for (int q = 0; q < ni; q++) a.in[q] = in[q];
     for (int q = 0; q < no; q++) a.out[q] = out[q];
     a.flags = flags;
+    set_f64_tables(a, m->d_rates);
     cudaError_t e = launch(KM, tab, (uint32_t)tab_bytes, &a, n, st, m->d_status);
     return e == cudaSuccess ? CB_OK : cuda_fail(e, what);
 }
@@ -89,6 +96,16 @@ int dispatch(cb_mech* m, size_t n, const double* const* in, int ni, double* cons
     }
 }
 
+// The plain rates: the fixed-point kernel, or the FP64 one for a mechanism out of its range.
+int launch_rates_path(cb_mech* m, size_t n, const double* const* in, double* const* out, uint32_t flags, cudaStream_t st) {
+    const int K = m->host.K, A = m->host.A;
+    if (m->d_rates_fixed)
+        return dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, cbg::launch_rates_x, m->d_rates_fixed,
+                                        m->host.rates_fixed_blob.size(), "rates kernel");
+    return dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, cbg::launch_rates, m->d_rates,
+                                    m->host.rates_blob.size(), "rates kernel");
+}
+
 // One call on device pointers (pointer arrays already resolved).
 int launch_path(cb_mech* m, Path path, size_t n, const double* const* in, double* const* out, uint32_t flags,
                 cudaStream_t st) {
@@ -97,18 +114,20 @@ int launch_path(cb_mech* m, Path path, size_t n, const double* const* in, double
     const size_t rb = m->host.rates_blob.size(), tb = m->host.transport_blob.size();
     switch (path) {
     case Path::Rates:
-        return dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, cbg::launch_rates, m->d_rates, rb,
-                                        "rates kernel");
+        return launch_rates_path(m, n, in, out, flags, st);
     case Path::ReactionRates:
         if (R > cbg::kMaxReactions) return fail(CB_ERR_UNSUPPORTED, "more reactions than per-reaction outputs support");
+        if (m->d_rates_fixed)
+            return dispatch<cbg::ReactionRatesArgs>(m, n, in, K + 2, out, R, flags, st, cbg::launch_reaction_rates_x,
+                                                    m->d_rates_fixed, m->host.rates_fixed_blob.size(),
+                                                    "reaction rates kernel");
         return dispatch<cbg::ReactionRatesArgs>(m, n, in, K + 2, out, R, flags, st, cbg::launch_reaction_rates,
                                                 m->d_rates, rb, "reaction rates kernel");
     case Path::Transport:
         return dispatch<cbg::TransportArgs>(m, n, in, K + 1, out, K + 2, flags, st, cbg::launch_transport,
                                             m->d_transport, tb, "transport kernel");
     case Path::Fused: {
-        int rc = dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, cbg::launch_rates, m->d_rates, rb,
-                                          "rates kernel");
+        int rc = launch_rates_path(m, n, in, out, flags, st);
         if (rc) return rc;
         return dispatch<cbg::TransportArgs>(m, n, in, K + 3, out + (A + 2), K + 2, flags | cbg::kFromRates, st,
                                             cbg::launch_transport, m->d_transport, tb, "transport kernel");
@@ -161,12 +180,16 @@ size_t path_wave(const cb_mech* m, Path path) {
     const uint32_t rb = (uint32_t)m->host.rates_blob.size(), tb = (uint32_t)m->host.transport_blob.size();
     const uint32_t rmb = (uint32_t)m->host.rates_mixed_blob.size();
     const uint32_t tmb = (uint32_t)m->host.transport_mixed_blob.size();
+    const uint32_t rfb = (uint32_t)m->host.rates_fixed_blob.size();
+    auto rates_wave = [&] { return m->d_rates_fixed ? cbg::wave_rates_x(m->kmax, rfb) : cbg::wave_rates(m->kmax, rb); };
     size_t w[2] = {0, 0};
     switch (path) {
-    case Path::Rates: w[0] = cbg::wave_rates(m->kmax, rb); break;
-    case Path::ReactionRates: w[0] = cbg::wave_reaction_rates(m->kmax, rb); break;
+    case Path::Rates: w[0] = rates_wave(); break;
+    case Path::ReactionRates:
+        w[0] = m->d_rates_fixed ? cbg::wave_reaction_rates_x(m->kmax, rfb) : cbg::wave_reaction_rates(m->kmax, rb);
+        break;
     case Path::Transport: w[0] = cbg::wave_transport(m->kmax, tb); break;
-    case Path::Fused: w[0] = cbg::wave_rates(m->kmax, rb); w[1] = cbg::wave_transport(m->kmax, tb); break;
+    case Path::Fused: w[0] = rates_wave(); w[1] = cbg::wave_transport(m->kmax, tb); break;
     case Path::RatesMixed: w[0] = cbg::wave_rates_mixed(m->kmax, rmb); break;
     case Path::TransportMixed: w[0] = cbg::wave_transport_mixed(m->kmax, tmb); break;
     case Path::FusedMixed:
@@ -385,6 +408,12 @@ int cb_mech_create(const cb_mech_desc* desc, cb_mech** out) {
     cudaError_t e = cudaGetDevice(&m->device);
     if (e == cudaSuccess) e = cudaMalloc(&m->d_rates, m->host.rates_blob.size());
     if (e == cudaSuccess) e = cudaMemcpy(m->d_rates, m->host.rates_blob.data(), m->host.rates_blob.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && cbg::build_rates_fixed(m->host)) {
+        e = cudaMalloc(&m->d_rates_fixed, m->host.rates_fixed_blob.size());
+        if (e == cudaSuccess)
+            e = cudaMemcpy(m->d_rates_fixed, m->host.rates_fixed_blob.data(), m->host.rates_fixed_blob.size(),
+                           cudaMemcpyHostToDevice);
+    }
     if (e == cudaSuccess) e = cudaMalloc(&m->d_rates_mixed, m->host.rates_mixed_blob.size());
     if (e == cudaSuccess)
         e = cudaMemcpy(m->d_rates_mixed, m->host.rates_mixed_blob.data(), m->host.rates_mixed_blob.size(),
@@ -464,6 +493,7 @@ int cb_mech_destroy(cb_mech* m) {
         for (int e = 0; e < 3; e++)
             if (m->slot_event[s][e]) cudaEventDestroy(m->slot_event[s][e]);
     cudaFree(m->d_rates);
+    cudaFree(m->d_rates_fixed);
     cudaFree(m->d_transport);
     cudaFree(m->d_rates_mixed);
     cudaFree(m->d_transport_mixed);

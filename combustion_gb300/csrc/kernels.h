@@ -14,6 +14,9 @@ namespace cbg {
 // faster (the FP64 pipe is 97 % busy either way) and its per-thread arrays then spilled past L1 into
 // DRAM (24 KB per cell instead of 2 KB).
 constexpr int kBlock = 768;
+// The fixed-point rates kernels are bound by latency (integer chains, thread-local arrays in L2) as much as by
+// a pipe: 1,024 threads (64 registers) 40.2 ms, 768 (80) 48.0 ms at 2^22 cells of 53 species.
+constexpr int kRatesXBlock = 1024;
 constexpr int kTransportBlock = 256;
 constexpr int kTransportMixedBlock = 768;
 
@@ -23,6 +26,7 @@ struct RatesArgs {
     const double* in[KMAX + 3];  // P/R, R/P, T, V, n_0 .. n_{K-2}
     double* out[KMAX + 2];       // dT/dt, dV/dt, wdot_0 .. wdot_{A-1}
     uint32_t flags;              // bit 1: P/R and R/P are single values
+    const uint8_t* f64_tab;      // fixed-point kernels: the FP64 tables, in global memory
 };
 
 // Per-reaction rates of progress: inputs P/R, T, V, n_0 .. n_{K-2}; one output per reaction.
@@ -32,6 +36,7 @@ struct ReactionRatesArgs {
     const double* in[KMAX + 2];
     double* out[kMaxReactions];
     uint32_t flags;
+    const uint8_t* f64_tab;
 };
 
 // Transport input layouts: the reference's (sum n, T/T0, n...) or, with kFromRates, the rates inputs
@@ -62,6 +67,7 @@ inline int kmax_for(int K, int n_eff) {
 
 int max_table_smem();
 cudaError_t set_stage_wait_polls(long long polls);
+cudaError_t set_stage_wait_polls_x(long long polls);  // of the fixed-point kernels' translation unit
 
 // Non-finite values (NaN, infinity) in up to kCountArrays arrays of n doubles, added to *count.
 constexpr int kCountArrays = 512;
@@ -112,6 +118,13 @@ cudaError_t launch_rates(int kmax, const uint8_t* tab, uint32_t tab_bytes, const
                          cudaStream_t st, int* status);
 cudaError_t launch_reaction_rates(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                   cudaStream_t st, int* status);
+// The fixed-point forms (kernels_fixed.cu); `args` carries the FP64 tables as well.
+cudaError_t launch_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
+                           cudaStream_t st, int* status);
+cudaError_t launch_reaction_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
+                                    cudaStream_t st, int* status);
+size_t wave_rates_x(int kmax, uint32_t tab_bytes);
+size_t wave_reaction_rates_x(int kmax, uint32_t tab_bytes);
 cudaError_t launch_rates_mixed(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                cudaStream_t st, int* status);
 cudaError_t launch_transport_mixed(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,

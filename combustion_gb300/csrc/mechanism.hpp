@@ -24,6 +24,7 @@ struct HostMechanism {
 
     std::vector<uint8_t> rates_blob;
     std::vector<uint8_t> rates_mixed_blob;  // tables of the mixed-precision form
+    std::vector<uint8_t> rates_fixed_blob;  // fixed-point tables of the plain form (empty: out of their range)
     Work rates_work;
 
     bool transport_ready = false;
@@ -39,6 +40,10 @@ struct HostMechanism {
 int build_mechanism(const cb_mech_desc* d, HostMechanism& m, std::string& err);
 // Fits the species properties and packs the transport tables for the given normalisation.
 int build_transport(HostMechanism& m, double T0, double mu0, double lambda0, std::string& err);
+
+// Fixed-point tables of the plain rates kernels (fixed_tables.cpp); false, and no tables, when a constant
+// is out of their range.
+bool build_rates_fixed(HostMechanism& m);
 
 struct MathTables;
 MathTables make_math_tables();

@@ -1,0 +1,105 @@
+// Tables of the plain rates kernels' fixed-point form (fixed_math.cuh, kernels.cu), built by
+// fixed_tables.cpp from the FP64 tables (tables.h) of the same mechanism.
+//
+// Everything that depends on the temperature alone (rate constants, Gibbs energies) is evaluated as a
+// base-2 logarithm in 64-bit fixed point on the integer pipe; the third-body sums are fixed-point dot
+// products. Numbers are Qn: the integer times 2^-n. A product term keeps each factor as two signed
+// 32-bit words, value = (hi 2^29 + lo) 2^-(q + 29) with |lo| <= 2^28, hi Qq.
+#pragma once
+#include <stdint.h>
+
+#include "tables.h"
+
+namespace cbg {
+
+constexpr int kExpTable = 1024, kLogTable = 512;
+struct FixMath {
+    uint64_t exp2t[kExpTable];  // 2^(j/1024), Q62
+    int64_t log2c[kLogTable];   // -log2(rc[j] / 4096), Q62
+    uint32_t rc[kLogTable];     // nearest 12-bit reciprocal of 1 + (j + 1/2) / 512, Q12
+};
+constexpr int kFixMathBytes = (int)sizeof(FixMath);
+static_assert(kFixMathBytes % kAlign == 0, "fixed-point tables must keep the blob sections aligned");
+
+// Bounds of the fixed-point form. A cell takes it for T in [kFixTmin, kFixTmax); a mechanism when every
+// constant fits its word over that range (fixed_tables.cpp checks; otherwise the FP64 form runs).
+constexpr double kFixTmin = 200.0, kFixTmax = 8192.0, kFixTmid = 2048.0;
+constexpr int kYq = 51;    // base-2 logarithms: |y| < 2^12
+constexpr int kLo = 29;    // bits of a low word
+constexpr int kLq = 27;    // log2 T, hi word (log2 T < 13)
+constexpr int kBq = 24;    // its factor, |.| < 64
+constexpr int kRq = 37;    // 1 / T, hi word (1/T <= 1/200)
+constexpr int kEq = 14;    // its factor, |.| < 2^17
+constexpr int kPq = 30;    // (T / 2^p)^i, hi word, p = 11 below 2048 K and 13 above
+constexpr int kGq = 18;    // its factor, |.| < 4096
+constexpr int kCq = 29;    // C_k / S, hi word (S a power of two above every sum of concentrations)
+constexpr int kEffBits = 55;  // |efficiency - 1| 2^eff_shift < 2^kEffBits
+
+struct Word2 {
+    int32_t hi, lo;
+};
+
+// log2 of k = exp(beta ln T + mEa / T + ln A).
+struct ArrheniusX {
+    Word2 b, e;  // factors of log2 T and 1 / T
+    int64_t a;   // Qy
+};
+
+// Shape flags of a reaction (ReactionX::shape).
+enum Shape : uint32_t {
+    kShapeR2 = 1,        // two reactant factors (else one)
+    kShapeP2 = 2,        // two product factors (else one)
+    kShapeNet = 4,       // net species: bits 2-4 (1 .. 4)
+    kShapeNeg = 32,      // bit 5 + j: net species j is consumed
+    kShapeTwo = 512,     // bit 9 + j: by two
+    kShapeMsn = 8192,    // minus the net order, plus 2: bits 13-15
+    kShapeGeneral = 65536  // none of the above but the order: the lists below with their multiplicities
+};
+struct ReactionX {  // 64 bytes
+    ArrheniusX k;
+    uint32_t shape;
+    int32_t orig;
+    // up to two factors on each side (a doubled species twice) and four net species changing by one or two,
+    // or (kShapeGeneral) distinct species with the multiplicities that follow
+    uint8_t r_k[kMaxSide], p_k[kMaxSide], net_k[kMaxNet];
+    int8_t r_n[kMaxSide], p_n[kMaxSide], net_n[kMaxNet];
+};
+static_assert(sizeof(ReactionX) == 64, "four 16-byte loads");
+
+// One per reaction of models 2-5, in reaction order (three-body entries unused). Exponents and
+// logarithms in base 2.
+struct FalloffX {
+    ArrheniusX k0;
+    double ainf, c1mA, cA, c3, c1, cmT2, l2_fcent;
+    int64_t lainf;          // log2(ainf), Qy
+    int32_t flags, sri_flags;
+    double sA, smB, smrC, sD, sE;
+};
+
+// Gibbs energy over RT in base-2 units: piece 0 for T <= split, else 1 below kFixTmid and 2 above (the
+// same polynomial in (T / 2^11) and (T / 2^13)).
+struct SpeciesX {
+    double split;
+    int64_t g0[3];
+    Word2 g[3][6];  // factors of log2 T, 1/T, (T/2^p)^1 .. ^4
+    int32_t need_exp, need_exp_neg;
+};
+
+// h / RT (powers 1 .. 4 of T / 2^p, then 1/T) and cp / R, pieces as SpeciesX::g.
+struct ThermoX {
+    double split, dtE;
+    int64_t h0[3], cp0[3];  // Qy
+    Word2 h[3][5];          // factors of (T/2^p)^1 .. ^4, 1/T
+    Word2 cp[3][4];
+};
+
+struct RatesXHeader {
+    int32_t K, A, R, n_eff, total_bytes, off_species, off_thermo, off_reactions, off_falloff, off_eff;
+    int32_t group_end[6];
+    int64_t lM3, lcbrt, lC0;  // log2 of the Gibbs exponentials' caps and of P0 / R, Qy
+    int32_t eff_shift;        // efficiency words are (e - 1) 2^eff_shift, eff_shift <= kEffBits
+    int32_t pad;
+    double l10_04, l10_075;   // 0.4 and 0.75 log2(10)
+};
+
+}  // namespace cbg

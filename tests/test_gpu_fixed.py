@@ -1,0 +1,110 @@
+"""The plain rates kernels' fixed-point form at the edges of its range, against the FP64 oracle.
+
+Cells at and around the temperatures where a cell changes form (200 K, 8,192 K: the FP64 form outside) or
+table piece (2,048 K), in one call with ordinary ones; reactions of every shape (one to four factors on a
+side, multiplicities up to three, one to seven net species, every net order, irreversible); a mechanism whose
+constants are out of range (the FP64 kernel); calls of 1 cell to more than two waves.
+The bar is the plain form's: 1e-12 condition-scaled.
+"""
+import copy
+import os
+
+import numpy as np
+import pytest
+
+import util
+from combustion_gb300 import synthetic
+
+pytestmark = pytest.mark.gpu
+NTHREADS = os.cpu_count() or 4
+
+
+def shapes_mechanism(config):
+    """The generator's mechanism with reactions of the shapes it never draws."""
+    m = copy.deepcopy(util.mechanism(config))
+    K = m.K
+    sides = [  # reactants, products (species index: multiplicity); net order within -1 .. 2
+        ({0: 3}, {1: 1, 2: 1, 3: 1}), ({0: 1, 1: 1, 2: 1}, {3: 2, 4: 1}), ({2: 2, 3: 1, 4: 1}, {5: 1, 6: 1, 7: 1}),
+        ({5: 1}, {6: 2}), ({6: 1}, {5: 1, 7: 1, 8: 1}), ({7: 2}, {8: 1}), ({1: 1, K - 1: 1}, {2: 1, K - 1: 1}),
+        ({0: 1, 1: 1, 2: 1, 3: 1}, {4: 1, 5: 1, 6: 2}), ({8: 1}, {7: 1}), ({4: 2}, {0: 2})]
+    kinds = [np.flatnonzero(m.model == k) for k in (synthetic.ELEMENTARY, synthetic.THREE_BODY, synthetic.TROE)]
+    rows = list(kinds[0][:len(sides)]) + [kinds[1][0], kinds[2][0]]
+    for r, (lhs, rhs) in zip(rows, sides + [sides[1], sides[4]]):
+        m.reactants[r] = 0
+        m.products[r] = 0
+        for k, n in lhs.items():
+            m.reactants[r, k] = n
+        for k, n in rhs.items():
+            m.products[r, k] = n
+    m.model[rows[2]] = synthetic.IRREVERSIBLE
+    lin = kinds[0][len(sides)]
+    m.model[lin] = synthetic.LINDEMANN
+    m.k0[lin] = (m.rate[lin, 0] * 1e-3, m.rate[lin, 1] - 0.3, m.rate[lin, 2] * 0.7)
+    m.efficiencies[lin] = np.linspace(0.5, 4.0, K)
+    m.meta = {"config": config + "-shapes"}
+    assert m.active() == K - 1
+    return m
+
+
+def out_of_range_mechanism(config):
+    m = copy.deepcopy(util.mechanism(config))
+    m.rate[0] = (1e40, 0.0, 2e5)
+    return m
+
+
+def edge_temperatures(config, n):
+    cells = synthetic.generate_cells(util.mechanism(config).K, n, config, seed=31)
+    up = np.nextafter
+    edges = [150.0, up(200.0, 0), 200.0, up(200.0, 1e9), 999.0, 1000.0, up(1000.0, 1e9), up(2048.0, 0), 2048.0,
+             up(2048.0, 1e9), 4096.0, up(8192.0, 0), 8192.0, 9000.0]
+    scale = cells.temperature.copy()
+    cells.temperature[:len(edges)] = edges[:n]
+    scale /= cells.temperature  # the ideal-gas total keeps P and V
+    cells.total_amount *= scale
+    cells.amounts *= scale
+    return cells
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+@pytest.mark.parametrize("make", [util.mechanism, shapes_mechanism, out_of_range_mechanism],
+                         ids=["generator", "shapes", "out-of-range"])
+def test_range_and_shapes(config, make):
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = make(config)
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    cells = edge_temperatures(config, 96)
+    rin = o.rates_inputs(cells)
+    dev = lambda x: torch.tensor(np.array(x), dtype=torch.float64, device="cuda")  # noqa: E731
+    out = torch.full((mech.A + 2, cells.n), float("nan"), dtype=torch.float64, device="cuda")
+    mech.rates(dev(rin), out)
+    pin = o.reaction_rates_inputs(cells)
+    progress = torch.full((mech.R, cells.n), float("nan"), dtype=torch.float64, device="cuda")
+    mech.reaction_rates(dev(pin), progress)
+    mech.synchronize()
+    for name, x, (ref, sc) in (("rates", out, o.rates(rin, nthreads=NTHREADS, scale=True)),
+                               ("progress", progress, o.reaction_rates(pin, nthreads=NTHREADS, scale=True))):
+        x = x.cpu().numpy()
+        assert np.array_equal(np.isfinite(x), np.isfinite(ref))
+        e = util.cond_err(x, ref, sc)
+        print(f"{config} {name}: max cond err {np.nanmax(e):.2e} (cell T = {cells.temperature[np.nanargmax(np.nanmax(e, 0))]:g})")
+        assert np.nanmax(e) <= util.PLAIN_TOL
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1023, 4865, 155649, 311297])
+def test_call_sizes(n):
+    """Every launch shape gives each cell the value it has in a call of its own block."""
+    import torch
+    import combustion_gb300 as cb
+    from combustion_gb300 import surrogate as S
+    mech = cb.Mechanism(util.mechanism("k10"))
+    cells = S.generate_cells(mech, n, S.distribution("k53", seed=9))
+    out = torch.full((mech.A + 2, n), float("nan"), dtype=torch.float64, device="cuda")
+    mech.rates(cells, out)
+    pick = torch.unique(torch.tensor([0, n // 3, n // 2, n - 1], device="cuda"))
+    few = torch.empty((mech.A + 2, len(pick)), dtype=torch.float64, device="cuda")
+    mech.rates(cells[:, pick].contiguous(), few)
+    assert torch.isfinite(out).all()
+    scale = out.abs().amax(dim=0)
+    assert ((out[:, pick] - few).abs() <= 1e-12 * scale[pick]).all()
