@@ -22,6 +22,7 @@ struct cb_mech {
     uint8_t* d_rates = nullptr;      // rates table blob
     uint8_t* d_rates_fixed = nullptr;  // the same in fixed point (null: the mechanism is out of its range)
     uint8_t* d_transport = nullptr;  // transport table blob
+    uint8_t* d_transport_fixed = nullptr;  // the same in fixed point (null: out of its range)
     uint8_t* d_rates_mixed = nullptr;      // tables of the mixed-precision form
     uint8_t* d_transport_mixed = nullptr;
     int* d_status = nullptr;         // kernel status bits
@@ -64,9 +65,9 @@ int check_status(cb_mech* m) {
 enum class Path { Rates, ReactionRates, Transport, Fused, RatesMixed, TransportMixed, FusedMixed };
 
 template <class Args>
-auto set_f64_tables(Args& a, const uint8_t* tab) -> decltype((void)(a.f64_tab = tab)) { a.f64_tab = tab; }
+void set_f64_tables(Args& a, const cb_mech* m) { a.f64_tab = m->d_rates; }
 template <int KM>
-void set_f64_tables(cbg::TransportArgs<KM>&, const uint8_t*) {}
+void set_f64_tables(cbg::TransportArgs<KM>& a, const cb_mech* m) { a.f64_tab = m->d_transport; }
 
 template <template <int> class Args, int KM>
 int fill_and_launch(cb_mech* m, size_t n, const double* const* in, int ni, double* const* out, int no,
@@ -78,7 +79,7 @@ int fill_and_launch(cb_mech* m, size_t n, const double* const* in, int ni, doubl
     for (int q = 0; q < ni; q++) a.in[q] = in[q];
     for (int q = 0; q < no; q++) a.out[q] = out[q];
     a.flags = flags;
-    set_f64_tables(a, m->d_rates);
+    set_f64_tables(a, m);
     cudaError_t e = launch(KM, tab, (uint32_t)tab_bytes, &a, n, st, m->d_status);
     return e == cudaSuccess ? CB_OK : cuda_fail(e, what);
 }
@@ -106,12 +107,25 @@ int launch_rates_path(cb_mech* m, size_t n, const double* const* in, double* con
                                     m->host.rates_blob.size(), "rates kernel");
 }
 
+// The plain transport: the fixed-point kernels, or the FP64 ones.
+struct TransportLaunch {
+    cudaError_t (*launch)(int, const uint8_t*, uint32_t, const void*, size_t, cudaStream_t, int*);
+    const uint8_t* tab;
+    size_t bytes;
+};
+TransportLaunch transport_launch(const cb_mech* m) {
+    if (m->d_transport_fixed)
+        return {cbg::launch_transport_x, m->d_transport_fixed, m->host.transport_fixed_blob.size()};
+    return {cbg::launch_transport, m->d_transport, m->host.transport_blob.size()};
+}
+
 // One call on device pointers (pointer arrays already resolved).
 int launch_path(cb_mech* m, Path path, size_t n, const double* const* in, double* const* out, uint32_t flags,
                 cudaStream_t st) {
     const int K = m->host.K, A = m->host.A, R = m->host.R;
     if (n == 0) return CB_OK;
-    const size_t rb = m->host.rates_blob.size(), tb = m->host.transport_blob.size();
+    const size_t rb = m->host.rates_blob.size();
+    const TransportLaunch t = transport_launch(m);
     switch (path) {
     case Path::Rates:
         return launch_rates_path(m, n, in, out, flags, st);
@@ -124,13 +138,13 @@ int launch_path(cb_mech* m, Path path, size_t n, const double* const* in, double
         return dispatch<cbg::ReactionRatesArgs>(m, n, in, K + 2, out, R, flags, st, cbg::launch_reaction_rates,
                                                 m->d_rates, rb, "reaction rates kernel");
     case Path::Transport:
-        return dispatch<cbg::TransportArgs>(m, n, in, K + 1, out, K + 2, flags, st, cbg::launch_transport,
-                                            m->d_transport, tb, "transport kernel");
+        return dispatch<cbg::TransportArgs>(m, n, in, K + 1, out, K + 2, flags, st, t.launch, t.tab, t.bytes,
+                                            "transport kernel");
     case Path::Fused: {
         int rc = launch_rates_path(m, n, in, out, flags, st);
         if (rc) return rc;
-        return dispatch<cbg::TransportArgs>(m, n, in, K + 3, out + (A + 2), K + 2, flags | cbg::kFromRates, st,
-                                            cbg::launch_transport, m->d_transport, tb, "transport kernel");
+        return dispatch<cbg::TransportArgs>(m, n, in, K + 3, out + (A + 2), K + 2, flags | cbg::kFromRates, st, t.launch,
+                                            t.tab, t.bytes, "transport kernel");
     }
     case Path::RatesMixed:
         return dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, cbg::launch_rates_mixed,
@@ -182,14 +196,18 @@ size_t path_wave(const cb_mech* m, Path path) {
     const uint32_t tmb = (uint32_t)m->host.transport_mixed_blob.size();
     const uint32_t rfb = (uint32_t)m->host.rates_fixed_blob.size();
     auto rates_wave = [&] { return m->d_rates_fixed ? cbg::wave_rates_x(m->kmax, rfb) : cbg::wave_rates(m->kmax, rb); };
+    const uint32_t tfb = (uint32_t)m->host.transport_fixed_blob.size();
+    auto transport_wave = [&] {
+        return m->d_transport_fixed ? cbg::wave_transport_x(m->kmax, tfb) : cbg::wave_transport(m->kmax, tb);
+    };
     size_t w[2] = {0, 0};
     switch (path) {
     case Path::Rates: w[0] = rates_wave(); break;
     case Path::ReactionRates:
         w[0] = m->d_rates_fixed ? cbg::wave_reaction_rates_x(m->kmax, rfb) : cbg::wave_reaction_rates(m->kmax, rb);
         break;
-    case Path::Transport: w[0] = cbg::wave_transport(m->kmax, tb); break;
-    case Path::Fused: w[0] = rates_wave(); w[1] = cbg::wave_transport(m->kmax, tb); break;
+    case Path::Transport: w[0] = transport_wave(); break;
+    case Path::Fused: w[0] = rates_wave(); w[1] = transport_wave(); break;
     case Path::RatesMixed: w[0] = cbg::wave_rates_mixed(m->kmax, rmb); break;
     case Path::TransportMixed: w[0] = cbg::wave_transport_mixed(m->kmax, tmb); break;
     case Path::FusedMixed:
@@ -337,8 +355,9 @@ int gather_launch(cb_mech* m, size_t n, const double* const* in, double* const* 
     a.flags = (flags & CB_UNIFORM_PRESSURE) | cbg::kFromRates | (compact ? cbg::kCompactOut : 0u);
     a.index = index;
     a.count = count;
-    cudaError_t e = cbg::launch_transport(KM, m->d_transport, (uint32_t)m->host.transport_blob.size(), &a, n, st,
-                                          m->d_status);
+    set_f64_tables(a, m);
+    const TransportLaunch t = transport_launch(m);
+    cudaError_t e = t.launch(KM, t.tab, (uint32_t)t.bytes, &a, n, st, m->d_status);
     return e == cudaSuccess ? CB_OK : cuda_fail(e, "transport kernel (gathered cells)");
 }
 
@@ -495,6 +514,7 @@ int cb_mech_destroy(cb_mech* m) {
     cudaFree(m->d_rates);
     cudaFree(m->d_rates_fixed);
     cudaFree(m->d_transport);
+    cudaFree(m->d_transport_fixed);
     cudaFree(m->d_rates_mixed);
     cudaFree(m->d_transport_mixed);
     cudaFree(m->d_status);
@@ -531,14 +551,20 @@ int cb_transport_setup(cb_mech* m, double T0, double viscosity0, double conducti
     if (m->d_transport || m->d_transport_mixed) {
         CB_CUDA(cudaDeviceSynchronize());
         cudaFree(m->d_transport);
+        cudaFree(m->d_transport_fixed);
         cudaFree(m->d_transport_mixed);
-        m->d_transport = m->d_transport_mixed = nullptr;
+        m->d_transport = m->d_transport_fixed = m->d_transport_mixed = nullptr;
     }
     CB_CUDA(cudaMalloc(&m->d_transport, m->host.transport_blob.size()));
     CB_CUDA(cudaMemcpy(m->d_transport, m->host.transport_blob.data(), m->host.transport_blob.size(), cudaMemcpyHostToDevice));
     CB_CUDA(cudaMalloc(&m->d_transport_mixed, m->host.transport_mixed_blob.size()));
     CB_CUDA(cudaMemcpy(m->d_transport_mixed, m->host.transport_mixed_blob.data(), m->host.transport_mixed_blob.size(),
                        cudaMemcpyHostToDevice));
+    if (cbg::build_transport_fixed(m->host)) {
+        CB_CUDA(cudaMalloc(&m->d_transport_fixed, m->host.transport_fixed_blob.size()));
+        CB_CUDA(cudaMemcpy(m->d_transport_fixed, m->host.transport_fixed_blob.data(), m->host.transport_fixed_blob.size(),
+                           cudaMemcpyHostToDevice));
+    }
     return CB_OK;
 }
 

@@ -29,11 +29,12 @@ __device__ __forceinline__ unsigned long long mul_wide_u(unsigned a, unsigned b)
     return d;
 }
 
-// Words of a fixed-point integer (|v| < 2^60): v = hi 2^29 + lo, lo balanced.
+// Words of a fixed-point integer (|v| < 2^60): v = hi 2^LO + lo, lo balanced.
+template <int LO = kLo>
 __device__ __forceinline__ Word2 split_word(long long v) {
     Word2 w;
-    w.hi = (int)((v + (1ll << (kLo - 1))) >> kLo);
-    w.lo = (int)(v - ((long long)w.hi << kLo));
+    w.hi = (int)((v + (1ll << (LO - 1))) >> LO);
+    w.lo = (int)(v - ((long long)w.hi << LO));
     return w;
 }
 
@@ -144,6 +145,25 @@ __device__ __forceinline__ double log2_dbl(double x) {
     const int hi = __double2hiint(x);
     if (hi < 0x00100000 || hi >= 0x7ff00000) return log2_slow(x);  // <= 0, subnormal, inf or NaN
     return fix_to_dbl(log2_fix(x), kYq);
+}
+
+
+// 1 / (d 2^-60 2^sp) for 2^54 < d < 2^61, as a double; bias = PolyX::rcp_bias. A 24-bit estimate R0 2^-84 of 1/d,
+// its residual e = 1 - d R0 2^-84 exactly (modulo 2^64), and R0 (1 + e + e^2): e^3 is below 2^-60.
+__device__ __forceinline__ double rcp_fixed(long long d, int bias) {
+    const float f = __uint2float_rn((unsigned)(d >> 30));
+    float r0;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(f));
+    const unsigned R0 = __float2uint_rn(r0 * 0x1p54f);
+    const long long e = -(long long)((unsigned long long)d * R0);  // Q84
+    const int eh = (int)(e >> 32);                                 // Q52
+    const long long s = e + (mad_wide(eh, eh, 0) >> 20);
+    const long long corr = mad_wide((int)R0, (int)(s >> 32), 0) + __umulhi(R0, (unsigned)s);  // R0 s, Q52
+    const unsigned long long R = ((unsigned long long)R0 << 32) + (unsigned long long)(corr >> 20);
+    const int lz = __clz((int)(R >> 32));
+    const unsigned hi = __funnelshift_l((unsigned)R, (unsigned)(R >> 32), lz), lo = (unsigned)R << lz;
+    const unsigned long long m = ((unsigned long long)hi << 32) | lo;
+    return __longlong_as_double(((long long)(bias - lz) << 52) + (long long)(m >> 11) + (long long)((m >> 10) & 1));
 }
 
 }  // namespace cbg

@@ -18,16 +18,16 @@ bool to_fix(long double x, int q, long double limit, int64_t& v) {
     v = (int64_t)std::llround(std::ldexp(x, q));
     return true;
 }
-Word2 words(int64_t v) {
+Word2 words(int64_t v, int lo = kLo) {
     Word2 w;
-    w.hi = (int32_t)((v + (1ll << (kLo - 1))) >> kLo);
-    w.lo = (int32_t)(v - ((int64_t)w.hi << kLo));
+    w.hi = (int32_t)((v + (1ll << (lo - 1))) >> lo);
+    w.lo = (int32_t)(v - ((int64_t)w.hi << lo));
     return w;
 }
-bool to_words(long double x, int q_hi, long double limit, Word2& w) {
+bool to_words(long double x, int q_hi, long double limit, Word2& w, int lo = kLo) {
     int64_t v;
-    if (!to_fix(x, q_hi + kLo, limit, v)) return false;
-    w = words(v);
+    if (!to_fix(x, q_hi + lo, limit, v)) return false;
+    w = words(v, lo);
     return true;
 }
 
@@ -248,6 +248,106 @@ bool build_rates_fixed(HostMechanism& m) {
     X.off_reactions = put(b, fx.data(), fx.size());
     X.off_falloff = put(b, ff.data(), ff.size());
     X.off_eff = put(b, ef.data(), ef.size());
+    while (b.size() % kAlign) b.push_back(0);
+    X.total_bytes = (int32_t)b.size();
+    std::memcpy(b.data() + off_header, &X, sizeof X);
+    return true;
+}
+
+namespace {
+
+// A polynomial over the fixed-point temperature range: positive, within a factor of 2^5, coefficients that fit.
+bool poly_fix(const double* P, double T0, int pw, long double scale, PolyX& f) {
+    long double lo = 1e300L, hi = 0.0L;
+    const long double a = std::log((long double)kFixTransportTmin / T0), b = std::log((long double)kFixTransportTmax / T0);
+    for (int i = 0; i <= 256; i++) {
+        const long double L = a + (b - a) * i / 256.0L;
+        const long double D = scale * (P[0] + L * (P[1] + L * (P[2] + L * (P[3] + L * (long double)P[4]))));
+        lo = std::min(lo, D);
+        hi = std::max(hi, D);
+    }
+    if (!(lo > 1e-290L) || !(hi < 1e290L)) return false;
+    int e;
+    std::frexp((double)(hi * 1.0001L), &e);  // hi < 2^e
+    if (!(lo > std::ldexp(1.0L, e - 5))) return false;
+    f.sp = e;
+    f.rcp_bias = 1022 + 63 - 56 - e;
+    if (!to_fix(std::ldexp((long double)P[0] * scale, -e), kDq, 4.0L, f.p0)) return false;
+    for (int m = 1; m <= 4; m++)
+        if (!to_words(std::ldexp((long double)P[m] * scale, pw * m - e), kPpq, 4.0L, f.p[m - 1], kPlo)) return false;
+    return true;
+}
+
+}  // namespace
+
+bool build_transport_fixed(HostMechanism& m) {
+    m.transport_fixed_blob.clear();
+    const uint8_t* blob = m.transport_blob.data();
+    TransportHeader H;
+    std::memcpy(&H, blob + kMathBytes, sizeof H);
+    const int K = H.K;
+    if (K > 256) return false;
+    auto doubles = [&](int32_t off, size_t n) {
+        std::vector<double> v(n);
+        std::memcpy(v.data(), blob + off, n * sizeof(double));
+        return v;
+    };
+    const std::vector<double> cond = doubles(H.off_cond, (size_t)K * 5), visc = doubles(H.off_visc, (size_t)K * 5);
+    const std::vector<double> W = doubles(H.off_W, K), diff = doubles(H.off_diff, (size_t)H.n_pairs * 5);
+    const std::vector<double> A2 = doubles(H.off_A2, (size_t)K * K), AB = doubles(H.off_AB, (size_t)K * K);
+    const std::vector<double> B2 = doubles(H.off_B2, (size_t)K * K);
+    TransportXHeader X;
+    std::memset(&X, 0, sizeof X);
+    X.K = K;
+    X.n_pairs = H.n_pairs;
+    X.T0 = H.T0;
+    X.Tn_lo = kFixTransportTmin / H.T0;
+    X.Tn_hi = kFixTransportTmax / H.T0;
+    const double Lmax = std::max(std::fabs(std::log(X.Tn_lo)), std::fabs(std::log(X.Tn_hi)));
+    while (std::ldexp(1.0, X.pw) <= Lmax) X.pw++;
+    if (X.pw > 4) return false;
+    std::vector<PolyX> pc(K), pv(K), pd(std::max(H.n_pairs, 1));
+    std::memset(pc.data(), 0, pc.size() * sizeof(PolyX));
+    std::memset(pv.data(), 0, pv.size() * sizeof(PolyX));
+    std::memset(pd.data(), 0, pd.size() * sizeof(PolyX));
+    std::vector<double> W4(K);
+    std::vector<long double> w4(K);  // W^(1/4)
+    for (int k = 0; k < K; k++) {
+        w4[k] = std::sqrt(std::sqrt((long double)m.W[k]));
+        W4[k] = (double)std::sqrt((long double)m.W[k]);
+        if (!poly_fix(&cond[(size_t)k * 5], H.T0, X.pw, 1.0, pc[k])) return false;
+        if (!poly_fix(&visc[(size_t)k * 5], H.T0, X.pw, 1.0L / w4[k], pv[k])) return false;
+    }
+    for (int p = 0; p < H.n_pairs; p++)
+        if (!poly_fix(&diff[(size_t)p * 5], H.T0, X.pw, 1.0, pd[p])) return false;
+    // b_kj = a_kj (W_j / W_k)^(1/4) to FP64 rounding (a constant that the reference's builder folds to 0 or 1 is
+    // not); |a^2| to the words' position
+    double largest = 0.;
+    for (int k = 0; k < K; k++)
+        for (int j = 0; j < K; j++) {
+            const size_t i = (size_t)k * K + j;
+            const long double r = w4[j] / w4[k], a2 = A2[i];
+            if (!(A2[i] > 0.) || std::fabs(AB[i] / (2.0L * a2 * r) - 1.0L) > 2e-15L || std::fabs(B2[i] / (a2 * r * r) - 1.0L) > 2e-15L)
+                return false;
+            largest = std::max(largest, A2[i]);
+        }
+    const int bits = K <= 64 ? kMixAq<64> : kMixAq<256>;
+    X.a_shift = bits;
+    while (std::ldexp(largest, X.a_shift) >= std::ldexp(1.0, bits)) X.a_shift--;
+    while (std::ldexp(largest, X.a_shift + 1) < std::ldexp(1.0, bits)) X.a_shift++;
+    std::vector<Word2> a2((size_t)K * K);
+    for (size_t i = 0; i < a2.size(); i++) a2[i] = words((int64_t)std::llround(std::ldexp((long double)A2[i], X.a_shift)));
+
+    std::vector<uint8_t>& b = m.transport_fixed_blob;
+    b.insert(b.end(), blob, blob + kMathBytes);
+    const int32_t off_header = put(b, &X, 1);
+    if (off_header != kMathBytes) return false;
+    X.off_cond = put(b, pc.data(), pc.size());
+    X.off_visc = put(b, pv.data(), pv.size());
+    X.off_W = put(b, W.data(), W.size());
+    X.off_W4 = put(b, W4.data(), W4.size());
+    X.off_diff = put(b, pd.data(), pd.size());
+    X.off_A2 = put(b, a2.data(), a2.size());
     while (b.size() % kAlign) b.push_back(0);
     X.total_bytes = (int32_t)b.size();
     std::memcpy(b.data() + off_header, &X, sizeof X);

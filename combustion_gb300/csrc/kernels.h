@@ -17,6 +17,11 @@ constexpr int kBlock = 768;
 // The fixed-point rates kernels are bound by latency (integer chains, thread-local arrays in L2) as much as by
 // a pipe: 1,024 threads (64 registers) 40.2 ms, 768 (80) 48.0 ms at 2^22 cells of 53 species.
 constexpr int kRatesXBlock = 1024;
+// Fixed-point transport, 2^22 cells: 53 species 45.1 ms with 512 threads (128 registers, Wilke rows without spills),
+// 48.3 with 640; 10 species 2.95 ms with 512, 2.80 with 768; 250 species (131,072 cells), whose arrays are in L2
+// either way, 50 ms with 512 and 40 with 1,024.
+template <int KMAX>
+constexpr int kTransportXBlock = KMAX == 16 ? 768 : KMAX == 64 ? 512 : 1024;
 constexpr int kTransportBlock = 256;
 constexpr int kTransportMixedBlock = 768;
 
@@ -55,6 +60,7 @@ struct TransportArgs {
     uint32_t flags;
     const uint32_t* index;       // gathered cells (null: cell j is input j)
     const uint32_t* count;       // number of gathered cells, read on the device (null: n)
+    const uint8_t* f64_tab;      // fixed-point kernels: the FP64 tables, in global memory
 };
 
 // Smallest compiled capacity holding K species (0 if none).
@@ -67,7 +73,9 @@ inline int kmax_for(int K, int n_eff) {
 
 int max_table_smem();
 cudaError_t set_stage_wait_polls(long long polls);
-cudaError_t set_stage_wait_polls_x(long long polls);  // of the fixed-point kernels' translation unit
+// The same of the fixed-point kernels' translation units.
+cudaError_t set_stage_wait_polls_x(long long polls);
+cudaError_t set_stage_wait_polls_tx(long long polls);
 
 // Non-finite values (NaN, infinity) in up to kCountArrays arrays of n doubles, added to *count.
 constexpr int kCountArrays = 512;
@@ -123,6 +131,9 @@ cudaError_t launch_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, con
                            cudaStream_t st, int* status);
 cudaError_t launch_reaction_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                     cudaStream_t st, int* status);
+cudaError_t launch_transport_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
+                               cudaStream_t st, int* status);
+size_t wave_transport_x(int kmax, uint32_t tab_bytes);
 size_t wave_rates_x(int kmax, uint32_t tab_bytes);
 size_t wave_reaction_rates_x(int kmax, uint32_t tab_bytes);
 cudaError_t launch_rates_mixed(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,

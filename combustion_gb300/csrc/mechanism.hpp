@@ -32,6 +32,7 @@ struct HostMechanism {
     std::vector<double> fit_cond, fit_visc, fit_diff;  // raw fits [K*5], [K*5], [K*K*5]
     std::vector<uint8_t> transport_blob;
     std::vector<uint8_t> transport_mixed_blob;
+    std::vector<uint8_t> transport_fixed_blob;  // fixed-point tables of the plain form (empty: out of their range)
     Work transport_work;
 };
 
@@ -41,9 +42,10 @@ int build_mechanism(const cb_mech_desc* d, HostMechanism& m, std::string& err);
 // Fits the species properties and packs the transport tables for the given normalisation.
 int build_transport(HostMechanism& m, double T0, double mu0, double lambda0, std::string& err);
 
-// Fixed-point tables of the plain rates kernels (fixed_tables.cpp); false, and no tables, when a constant
+// Fixed-point tables of the plain kernels (fixed_tables.cpp); false, and no tables, when a constant
 // is out of their range.
 bool build_rates_fixed(HostMechanism& m);
+bool build_transport_fixed(HostMechanism& m);
 
 struct MathTables;
 MathTables make_math_tables();

@@ -102,4 +102,32 @@ struct RatesXHeader {
     double l10_04, l10_075;   // 0.4 and 0.75 log2(10)
 };
 
+// ---- transport --------------------------------------------------------------------------------------
+// A fitted polynomial D = P0 + P1 L + .. + P4 L^4 in L = ln(T/T0), over 2^sp so that it lies in (2^-6, 1) over
+// the fixed-point temperature range.
+constexpr int kFixTransportTmin = 200, kFixTransportTmax = 4000;
+constexpr int kLpq = 29;  // (L / 2^pw)^m, hi word
+constexpr int kPpq = 28;  // its coefficient, |.| < 4
+constexpr int kPlo = 30;  // bits of their low words
+constexpr int kDq = 60;   // D 2^-sp
+struct PolyX {  // 48 bytes
+    Word2 p[4];
+    int64_t p0;
+    int32_t sp, rcp_bias;  // D = d 2^(sp - 60), 1/D = R 2^-(56 + sp) (rcp_fixed): its exponent bias
+};
+static_assert(sizeof(PolyX) == 48, "three 16-byte loads");
+
+// Words of the Wilke sums: a row of a^2 over 2^row_shift times a cell's X, X/v', X/v'^2 over their largest.
+template <int KMAX>
+constexpr int kMixAq = KMAX <= 64 ? 56 : 54;  // |a^2| 2^a_shift < 2^this
+template <int KMAX>
+constexpr int kMixXq = KMAX <= 64 ? 57 : 55;  // |X| over a power of two above the largest, < 2^this
+
+struct TransportXHeader {
+    int32_t K, n_pairs, total_bytes, pw;
+    int32_t off_cond, off_visc, off_W, off_W4, off_diff, off_A2;  // polynomials, W, sqrt(W), pairs, a^2 [K][K]
+    int32_t a_shift, pad;
+    double T0, Tn_lo, Tn_hi, pad2;
+};
+
 }  // namespace cbg

@@ -108,3 +108,56 @@ def test_call_sizes(n):
     assert torch.isfinite(out).all()
     scale = out.abs().amax(dim=0)
     assert ((out[:, pick] - few).abs() <= 1e-12 * scale[pick]).all()
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+def test_transport_range_and_forms(config):
+    """Transport at the edges of its fixed-point temperatures (200 and 4,000 K), with pure, negative, zero, huge and
+    non-finite amounts, against the oracle; and a cell has the same bits in a small call (one cell per warp) as in a
+    large one (one per thread)."""
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = util.mechanism(config)
+    K = m.K
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    scales = synthetic.transport_scales(m)
+    mech.transport_setup(*scales)
+    o.set_transport(*scales, *mech.transport_coefficients())
+    cells = synthetic.generate_cells(K, 64, config, seed=33)
+    tin = np.array(o.transport_inputs(cells))  # sum n, T/T0, n_0 ..
+    T0 = scales[0]
+    edges = [150.0, np.nextafter(200.0, 0), 200.0, 300.0, 1000.0, 3000.0, np.nextafter(4000.0, 0), 4000.0, 5000.0]
+    for c, T in enumerate(edges):
+        tin[1, c] = T / T0
+    c = len(edges)
+    tin[2:, c] *= 1e-170            # subnormal products
+    tin[0, c] *= 1e-170
+    tin[2:, c + 1] *= 1e160
+    tin[0, c + 1] *= 1e160
+    tin[2, c + 2] = -0.2 * tin[0, c + 2]
+    tin[2 + K // 2, c + 3] = 0.0
+    tin[2:, c + 4] = 1e-9 * tin[0, c + 4] / K  # the bulk species but for traces
+    tin[2:, c + 5] = 1e-9 * tin[0, c + 5] / K  # species 0 but for traces
+    tin[2, c + 5] = tin[0, c + 5] * (1.0 - 1e-8)
+    dev = lambda x: torch.tensor(x, dtype=torch.float64, device="cuda")  # noqa: E731
+
+    def run(x):
+        out = torch.full((K + 2, x.shape[1]), float("nan"), dtype=torch.float64, device="cuda")
+        mech.transport(dev(x), out)
+        mech.synchronize()
+        return out.cpu().numpy()
+
+    small = run(tin)
+    ref, sc = o.transport(list(tin), nthreads=NTHREADS, scale=True)
+    assert np.array_equal(np.isfinite(small), np.isfinite(ref))
+    e = util.cond_err(small, ref, sc)
+    print(f"{config} transport: max cond err {np.nanmax(e):.2e} (cell {np.nanargmax(np.nanmax(e, 0))})")
+    assert np.nanmax(e) <= util.PLAIN_TOL
+    bad = tin.copy()
+    bad[2, 0], bad[0, 1], bad[1, 2] = np.nan, np.inf, np.nan
+    for x in (tin, bad):  # the same cells in a call of one cell per thread
+        reps = {"k10": 64, "k53": 192, "k250": 520}[config] * 152 // 64 + 1
+        large = run(np.tile(x, (1, reps)))
+        assert np.array_equal(large[:, :64], large[:, -64:], equal_nan=True)
+        assert np.array_equal(run(x), large[:, :64], equal_nan=True)
