@@ -69,11 +69,9 @@ void set_f64_tables(Args& a, const cb_mech* m) { a.f64_tab = m->d_rates; }
 template <int KM>
 void set_f64_tables(cbg::TransportArgs<KM>& a, const cb_mech* m) { a.f64_tab = m->d_transport; }
 
-template <template <int> class Args, int KM>
+template <template <int> class Args, int KM, class Launch>
 int fill_and_launch(cb_mech* m, size_t n, const double* const* in, int ni, double* const* out, int no,
-                    uint32_t flags, cudaStream_t st,
-                    cudaError_t (*launch)(int, const uint8_t*, uint32_t, const void*, size_t, cudaStream_t, int*),
-                    const uint8_t* tab, size_t tab_bytes, const char* what) {
+                    uint32_t flags, cudaStream_t st, Launch launch, const uint8_t* tab, size_t tab_bytes, const char* what) {
     Args<KM> a;
     std::memset(&a, 0, sizeof a);
     for (int q = 0; q < ni; q++) a.in[q] = in[q];
@@ -84,11 +82,9 @@ int fill_and_launch(cb_mech* m, size_t n, const double* const* in, int ni, doubl
     return e == cudaSuccess ? CB_OK : cuda_fail(e, what);
 }
 
-template <template <int> class Args>
+template <template <int> class Args, class Launch>
 int dispatch(cb_mech* m, size_t n, const double* const* in, int ni, double* const* out, int no, uint32_t flags,
-             cudaStream_t st,
-             cudaError_t (*launch)(int, const uint8_t*, uint32_t, const void*, size_t, cudaStream_t, int*),
-             const uint8_t* tab, size_t tab_bytes, const char* what) {
+             cudaStream_t st, Launch launch, const uint8_t* tab, size_t tab_bytes, const char* what) {
     switch (m->kmax) {
     case 16: return fill_and_launch<Args, 16>(m, n, in, ni, out, no, flags, st, launch, tab, tab_bytes, what);
     case 64: return fill_and_launch<Args, 64>(m, n, in, ni, out, no, flags, st, launch, tab, tab_bytes, what);
@@ -98,11 +94,16 @@ int dispatch(cb_mech* m, size_t n, const double* const* in, int ni, double* cons
 }
 
 // The plain rates: the fixed-point kernel, or the FP64 one for a mechanism out of its range.
+size_t rates_warp_bytes(const cb_mech* m) { return cbg::rates_warp_bytes(m->host.K, m->host.R, m->host.n_eff); }
 int launch_rates_path(cb_mech* m, size_t n, const double* const* in, double* const* out, uint32_t flags, cudaStream_t st) {
     const int K = m->host.K, A = m->host.A;
-    if (m->d_rates_fixed)
-        return dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, cbg::launch_rates_x, m->d_rates_fixed,
+    if (m->d_rates_fixed) {
+        auto launch = [m](int kmax, const uint8_t* tab, uint32_t bytes, const void* args, size_t cells, cudaStream_t s, int* status) {
+            return cbg::launch_rates_x(kmax, tab, bytes, args, cells, rates_warp_bytes(m), s, status);
+        };
+        return dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, launch, m->d_rates_fixed,
                                         m->host.rates_fixed_blob.size(), "rates kernel");
+    }
     return dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, cbg::launch_rates, m->d_rates,
                                     m->host.rates_blob.size(), "rates kernel");
 }
@@ -131,10 +132,14 @@ int launch_path(cb_mech* m, Path path, size_t n, const double* const* in, double
         return launch_rates_path(m, n, in, out, flags, st);
     case Path::ReactionRates:
         if (R > cbg::kMaxReactions) return fail(CB_ERR_UNSUPPORTED, "more reactions than per-reaction outputs support");
-        if (m->d_rates_fixed)
-            return dispatch<cbg::ReactionRatesArgs>(m, n, in, K + 2, out, R, flags, st, cbg::launch_reaction_rates_x,
-                                                    m->d_rates_fixed, m->host.rates_fixed_blob.size(),
-                                                    "reaction rates kernel");
+        if (m->d_rates_fixed) {
+            auto launch = [m](int kmax, const uint8_t* tab, uint32_t bytes, const void* args, size_t cells, cudaStream_t s,
+                              int* status) {
+                return cbg::launch_reaction_rates_x(kmax, tab, bytes, args, cells, rates_warp_bytes(m), s, status);
+            };
+            return dispatch<cbg::ReactionRatesArgs>(m, n, in, K + 2, out, R, flags, st, launch, m->d_rates_fixed,
+                                                    m->host.rates_fixed_blob.size(), "reaction rates kernel");
+        }
         return dispatch<cbg::ReactionRatesArgs>(m, n, in, K + 2, out, R, flags, st, cbg::launch_reaction_rates,
                                                 m->d_rates, rb, "reaction rates kernel");
     case Path::Transport:

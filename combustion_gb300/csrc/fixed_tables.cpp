@@ -248,6 +248,15 @@ bool build_rates_fixed(HostMechanism& m) {
     X.off_reactions = put(b, fx.data(), fx.size());
     X.off_falloff = put(b, ff.data(), ff.size());
     X.off_eff = put(b, ef.data(), ef.size());
+    std::vector<int32_t> start(K + 1, 0), lists;
+    for (int k = 0; k < K; k++) {
+        for (int r = 0; r < R; r++)
+            for (int i = 0; i < rx[r].n_net; i++)
+                if (rx[r].net_k[i] == k) lists.push_back((r << 8) | (rx[r].net_n[i] & 0xff));
+        start[k + 1] = (int32_t)lists.size();
+    }
+    X.off_csr_start = put(b, start.data(), start.size());
+    X.off_csr = put(b, lists.data(), lists.size());
     while (b.size() % kAlign) b.push_back(0);
     X.total_bytes = (int32_t)b.size();
     std::memcpy(b.data() + off_header, &X, sizeof X);

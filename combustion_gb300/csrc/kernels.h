@@ -127,10 +127,12 @@ cudaError_t launch_rates(int kmax, const uint8_t* tab, uint32_t tab_bytes, const
 cudaError_t launch_reaction_rates(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                   cudaStream_t st, int* status);
 // The fixed-point forms (kernels_fixed.cu); `args` carries the FP64 tables as well.
-cudaError_t launch_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
+// warp_bytes: a warp's scratch in the form of one cell per warp (rates_warp_bytes).
+cudaError_t launch_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n, size_t warp_bytes,
                            cudaStream_t st, int* status);
 cudaError_t launch_reaction_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
-                                    cudaStream_t st, int* status);
+                                    size_t warp_bytes, cudaStream_t st, int* status);
+inline size_t rates_warp_bytes(int K, int R, int n_eff) { return (4 * (size_t)K + (size_t)n_eff + (size_t)R) * sizeof(double); }
 cudaError_t launch_transport_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                cudaStream_t st, int* status);
 size_t wave_transport_x(int kmax, uint32_t tab_bytes);

@@ -29,6 +29,9 @@ struct CellX {
     long long g[KMAX];  // Gibbs energies over RT, base 2, Qy
 };
 
+// e with S < 2^e, S positive and normal.
+__device__ __forceinline__ int exponent_above_x(double S) { return ((__double2hiint(S) >> 20) & 0x7ff) - 1022; }
+
 // Prologue of reaction.rs:362-373; false where the cell needs the FP64 form.
 template <int KMAX>
 __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pressure_R, double T, double V,
@@ -50,7 +53,7 @@ __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pres
     const double S = sum > c.Ctot ? sum : c.Ctot;
     if (!(S > 1e-200 && S < 1e200 && c.Ctot > 0.0)) return false;
     c.C[K - 1] = c.Ctot - sum;
-    const int ex = ((__double2hiint(S) >> 20) & 0x7ff) - 1022;  // S < 2^ex
+    const int ex = exponent_above_x(S);
     c.m_q = H.eff_shift + 6 - ex;
     c.ctot = dbl_to_fix(c.Ctot, c.m_q);
     if (H.n_eff)
@@ -207,8 +210,277 @@ __global__ void __launch_bounds__(kRatesXBlock) reaction_rates_x_kernel(const ui
     }
 }
 
-CB_DISPATCH(launch_rates_x, rates_x_kernel, RatesArgs, kRatesXBlock, kMathBytes + kFixMathBytes, true)
-CB_DISPATCH(launch_reaction_rates_x, reaction_rates_x_kernel, ReactionRatesArgs, kRatesXBlock, kMathBytes + kFixMathBytes, true)
+// ---------------------------------------------------------------------------------------------------
+// One cell per warp, for calls too small to fill the GPU with one per thread: lanes share out species, third-body
+// rows and reactions; every FP64 sum runs on one lane in the thread form's order (the integer sums are exact), so that
+// a cell has the same bits in both forms.
+constexpr int kRatesWarps = 16;  // cells per block at most
+
+template <int KMAX>
+struct CellXW {
+    TempsX t;
+    double rcpT, Ctot;
+    long long ctot;
+    int m_q;
+    const double* C;
+    const long long* g;
+};
+
+// The cell's rates of progress into cR [R] (grouped order); the concentrations stay in sh, followed by two free arrays
+// of K doubles and the species rates'. False where the cell needs the FP64 form (warp-uniform).
+template <int KMAX>
+__device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, double pressure_R, double T, double V,
+                                                   const double* const* amounts, size_t i, double* sh, int lane,
+                                                   CellXW<KMAX>& c) {
+    const RatesXHeader& H = *tb.H;
+    const int K = H.K, A = H.A;
+    if (!(T >= kFixTmin && T < kFixTmax)) return false;
+    double* C = sh;
+    double* cw = sh + K;
+    long long* g = reinterpret_cast<long long*>(sh + 2 * K);
+    double* M = sh + 4 * K;
+    double* cR = M + H.n_eff;
+    const double md = __drcp_rn(V);
+    c.rcpT = __drcp_rn(T);
+    for (int k = lane; k < K - 1; k += 32) C[k] = __dmul_rn(md, max0(amounts[k][i]));
+    __syncwarp();
+    double sum = 0.0;
+    if (lane == 0) {
+#pragma unroll 4
+        for (int k = 0; k < K - 1; k++) sum += C[k];
+    }
+    sum = __shfl_sync(0xffffffffu, sum, 0);
+    c.Ctot = __dmul_rn(pressure_R, c.rcpT);
+    const double S = sum > c.Ctot ? sum : c.Ctot;
+    if (!(S > 1e-200 && S < 1e200 && c.Ctot > 0.0)) return false;
+    if (lane == 0) C[K - 1] = c.Ctot - sum;
+    __syncwarp();
+    const int ex = exponent_above_x(S);
+    c.m_q = H.eff_shift + 6 - ex;
+    c.ctot = dbl_to_fix(c.Ctot, c.m_q);
+    c.t = make_temps(H, T, c.rcpT);
+    c.C = C;
+    c.g = g;
+    for (int k = lane; k < K; k += 32) {
+        const Word2 w = split_word(dbl_to_fix(C[k], kCq + kLo - ex));
+        cw[k] = __hiloint2double(w.hi, w.lo);
+        if (k < A && (tb.species[k].need_exp | tb.species[k].need_exp_neg)) g[k] = gibbs_log2(tb.species[k], c.t);
+    }
+    __syncwarp();
+    for (int e = lane; e < H.n_eff; e += 32) {
+        const Word2* E = tb.eff + (size_t)e * K;
+        long long s1 = 0, s2 = 0;
+#pragma unroll 4
+        for (int k = 0; k < K; k++) dot_term(E[k], Word2{__double2hiint(cw[k]), __double2loint(cw[k])}, s1, s2);
+        M[e] = third_body(c, s1, s2);
+    }
+    __syncwarp();
+    const int first = H.group_end[1];
+#pragma unroll 1
+    for (int m = 0; m < 6; m++) {  // one model's program at a time
+#pragma unroll 1
+        for (int r = (m ? H.group_end[m - 1] : 0) + lane; r < H.group_end[m]; r += 32) {
+            auto store = [&](int, double v) { cR[r] = v; };
+            if (m == 1) {
+                reaction_x<false, false>(tb, r, c, nullptr, [&](const ArrheniusX& k) { return rate_constant(k, c.t); }, store);
+            } else {
+                auto forward = [&](const ArrheniusX& k) {
+                    if (m == 0) return rate_constant(k, c.t);
+                    const FalloffX* f = tb.falloff + (r - first);
+                    if (m == 2) return forward_x<2>(H, k, f, c.t, c.rcpT, M[r - first]);
+                    if (m == 3) return forward_x<3>(H, k, f, c.t, c.rcpT, M[r - first]);
+                    if (m == 4) return forward_x<4>(H, k, f, c.t, c.rcpT, M[r - first]);
+                    return forward_x<5>(H, k, f, c.t, c.rcpT, M[r - first]);
+                };
+                reaction_x<true, false>(tb, r, c, nullptr, forward, store);
+            }
+        }
+    }
+    __syncwarp();
+    return true;
+}
+
+template <int KMAX>
+__device__ __forceinline__ bool rates_cell_warp(const RatesXTables& tb, const RatesArgs<KMAX>& io, size_t i, double* sh,
+                                                int lane) {
+    const RatesXHeader& H = *tb.H;
+    const int K = H.K, A = H.A;
+    const bool uniform = io.flags & kUniformPressure;
+    const double T = io.in[2][i], V = io.in[3][i];
+    CellXW<KMAX> c;
+    if (!cell_progress_warp<KMAX>(tb, uniform ? io.in[0][0] : io.in[0][i], T, V, io.in + 4, i, sh, lane, c)) return false;
+    double *C = sh, *h = sh + K, *cp = sh + 2 * K, *w = sh + 3 * K, *cR = sh + 4 * K + H.n_eff;
+    for (int k = lane; k < K; k += 32) {
+        if (k < A) {
+            double v = 0.0;
+            const int end = tb.csr_start[k + 1];
+#pragma unroll 4
+            for (int q = tb.csr_start[k]; q < end; q++) {
+                const int e = tb.csr[q];
+                v = fma(small_int_to_double((int)(int8_t)(e & 0xff)), cR[e >> 8], v);
+            }
+            w[k] = v;
+            io.out[2 + k][i] = v;
+        }
+        const ThermoX& s = tb.thermo[k];
+        const int set = piece_x(s.split, T);
+        if (k < A) h[k] = enthalpy_x(s, set, c.t);
+        cp[k] = heat_capacity_x(s, set, c.t);
+    }
+    __syncwarp();
+    double acc = 0.0;  // E, Cp and dtE on lanes 0, 1, 2
+    if (lane < 3) {
+        const int n = lane == 1 ? K : A;
+#pragma unroll 4
+        for (int k = 0; k < n; k++)
+            acc = fma(lane == 0 ? w[k] : lane == 1 ? cp[k] : tb.thermo[k].dtE, lane == 0 ? h[k] : lane == 1 ? C[k] : w[k], acc);
+    }
+    const double E = __shfl_sync(0xffffffffu, acc, 0), Cp = __shfl_sync(0xffffffffu, acc, 1),
+                 dtE = __shfl_sync(0xffffffffu, acc, 2);
+    if (lane == 0) {
+        const double dtT_T = div64(-E, Cp), rcp_pressure_R = uniform ? io.in[1][0] : io.in[1][i];
+        io.out[0][i] = T * dtT_T;
+        io.out[1][i] = V * fma(rcp_pressure_R * T, dtE, dtT_T);
+    }
+    __syncwarp();  // the scratch is the warp's next cell's
+    return true;
+}
+
+template <int KMAX>
+__device__ __forceinline__ bool reaction_rates_cell_warp(const RatesXTables& tb, const ReactionRatesArgs<KMAX>& io, size_t i,
+                                                         double* sh, int lane) {
+    CellXW<KMAX> c;
+    if (!cell_progress_warp<KMAX>(tb, io.in[0][i], io.in[1][i], io.in[2][i], io.in + 3, i, sh, lane, c)) return false;
+    const double* cR = sh + 4 * tb.H->K + tb.H->n_eff;
+    for (int r = lane; r < tb.H->R; r += 32) io.out[tb.reactions[r].orig][i] = cR[r];
+    __syncwarp();
+    return true;
+}
+
+// The warp's cells; those that need the FP64 form are put off until there are 32, one per lane.
+template <bool SMEM, class Cell, class F64>
+__device__ __forceinline__ void warp_cells(const uint8_t* gtab, uint32_t tab_bytes, size_t n, int* status, Cell cell, F64 f64) {
+    __shared__ uint64_t bar;
+    if (!stage_x<SMEM>(gtab, tab_bytes, &bar, status)) return;
+    const RatesXTables tb(SMEM ? cb_dsmem : gtab);
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const uint32_t tables = SMEM ? tab_bytes : (uint32_t)(kMathBytes + kFixMathBytes);
+    double* sh = reinterpret_cast<double*>(cb_dsmem + tables) +
+                 (size_t)(threadIdx.x >> 5) * (4 * tb.H->K + tb.H->n_eff + tb.H->R);  // rates_warp_bytes
+    size_t later = 0;
+    int put_off = 0;
+    for (size_t i = (size_t)blockIdx.x * warps + (threadIdx.x >> 5); i < n; i += (size_t)gridDim.x * warps) {
+        if (cell(tb, i, sh, lane)) continue;
+        __syncwarp();
+        if (lane == put_off) later = i;
+        if (++put_off == 32) {
+            f64(later);
+            __syncwarp();
+            put_off = 0;
+        }
+    }
+    if (lane < put_off) f64(later);
+}
+
+template <int KMAX, bool SMEM>
+__global__ void __launch_bounds__(32 * kRatesWarps) rates_x_warp_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
+                                                                      const __grid_constant__ RatesArgs<KMAX> io, size_t n,
+                                                                      int* status) {
+    warp_cells<SMEM>(
+        gtab, tab_bytes, n, status,
+        [&](const RatesXTables& tb, size_t i, double* sh, int lane) { return rates_cell_warp<KMAX>(tb, io, i, sh, lane); },
+        [&](size_t i) { rates_cell_f64<KMAX>(io, i); });
+}
+template <int KMAX, bool SMEM>
+__global__ void __launch_bounds__(32 * kRatesWarps)
+    reaction_rates_x_warp_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
+                                 const __grid_constant__ ReactionRatesArgs<KMAX> io, size_t n, int* status) {
+    warp_cells<SMEM>(
+        gtab, tab_bytes, n, status,
+        [&](const RatesXTables& tb, size_t i, double* sh, int lane) {
+            return reaction_rates_cell_warp<KMAX>(tb, io, i, sh, lane);
+        },
+        [&](size_t i) { reaction_rates_cell_f64<KMAX>(io, i); });
+}
+
+namespace {
+// Calls of up to this many cells per SM go one cell per warp. A thread's cell takes 60, 500 and 5,000 us however few
+// there are (10, 53, 250 species), a warp's 34, 66 and 410 us and then 12, 24 and 360 ns per cell (bound by the FP64
+// chains that run on one lane); beyond these lines the thread form is the faster.
+template <int KMAX>
+constexpr size_t kWarpCellsPerSmR = KMAX == 16 ? 32 : KMAX == 64 ? 150 : 100;
+
+// As many warps as fit beside the tables (or, of a large mechanism, beside the functions' tables).
+template <class KS, class KG, class Args>
+cudaError_t launch_rates_warp(KS ksmem, KG kglobal, const uint8_t* tab, uint32_t tab_bytes, const Args& io, size_t n,
+                              size_t warp_bytes, cudaStream_t st, int* status) {
+    const size_t share = (n + sm_count() - 1) / sm_count();
+    const uint32_t math = kMathBytes + kFixMathBytes;
+    const bool smem = tab_bytes + 2 * warp_bytes <= (size_t)max_table_smem();
+    int warps = share < (size_t)kRatesWarps ? (int)share : kRatesWarps;
+    while (warps > 1 && (smem ? tab_bytes : math) + warps * warp_bytes > (size_t)max_table_smem()) warps--;
+    const size_t bytes = (smem ? tab_bytes : math) + warps * warp_bytes;
+    if (bytes > (size_t)max_table_smem()) return cudaErrorInvalidConfiguration;
+    cudaError_t e = smem ? cudaFuncSetAttribute(ksmem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
+                         : cudaFuncSetAttribute(kglobal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    int per_sm = 1;
+    if (smem) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ksmem, 32 * warps, bytes);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kglobal, 32 * warps, bytes);
+    if (per_sm < 1) per_sm = 1;
+    size_t grid = (size_t)sm_count() * per_sm;
+    const size_t want = (n + warps - 1) / warps;
+    if (want < grid) grid = want;
+    if (smem) ksmem<<<(unsigned)grid, 32 * warps, bytes, st>>>(tab, tab_bytes, io, n, status);
+    else kglobal<<<(unsigned)grid, 32 * warps, bytes, st>>>(tab, tab_bytes, io, n, status);
+    return cudaGetLastError();
+}
+
+template <int KMAX>
+cudaError_t launch_rates_xk(const uint8_t* tab, uint32_t tab_bytes, const RatesArgs<KMAX>& io, size_t n, size_t warp_bytes,
+                            cudaStream_t st, int* status) {
+    if (n <= (size_t)sm_count() * kWarpCellsPerSmR<KMAX> && 4 * warp_bytes + 32768 <= (size_t)max_table_smem())
+        return launch_rates_warp(rates_x_warp_kernel<KMAX, true>, rates_x_warp_kernel<KMAX, false>, tab, tab_bytes, io, n,
+                                 warp_bytes, st, status);
+    return launch_table_kernel<kRatesXBlock>(rates_x_kernel<KMAX, true>, rates_x_kernel<KMAX, false>, tab, tab_bytes, io, n,
+                                             kMathBytes + kFixMathBytes, true, st, status);
+}
+template <int KMAX>
+cudaError_t launch_reaction_rates_xk(const uint8_t* tab, uint32_t tab_bytes, const ReactionRatesArgs<KMAX>& io, size_t n,
+                                     size_t warp_bytes, cudaStream_t st, int* status) {
+    if (n <= (size_t)sm_count() * kWarpCellsPerSmR<KMAX> && 4 * warp_bytes + 32768 <= (size_t)max_table_smem())
+        return launch_rates_warp(reaction_rates_x_warp_kernel<KMAX, true>, reaction_rates_x_warp_kernel<KMAX, false>, tab,
+                                 tab_bytes, io, n, warp_bytes, st, status);
+    return launch_table_kernel<kRatesXBlock>(reaction_rates_x_kernel<KMAX, true>, reaction_rates_x_kernel<KMAX, false>, tab,
+                                             tab_bytes, io, n, kMathBytes + kFixMathBytes, true, st, status);
+}
+}  // namespace
+
+cudaError_t launch_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n, size_t warp_bytes,
+                           cudaStream_t st, int* status) {
+    switch (kmax) {
+    case 16: return launch_rates_xk<16>(tab, tab_bytes, *static_cast<const RatesArgs<16>*>(args), n, warp_bytes, st, status);
+    case 64: return launch_rates_xk<64>(tab, tab_bytes, *static_cast<const RatesArgs<64>*>(args), n, warp_bytes, st, status);
+    case 256:
+        return launch_rates_xk<256>(tab, tab_bytes, *static_cast<const RatesArgs<256>*>(args), n, warp_bytes, st, status);
+    default: return cudaErrorInvalidValue;
+    }
+}
+cudaError_t launch_reaction_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
+                                    size_t warp_bytes, cudaStream_t st, int* status) {
+    switch (kmax) {
+    case 16:
+        return launch_reaction_rates_xk<16>(tab, tab_bytes, *static_cast<const ReactionRatesArgs<16>*>(args), n, warp_bytes,
+                                            st, status);
+    case 64:
+        return launch_reaction_rates_xk<64>(tab, tab_bytes, *static_cast<const ReactionRatesArgs<64>*>(args), n, warp_bytes,
+                                            st, status);
+    case 256:
+        return launch_reaction_rates_xk<256>(tab, tab_bytes, *static_cast<const ReactionRatesArgs<256>*>(args), n, warp_bytes,
+                                             st, status);
+    default: return cudaErrorInvalidValue;
+    }
+}
 CB_WAVE(wave_rates_x, rates_x_kernel, kRatesXBlock, kMathBytes + kFixMathBytes)
 CB_WAVE(wave_reaction_rates_x, reaction_rates_x_kernel, kRatesXBlock, kMathBytes + kFixMathBytes)
 

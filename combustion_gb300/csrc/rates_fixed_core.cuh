@@ -19,13 +19,16 @@ struct RatesXTables {
     const ReactionX* reactions;
     const FalloffX* falloff;
     const Word2* eff;
+    const int32_t *csr_start, *csr;
     __device__ explicit RatesXTables(const uint8_t* tab)
         : H(reinterpret_cast<const RatesXHeader*>(tab + kMathBytes + kFixMathBytes)),
           species(reinterpret_cast<const SpeciesX*>(tab + H->off_species)),
           thermo(reinterpret_cast<const ThermoX*>(tab + H->off_thermo)),
           reactions(reinterpret_cast<const ReactionX*>(tab + H->off_reactions)),
           falloff(reinterpret_cast<const FalloffX*>(tab + H->off_falloff)),
-          eff(reinterpret_cast<const Word2*>(tab + H->off_eff)) {}
+          eff(reinterpret_cast<const Word2*>(tab + H->off_eff)),
+          csr_start(reinterpret_cast<const int32_t*>(tab + H->off_csr_start)),
+          csr(reinterpret_cast<const int32_t*>(tab + H->off_csr)) {}
 };
 
 // A cell's temperature in fixed point.

@@ -95,6 +95,7 @@ struct ThermoX {
 
 struct RatesXHeader {
     int32_t K, A, R, n_eff, total_bytes, off_species, off_thermo, off_reactions, off_falloff, off_eff;
+    int32_t off_csr_start, off_csr;  // per species the reactions that change it, in order: [K + 1]; r << 8 | nu
     int32_t group_end[6];
     int64_t lM3, lcbrt, lC0;  // log2 of the Gibbs exponentials' caps and of P0 / R, Qy
     int32_t eff_shift;        // efficiency words are (e - 1) 2^eff_shift, eff_shift <= kEffBits

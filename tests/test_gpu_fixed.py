@@ -161,3 +161,30 @@ def test_transport_range_and_forms(config):
         large = run(np.tile(x, (1, reps)))
         assert np.array_equal(large[:, :64], large[:, -64:], equal_nan=True)
         assert np.array_equal(run(x), large[:, :64], equal_nan=True)
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+@pytest.mark.parametrize("make", [util.mechanism, shapes_mechanism], ids=["generator", "shapes"])
+def test_rates_small_calls_match_large_ones(config, make):
+    """A cell has the same bits in a small call (one cell per warp) as in a large one (one per thread), those that
+    take the FP64 form among them (more than a warp's worth)."""
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = make(config)
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    cells = edge_temperatures(config, 48)
+    rin, pin = np.array(o.rates_inputs(cells)), np.array(o.reaction_rates_inputs(cells))
+    rin[4, 20] = np.nan
+    rin[0, 21] = pin[0, 21] = 0.0
+    dev = lambda x: torch.tensor(x, dtype=torch.float64, device="cuda")  # noqa: E731
+    reps = {"k10": 64, "k53": 400, "k250": 400}[config] * 152 // 48 + 1
+    for call, x, rows in ((mech.rates, rin, mech.A + 2), (mech.reaction_rates, pin, mech.R)):
+        out = {}
+        for r in (1, 40, reps):
+            t = torch.full((rows, 48 * r), float("nan"), dtype=torch.float64, device="cuda")
+            call(dev(np.tile(x, (1, r))), t)
+            mech.synchronize()
+            out[r] = t[:, -48:].cpu().numpy()
+        assert np.array_equal(out[1], out[40], equal_nan=True)
+        assert np.array_equal(out[1], out[reps], equal_nan=True)
