@@ -9,7 +9,7 @@ import ctypes as C
 
 import numpy as np
 
-from . import CombustionError, Mechanism, _check, _ptr_array, lib
+from . import CombustionError, Mechanism, _address, _check, _row_pointers, lib
 
 CB_UNIFORM_PRESSURE = 2
 CB_SURROGATE_NO_GATE = 8
@@ -99,8 +99,8 @@ def generate_cells(mech: Mechanism, n: int, dist: cb_cell_distribution, offset: 
     import torch
     L = _bind()
     out = torch.empty((mech.K + 3, n), dtype=torch.float64, device="cuda")
-    rows, _ = Mechanism._rows(out)
-    _check(L.cb_generate_cells(mech.h, n, offset, C.byref(dist), _ptr_array(rows), Mechanism._stream(stream)))
+    rows, _ = _row_pointers(out)
+    _check(L.cb_generate_cells(mech.h, n, offset, C.byref(dist), _address(rows), Mechanism._stream(stream)))
     return out
 
 
@@ -186,12 +186,12 @@ class Surrogate:
     def transport(self, inputs, outputs, audit_stride=1024, gate=True, uniform_pressure=False, stream=None,
                   timing=False):
         """Rates-layout inputs [K+3, n] -> transport outputs [K+2, n] (torch CUDA float64). Returns stats."""
-        ins, _ = Mechanism._rows(inputs)
-        outs, n = Mechanism._rows(outputs)
+        ins, _ = _row_pointers(inputs)
+        outs, n = _row_pointers(outputs)
         flags = (0 if gate else CB_SURROGATE_NO_GATE) | (CB_UNIFORM_PRESSURE if uniform_pressure else 0)
         flags |= CB_SURROGATE_TIMING if timing else 0
         st = cb_surrogate_stats()
-        _check(lib().cb_surrogate_transport(self.h, n, _ptr_array(ins), _ptr_array(outs), flags, audit_stride,
+        _check(lib().cb_surrogate_transport(self.h, n, _address(ins), _address(outs), flags, audit_stride,
                                             C.byref(st), Mechanism._stream(stream)))
         return st.as_dict()
 
@@ -203,8 +203,8 @@ def transport_pair(a: Surrogate, b: Surrogate, inputs, outputs, threshold: float
     the training range) go to the mixed ("mixed") or plain ("plain") kernel. `disagreement` (torch CUDA
     float32 [n]) receives each cell's estimate. Returns the stats."""
     L = _bind()
-    ins, _ = Mechanism._rows(inputs)
-    outs, n = Mechanism._rows(outputs)
+    ins, _ = _row_pointers(inputs)
+    outs, n = _row_pointers(outputs)
     flags = (CB_UNIFORM_PRESSURE if uniform_pressure else 0) | (CB_SURROGATE_TIMING if timing else 0)
     d_ptr = None
     if disagreement is not None:
@@ -214,7 +214,7 @@ def transport_pair(a: Surrogate, b: Surrogate, inputs, outputs, threshold: float
     g = cb_surrogate_gate(float(threshold), int(audit_stride),
                           {"mixed": CB_FALLBACK_MIXED, "plain": CB_FALLBACK_PLAIN}[fallback], d_ptr)
     st = cb_surrogate_stats()
-    _check(L.cb_surrogate_transport_pair(a.h, b.h, n, _ptr_array(ins), _ptr_array(outs), flags, C.byref(g),
+    _check(L.cb_surrogate_transport_pair(a.h, b.h, n, _address(ins), _address(outs), flags, C.byref(g),
                                          C.byref(st), Mechanism._stream(stream)))
     return st.as_dict()
 
