@@ -345,7 +345,9 @@ bool build_transport_fixed(HostMechanism& m) {
     while (std::ldexp(largest, X.a_shift) >= std::ldexp(1.0, bits)) X.a_shift--;
     while (std::ldexp(largest, X.a_shift + 1) < std::ldexp(1.0, bits)) X.a_shift++;
     std::vector<Word2> a2((size_t)K * K);
-    for (size_t i = 0; i < a2.size(); i++) a2[i] = words((int64_t)std::llround(std::ldexp((long double)A2[i], X.a_shift)));
+    for (int k = 0; k < K; k++)
+        for (int j = 0; j < K; j++)
+            a2[(size_t)j * K + k] = words((int64_t)std::llround(std::ldexp((long double)A2[(size_t)k * K + j], X.a_shift)));
 
     std::vector<uint8_t>& b = m.transport_fixed_blob;
     b.insert(b.end(), blob, blob + kMathBytes);

@@ -111,14 +111,15 @@ constexpr int kLpq = 29;  // (L / 2^pw)^m, hi word
 constexpr int kPpq = 28;  // its coefficient, |.| < 4
 constexpr int kPlo = 30;  // bits of their low words
 constexpr int kDq = 60;   // D 2^-sp
-struct PolyX {  // 48 bytes
+struct alignas(16) PolyX {  // three 16-byte loads
     Word2 p[4];
     int64_t p0;
     int32_t sp, rcp_bias;  // D = d 2^(sp - 60), 1/D = R 2^-(56 + sp) (rcp_fixed): its exponent bias
 };
 static_assert(sizeof(PolyX) == 48, "three 16-byte loads");
 
-// Words of the Wilke sums: a row of a^2 over 2^row_shift times a cell's X, X/v', X/v'^2 over their largest.
+// Words of the Wilke sums: a^2 (column j: the rows k, so that rows in registers or lanes read consecutive words) times
+// a cell's X, X/v', X/v'^2 over their largest.
 template <int KMAX>
 constexpr int kMixAq = KMAX <= 64 ? 56 : 54;  // |a^2| 2^a_shift < 2^this
 template <int KMAX>
@@ -126,7 +127,7 @@ constexpr int kMixXq = KMAX <= 64 ? 57 : 55;  // |X| over a power of two above t
 
 struct TransportXHeader {
     int32_t K, n_pairs, total_bytes, pw;
-    int32_t off_cond, off_visc, off_W, off_W4, off_diff, off_A2;  // polynomials, W, sqrt(W), pairs, a^2 [K][K]
+    int32_t off_cond, off_visc, off_W, off_W4, off_diff, off_A2;  // polynomials, W, sqrt(W), pairs, a^2 by columns
     int32_t a_shift, pad;
     double T0, Tn_lo, Tn_hi, pad2;
 };

@@ -17,12 +17,12 @@
 
 namespace cbg {
 
-// Rows k0 .. k0 + Q - 1 of Wilke's sums and their terms of mu, in row order.
+// Rows k0 .. k0 + Q - 1 of Wilke's sums and their terms of mu (rows k0, k0 + 2 in mu0, the others in mu1).
 template <int Q>
-__device__ __forceinline__ double wilke_rows_x(const TransportXTables& tb, int K, int k0, const double* X, const double* r,
+__device__ __forceinline__ void wilke_rows_x(const TransportXTables& tb, int K, int k0, const double* X, const double* r,
                                                const double* Xw, const double* Yw, const double* Zw, int q1, int q2,
-                                               int q3, double mu) {
-    const Word2* a = tb.A2 + (size_t)k0 * K;
+                                               int q3, double& mu0, double& mu1) {
+    const Word2* a = tb.A2 + k0;
     long long s[Q][3], t[Q][3];
 #pragma unroll
     for (int q = 0; q < Q; q++)
@@ -41,19 +41,20 @@ __device__ __forceinline__ double wilke_rows_x(const TransportXTables& tb, int K
         }
 #pragma unroll
         for (int q = 0; q < Q; q++) {
-            const Word2 w = a[q * K + j];
+            const Word2 w = a[(size_t)j * K + q];
             dot_term(w, x, s[q][0], t[q][0]);
             dot_term(w, y, s[q][1], t[q][1]);
             dot_term(w, z, s[q][2], t[q][2]);
         }
     }
 #pragma unroll
-    for (int q = 0; q < Q; q++)
-        mu = fma(wilke_factor(X[k0 + q], tb.W4[k0 + q]),
-                 wilke_rcp(mix_value(s[q][0], t[q][0]), mix_value(s[q][1], t[q][1]), mix_value(s[q][2], t[q][2]), q1, q2, q3,
-                           r[k0 + q]),
-                 mu);
-    return mu;
+    for (int q = 0; q < Q; q++) {
+        const double w = wilke_factor(X[k0 + q], tb.W4[k0 + q]),
+                     d = wilke_rcp(mix_value(s[q][0], t[q][0]), mix_value(s[q][1], t[q][1]), mix_value(s[q][2], t[q][2]), q1,
+                                   q2, q3, r[k0 + q]);
+        if (q & 1) mu1 = fma(w, d, mu1);
+        else mu0 = fma(w, d, mu0);
+    }
 }
 
 // Rows k0 .. k0 + Q - 1 of the diffusion pairs: S_k = sum over j < k of X_j / D_kj (even and odd j apart), and X_k / D_kj
@@ -79,7 +80,8 @@ __device__ __forceinline__ void diffusion_rows(const TransportXTables& tb, int k
             double sj = S[j + h];
 #pragma unroll
             for (int q = 0; q < Q; q++) {
-                const double R = rcp_fixed(poly_x(P[q][j + h], L), P[q][j + h].rcp_bias);
+                const PolyX p = P[q][j + h];
+                const double R = rcp_fixed(poly_x(p, L), p.rcp_bias);
                 if (h) t[q] = fma(xj, R, t[q]);
                 else s[q] = fma(xj, R, s[q]);
                 sj = fma(x[q], R, sj);
@@ -91,7 +93,8 @@ __device__ __forceinline__ void diffusion_rows(const TransportXTables& tb, int k
     for (int q = 0; q < Q; q++) {
 #pragma unroll
         for (int i = 0; i < q; i++) {
-            const double R = rcp_fixed(poly_x(P[q][k0 + i], L), P[q][k0 + i].rcp_bias);
+            const PolyX p = P[q][k0 + i];
+            const double R = rcp_fixed(poly_x(p, L), p.rcp_bias);
             if (i & 1) t[q] = fma(x[i], R, t[q]);
             else s[q] = fma(x[i], R, s[q]);
             s[i] = fma(x[q], R, s[i]);  // row i's own sum is complete
@@ -135,7 +138,7 @@ __device__ __forceinline__ bool transport_cell_x(const TransportXTables& tb, con
     // Conductivity (transport.rs:141-146).
     double A0 = 0.0, B0 = 0.0, A1 = 0.0, B1 = 0.0;
     auto conductivity = [&](int k, double& A, double& B) {
-        const PolyX& P = tb.cond[k];
+        const PolyX P = tb.cond[k];
         const long long d = poly_x(P, L);
         const double x = X[k];
         A = fma(x, fix_to_dbl(d, kDq - P.sp), A);
@@ -152,7 +155,7 @@ __device__ __forceinline__ bool transport_cell_x(const TransportXTables& tb, con
     // 1 / v'_k, and X, X / v', X / v'^2 as words
     int my = 0, mz = 0;
     for (int k = 0; k < K; k++) {
-        const PolyX& P = tb.visc[k];
+        const PolyX P = tb.visc[k];
         r[k] = rcp_fixed(poly_x(P, L), P.rcp_bias);
         Y[k] = __dmul_rn(X[k], r[k]);
         Z[k] = __dmul_rn(Y[k], r[k]);
@@ -177,12 +180,13 @@ __device__ __forceinline__ bool transport_cell_x(const TransportXTables& tb, con
     for (int part = 0; part < 2; part++) {
         int k = 0;
         if ((part == 0) != swap) {  // viscosity (transport.rs:148-158)
-            double mu = 0.0;
+            double mu0 = 0.0, mu1 = 0.0;  // even and odd species
 #pragma unroll 1
-            for (; k + 4 <= K; k += 4) mu = wilke_rows_x<4>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu);
+            for (; k + 4 <= K; k += 4) wilke_rows_x<4>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu0, mu1);
 #pragma unroll 1
-            for (; k < K; k++) mu = wilke_rows_x<1>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu);
-            io.out[1][o] = VT * mu;
+            for (; k + 2 <= K; k += 2) wilke_rows_x<2>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu0, mu1);
+            if (k < K) wilke_rows_x<1>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu0, mu1);
+            io.out[1][o] = VT * (mu0 + mu1);
         } else {  // mixture-averaged diffusion (transport.rs:162-177)
 #pragma unroll 1
             for (; k + 4 <= K; k += 4) diffusion_rows<4>(tb, k, L, X, S);
@@ -256,7 +260,7 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
     const PowersX L = log_powers(H, Tn);
     const double VT = sqrt(Tn);
     for (int k = lane; k < K; k += 32) {
-        const PolyX& P = tb.cond[k];
+        const PolyX P = tb.cond[k];
         const long long d = poly_x(P, L);
         v[k] = fix_to_dbl(d, kDq - P.sp);
         Y[k] = rcp_fixed(d, P.rcp_bias);
@@ -277,7 +281,7 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
 
     int my = 0, mz = 0;
     for (int k = lane; k < K; k += 32) {
-        const PolyX& P = tb.visc[k];
+        const PolyX P = tb.visc[k];
         v[k] = rcp_fixed(poly_x(P, L), P.rcp_bias);  // 1 / v'
         Y[k] = __dmul_rn(X[k], v[k]);
         Z[k] = __dmul_rn(Y[k], v[k]);
@@ -301,11 +305,11 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
     const int unit = H.a_shift + 1 - 2 * kLo;
 #pragma unroll 1
     for (int k = lane; k < K; k += 32) {
-        const Word2* a = tb.A2 + (size_t)k * K;
+        const Word2* a = tb.A2 + k;
         long long s[3] = {0, 0, 0}, t[3] = {0, 0, 0};
 #pragma unroll 2
         for (int j = 0; j < K; j++) {
-            const Word2 w = a[j];
+            const Word2 w = a[(size_t)j * K];
             dot_term(w, Word2{__double2hiint(Xw[j]), __double2loint(Xw[j])}, s[0], t[0]);
             dot_term(w, Word2{__double2hiint(Y[j]), __double2loint(Y[j])}, s[1], t[1]);
             dot_term(w, Word2{__double2hiint(Z[j]), __double2loint(Z[j])}, s[2], t[2]);
@@ -315,44 +319,53 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
                                  unit + qz, v[k]);
     }
     __syncwarp();
-    if (lane == 0) {
-        double mu = 0.0;
+    double mu = 0.0;
+    if (lane < 2) {
 #pragma unroll 4
-        for (int k = 0; k < K; k++) mu = fma(U[2 * k], U[2 * k + 1], mu);
-        io.out[1][o] = VT * mu;
+        for (int k = lane; k < K; k += 2) mu = fma(U[2 * k], U[2 * k + 1], mu);
     }
+    mu += __shfl_sync(0xffffffffu, mu, 1);
+    if (lane == 0) io.out[1][o] = VT * mu;
     __syncwarp();
 
+    // Diffusion, in tiles of 32 rows by 32 columns of pairs: lanes on consecutive pairs of a row (consecutive table
+    // records) leave the reciprocals in the tile, then lanes on rows add theirs, then lanes on columns.
     double* S = Y;
 #pragma unroll 1
     for (int b = 0; 32 * b < K; b++) {
-        const int r = 32 * b + lane;
-        const PolyX* P = tb.diff + ((size_t)r * (size_t)(r > 0 ? r - 1 : 0) / 2);  // pair (r, 0)
-        const int rows = min(32, K - 32 * b);
+        const int r = 32 * b + lane, rows = min(32, K - 32 * b);
         double sa = 0.0, sb = 0.0;
 #pragma unroll 1
         for (int t = 0; t <= b; t++) {
-            const int j0 = 32 * t;
-            const int j1 = r < K ? min(j0 + 32, r) : j0;
-            double* Trow = T + 33 * lane;
-            int j = j0;
+            const int j0 = 32 * t, jc = j0 + lane;
+            const PolyX* P = tb.diff + (size_t)(32 * b) * (32 * b - 1) / 2 + jc;  // pair (32 b, jc); row k + 1 is k records on
+            if (t < b) {
+#pragma unroll 4
+                for (int q = 0; q < rows; q++) {
+                    const PolyX p = P[(size_t)q * (32 * b) + q * (q - 1) / 2];
+                    T[33 * q + lane] = rcp_fixed(poly_x(p, L), p.rcp_bias);
+                }
+            } else {
 #pragma unroll 1
-            for (; j + 1 < j1; j += 2) {
-                const double Ra = rcp_fixed(poly_x(P[j], L), P[j].rcp_bias),
-                             Rb = rcp_fixed(poly_x(P[j + 1], L), P[j + 1].rcp_bias);
-                sa = fma(X[j], Ra, sa);
-                sb = fma(X[j + 1], Rb, sb);
-                Trow[j - j0] = Ra;
-                Trow[j + 1 - j0] = Rb;
+                for (int q = 1; q < rows; q++) {
+                    if (lane < q) {
+                        const PolyX p = P[(size_t)q * (32 * b) + q * (q - 1) / 2];
+                        T[33 * q + lane] = rcp_fixed(poly_x(p, L), p.rcp_bias);
+                    }
+                }
             }
-            if (j < j1) {
-                const double R = rcp_fixed(poly_x(P[j], L), P[j].rcp_bias);
-                sa = fma(X[j], R, sa);
-                Trow[j - j0] = R;
+            __syncwarp();
+            const int columns = r < K ? min(32, r - j0) : 0;  // j0 is even: even columns in sa, odd ones in sb
+            const double* Trow = T + 33 * lane;
+            int c = 0;
+#pragma unroll 4
+            for (; c + 1 < columns; c += 2) {
+                sa = fma(X[j0 + c], Trow[c], sa);
+                sb = fma(X[j0 + c + 1], Trow[c + 1], sb);
             }
+            if (c < columns) sa = fma(X[j0 + c], Trow[c], sa);
             if (t == b && r < K) S[r] = sa + sb;
             __syncwarp();
-            const int jc = j0 + lane;
             if (jc < K) {
                 double s = S[jc];
 #pragma unroll 4
@@ -366,13 +379,15 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
     return true;
 }
 
+constexpr int kWarpCellWarpsX = 16;  // cells per block, as many as fit in shared memory
+
 template <int KMAX>
 __device__ __noinline__ void transport_cell_f64_warp(const TransportArgs<KMAX>& io, size_t i, size_t o, double* sh) {
     transport_cell_warp<KMAX>(io.f64_tab, io, i, o, sh);
 }
 
 template <int KMAX, bool SMEM>
-__global__ void __launch_bounds__(32 * kWarpCellWarps) transport_x_warp_kernel(const uint8_t* __restrict__ gtab,
+__global__ void __launch_bounds__(32 * kWarpCellWarpsX) transport_x_warp_kernel(const uint8_t* __restrict__ gtab,
                                                                              uint32_t tab_bytes,
                                                                              const __grid_constant__ TransportArgs<KMAX> io,
                                                                              size_t n, int* status) {
@@ -399,20 +414,20 @@ __global__ void __launch_bounds__(32 * kWarpCellWarps) transport_x_warp_kernel(c
 
 namespace {
 // Calls and gathered launches of up to this many cells per SM go one cell per warp: a thread's cell takes 55, 460 and
-// 18,000 us however few there are (10, 53, 250 species), a warp's 30, 69 and 715 us and then 9, 40 and 630 ns per
+// 18,000 us however few there are (10, 53, 250 species), a warp's 30, 70 and 660 us and then 9, 34 and 480 ns per
 // cell; beyond these lines the thread form is the faster.
 template <int KMAX>
-constexpr size_t kWarpCellsPerSmX = KMAX == 16 ? 24 : KMAX == 64 ? 80 : 216;
+constexpr size_t kWarpCellsPerSmX = KMAX == 16 ? 24 : KMAX == 64 ? 96 : 256;
 
 template <int KMAX>
 cudaError_t launch_transport_xk(const uint8_t* tab, uint32_t tab_bytes, const TransportArgs<KMAX>& io, size_t n,
                                 cudaStream_t st, int* status) {
     if (n <= (size_t)sm_count() * kWarpCellsPerSmX<KMAX>) {
-        const size_t share = (n + sm_count() - 1) / sm_count();
-        const int warps = share < (size_t)kWarpCellWarps ? (int)share : kWarpCellWarps;
-        const size_t scratch = (size_t)warps * kWarpScratch<KMAX> * sizeof(double);
-        const bool smem = warp_table_bytes(true, tab_bytes) + scratch <= (size_t)max_table_smem();
-        const size_t bytes = warp_table_bytes(smem, tab_bytes) + scratch;
+        const size_t share = (n + sm_count() - 1) / sm_count(), scratch = kWarpScratch<KMAX> * sizeof(double);
+        const bool smem = warp_table_bytes(true, tab_bytes) + 4 * scratch <= (size_t)max_table_smem();
+        int warps = share < (size_t)kWarpCellWarpsX ? (int)share : kWarpCellWarpsX;
+        while (warps > 1 && warp_table_bytes(smem, tab_bytes) + warps * scratch > (size_t)max_table_smem()) warps--;
+        const size_t bytes = warp_table_bytes(smem, tab_bytes) + warps * scratch;
         auto kern = smem ? transport_x_warp_kernel<KMAX, true> : transport_x_warp_kernel<KMAX, false>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return e;
