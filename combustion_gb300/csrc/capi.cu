@@ -366,6 +366,27 @@ int gather_launch(cb_mech* m, size_t n, const double* const* in, double* const* 
     return e == cudaSuccess ? CB_OK : cuda_fail(e, "transport kernel (gathered cells)");
 }
 
+// Two gathered lists in one launch (gather_launch with the outputs of the first in place and of the second compact).
+template <int KM>
+int gather_launch_two(cb_mech* m, size_t n1, const uint32_t* index1, size_t n2, const uint32_t* index2,
+                      const double* const* in, double* const* out, double* out2, size_t stride2, uint32_t flags,
+                      cudaStream_t st) {
+    cbg::TransportArgs<KM> a;
+    std::memset(&a, 0, sizeof a);
+    for (int q = 0; q < m->host.K + 3; q++) a.in[q] = in[q];
+    for (int q = 0; q < m->host.K + 2; q++) a.out[q] = out[q];
+    a.flags = (flags & CB_UNIFORM_PRESSURE) | cbg::kFromRates;
+    a.index = index1;
+    a.index2 = index2;
+    a.n1 = n1;
+    a.out2 = out2;
+    a.stride2 = stride2;
+    set_f64_tables(a, m);
+    const TransportLaunch t = transport_launch(m);
+    cudaError_t e = t.launch(KM, t.tab, (uint32_t)t.bytes, &a, n1 + n2, st, m->d_status);
+    return e == cudaSuccess ? CB_OK : cuda_fail(e, "transport kernel (two lists)");
+}
+
 template <int KM>
 int gather_launch_mixed(cb_mech* m, size_t n, const double* const* in, double* const* out, const uint32_t* index,
                         const uint32_t* count, bool compact, uint32_t flags, cudaStream_t st) {
@@ -400,6 +421,22 @@ int transport_gather(cb_mech* m, size_t n, const double* const* in, double* cons
     case 256: return gather_launch<256>(m, n, in, out, index, count, compact, flags, st);
     default: return ::fail(CB_ERR_UNSUPPORTED, "species count outside the compiled capacities");
     }
+}
+int transport_gather_two(cb_mech* m, size_t n1, const uint32_t* index1, const uint32_t* count1, size_t n2,
+                         const uint32_t* index2, const uint32_t* count2, const double* const* in, double* const* out,
+                         double* out2, size_t stride2, uint32_t flags, cudaStream_t st) {
+    if (n1 && n2 && m->d_transport_fixed && n1 + n2 <= cbg::transport_x_warp_cells(m->kmax)) {
+        switch (m->kmax) {
+        case 16: return gather_launch_two<16>(m, n1, index1, n2, index2, in, out, out2, stride2, flags, st);
+        case 64: return gather_launch_two<64>(m, n1, index1, n2, index2, in, out, out2, stride2, flags, st);
+        case 256: return gather_launch_two<256>(m, n1, index1, n2, index2, in, out, out2, stride2, flags, st);
+        }
+    }
+    int rc = transport_gather(m, n1, in, out, index1, count1, false, flags, st);
+    if (rc) return rc;
+    std::vector<double*> rows(m->host.K + 2);
+    for (size_t q = 0; q < rows.size(); q++) rows[q] = out2 + q * stride2;
+    return transport_gather(m, n2, in, rows.data(), index2, count2, true, flags, st);
 }
 int transport_gather_mixed(cb_mech* m, size_t n, const double* const* in, double* const* out, const uint32_t* index,
                            const uint32_t* count, bool compact, uint32_t flags, cudaStream_t st) {

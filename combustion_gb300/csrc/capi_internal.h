@@ -29,6 +29,11 @@ MechView view(const cb_mech* m);
 int transport_gather(cb_mech* m, size_t n, const double* const* in, double* const* out, const uint32_t* index,
                      const uint32_t* count, bool compact, uint32_t flags, cudaStream_t st);
 
+// Both lists of a gate whose lengths are known on the host: n1 cells of index1 in place, n2 of index2 to position j of
+// out2 + k stride2; in one launch when they are few.
+int transport_gather_two(cb_mech* m, size_t n1, const uint32_t* index1, const uint32_t* count1, size_t n2,
+                         const uint32_t* index2, const uint32_t* count2, const double* const* in, double* const* out,
+                         double* out2, size_t stride2, uint32_t flags, cudaStream_t st);
 // The same with the mixed-precision transport kernel (FP32 fits and mixing).
 int transport_gather_mixed(cb_mech* m, size_t n, const double* const* in, double* const* out,
                            const uint32_t* index, const uint32_t* count, bool compact, uint32_t flags,

@@ -61,6 +61,11 @@ struct TransportArgs {
     const uint32_t* index;       // gathered cells (null: cell j is input j)
     const uint32_t* count;       // number of gathered cells, read on the device (null: n)
     const uint8_t* f64_tab;      // fixed-point kernels: the FP64 tables, in global memory
+    // A second list behind the n1 cells of `index` (one cell per warp only): its outputs go to position j of
+    // out2 + k stride2.
+    const uint32_t* index2;
+    double* out2;
+    size_t n1, stride2;
 };
 
 // Smallest compiled capacity holding K species (0 if none).
@@ -136,6 +141,7 @@ inline size_t rates_warp_bytes(int K, int R, int n_eff) { return (4 * (size_t)K 
 cudaError_t launch_transport_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                cudaStream_t st, int* status);
 size_t wave_transport_x(int kmax, uint32_t tab_bytes);
+size_t transport_x_warp_cells(int kmax);  // most cells of a call that goes one cell per warp
 size_t wave_rates_x(int kmax, uint32_t tab_bytes);
 size_t wave_reaction_rates_x(int kmax, uint32_t tab_bytes);
 cudaError_t launch_rates_mixed(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,

@@ -335,8 +335,9 @@ int ensure_inference(cb_surrogate* s, size_t rows) {
 }
 
 // Inference forward over `rows` rows of Xi into Yi (FP32, normalised outputs): the fused kernel for the
-// 64 -> 256 x n -> 64 shape, one GEMM per layer otherwise.
-int infer_rows(cb_surrogate* s, int rows, const CUtensorMap& mX, cudaStream_t st) {
+// 64 -> 256 x n -> 64 shape, one GEMM per layer otherwise. `o` (the fused shape only): the transport properties of
+// its cells instead of Yi.
+int infer_rows(cb_surrogate* s, int rows, const CUtensorMap& mX, cudaStream_t st, const OutputArgs* o = nullptr) {
     if (mlp_fused_shape(s->dims, s->L)) {
         FusedMaps maps;
         std::memset(&maps, 0, sizeof maps);
@@ -351,6 +352,13 @@ int infer_rows(cb_surrogate* s, int rows, const CUtensorMap& mX, cudaStream_t st
         }
         p.Y = s->Yi;
         p.ldY = s->n_out;
+        if (o) {
+            p.n_feat = o->n_feat;
+            p.cells = (int)o->n;
+            p.mean = o->mean;
+            p.std = o->std;
+            for (int j = 0; j < o->n_feat; j++) p.out[j] = o->out[j];
+        }
         p.status = s->status;
         SUR_CUDA(mlp_infer(mX, maps, p, st));
         return CB_OK;
@@ -932,8 +940,6 @@ int cb_surrogate_transport(cb_surrogate* s, size_t n, const double* const* input
         SUR_CUDA(mark(0));
         SUR_CUDA(features(f, st));
         SUR_CUDA(mark(1));
-        SUR_RC(infer_rows(s, rows, s->mXi, st));
-        SUR_CUDA(mark(2));
         OutputArgs o;
         std::memset(&o, 0, sizeof o);
         o.Y = s->Yi;
@@ -943,7 +949,10 @@ int cb_surrogate_transport(cb_surrogate* s, size_t n, const double* const* input
         o.mean = nrm(s, kOutMean);
         o.std = nrm(s, kOutStd);
         for (int q = 0; q < K + 2; q++) o.out[q] = out[q];
-        SUR_CUDA(cbg::sur::outputs(o, st));
+        const bool fused = mlp_fused_shape(s->dims, s->L);  // its last layer writes the properties
+        SUR_RC(infer_rows(s, rows, s->mXi, st, fused ? &o : nullptr));
+        SUR_CUDA(mark(2));
+        if (!fused) SUR_CUDA(cbg::sur::outputs(o, st));
         SUR_CUDA(mark(3));
         SUR_CUDA(elapsed(0, 1));
         SUR_CUDA(elapsed(1, 2));
@@ -958,14 +967,10 @@ int cb_surrogate_transport(cb_surrogate* s, size_t n, const double* const* input
         n_audit = std::min<uint64_t>(cnt[1], audit_cap);
         SUR_CUDA(mark(3));
         const uint32_t pflags = uniform ? CB_UNIFORM_PRESSURE : 0;
-        if (n_fail)  // the plain kernel writes the rejected cells' outputs in place
-            SUR_RC(cbi::transport_gather(s->mech, n_fail, inputs, outputs, s->fail_idx, s->gate_count, false,
-                                         pflags, st));
+        // the plain kernel writes the rejected cells' outputs in place, and the audited cells' beside them
+        SUR_RC(cbi::transport_gather_two(s->mech, n_fail, s->fail_idx, s->gate_count, n_audit, s->audit_idx,
+                                         s->gate_count + 1, inputs, outputs, s->audit_plain, audit_cap, pflags, st));
         if (n_audit) {
-            std::vector<double*> aud(K + 2);
-            for (int q = 0; q < K + 2; q++) aud[q] = s->audit_plain + (size_t)q * audit_cap;
-            SUR_RC(cbi::transport_gather(s->mech, n_audit, inputs, aud.data(), s->audit_idx, s->gate_count + 1,
-                                         true, pflags, st));
             AuditArgs a;
             std::memset(&a, 0, sizeof a);
             a.idx = s->audit_idx;

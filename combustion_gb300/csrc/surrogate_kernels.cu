@@ -718,22 +718,24 @@ __device__ __forceinline__ int ordered(float f) {
 // throughout (the inputs converted with integer instructions): the features end as BF16, and FP64
 // arithmetic here would make the kernel FP64-pipe bound. Features come in order, so `s` accumulates the
 // amounts read so far and the bulk (the last feature) is N - s: every input is read once.
-__device__ __forceinline__ float raw_feature(const FeatureArgs& a, size_t c, int j, float logT, float logP,
-                                             float N, float rN, float& s) {
+__device__ __forceinline__ float raw_feature(const FeatureArgs& a, float amount, int j, float logT, float logP, float N,
+                                             float rN, float& s) {
     if (j == 0) return logT;
     if (j == 1) return logP;
-    const int k = j - 2;
-    if (k < a.K - 1) {
-        const float x = dbl_to_flt(a.in[4 + k][c]);
-        s += x;
-        return x * rN;
+    if (j - 2 < a.K - 1) {
+        s += amount;
+        return amount * rN;
     }
     return (N - s) * rN;
 }
 
+// STATS: with the raw copy or the training range (statistics of the training cells). Without them nothing is written
+// between a cell's loads: the amounts of eight features are loaded together (one at a time, each waiting for HBM, they
+// took 153 us per 524,288 cells at 53 species).
+template <bool STATS>
 __global__ void features_kernel(const FeatureArgs a) {
-    __shared__ int lo_s[kMaxOut], hi_s[kMaxOut];
-    const bool hull = a.hull_lo != nullptr;
+    __shared__ int lo_s[STATS ? kMaxOut : 1], hi_s[STATS ? kMaxOut : 1];
+    const bool hull = STATS && a.hull_lo != nullptr;
     if (hull) {
         for (int j = threadIdx.x; j < a.n_feat; j += blockDim.x) {
             lo_s[j] = 0x7fffffff;
@@ -753,15 +755,29 @@ __global__ void features_kernel(const FeatureArgs a) {
         float s = 0.f;
         const float logT = logf(T / (float)a.T0), logP = logf(pR * (float)a.R_over_P0);
         bool inside = true;
+        double next[8];
+        auto load = [&](int j0) {
+#pragma unroll
+            for (int h = 0; h < 8; h++) {
+                const int k = j0 + h - 2;
+                next[h] = k >= 0 && k < a.K - 1 ? a.in[4 + k][c] : 0.0;
+            }
+        };
+        load(0);
+#pragma unroll 1
         for (int j0 = 0; j0 < a.n_in; j0 += 8) {
+            double d[8];
+#pragma unroll
+            for (int h = 0; h < 8; h++) d[h] = next[h];
+            if (j0 + 8 < a.n_in) load(j0 + 8);
             float x[8];
 #pragma unroll
             for (int h = 0; h < 8; h++) {
                 const int j = j0 + h;
                 float f = 0.f;
                 if (j < a.n_feat) {
-                    f = raw_feature(a, c, j, logT, logP, N, rN, s);
-                    if (a.raw) a.raw[c * a.n_feat + j] = f;
+                    f = raw_feature(a, dbl_to_flt(d[h]), j, logT, logP, N, rN, s);
+                    if (STATS && a.raw) a.raw[c * a.n_feat + j] = f;
                     if (a.lo) inside &= (f >= a.lo[j]) & (f <= a.hi[j]);
                     if (hull) {
                         atomicMin(&lo_s[j], ordered(f));
@@ -798,7 +814,8 @@ cudaError_t features(const FeatureArgs& a, cudaStream_t st) {
     if (a.rows == 0) return cudaSuccess;
     size_t grid = (a.rows + 127) / 128;
     if (grid > 152 * 8) grid = 152 * 8;
-    features_kernel<<<(unsigned)grid, 128, 0, st>>>(a);
+    if (a.raw || a.hull_lo) features_kernel<true><<<(unsigned)grid, 128, 0, st>>>(a);
+    else features_kernel<false><<<(unsigned)grid, 128, 0, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -937,11 +954,13 @@ cudaError_t audit(const AuditArgs& a, size_t cap, cudaStream_t st) {
 // stay in shared memory between layers (written by the epilogue in the 128-byte-swizzled K-major layout
 // the next layer's MMAs read); weights stream through a two-stage ring by TMA; the accumulators of the
 // pair's two tiles live in the two halves of tensor memory, so that the epilogue of one tile overlaps
-// the MMAs of the other. Shape: 64 inputs, hidden width 256, 64 outputs (up to 62 species).
+// the MMAs of the other. The last layer's epilogue writes the transport properties themselves where they are wanted
+// (the network alone takes 262 us per 524,288 cells and as long with them; a pass over FP32 outputs took 82 more).
+// Shape: 64 inputs, hidden width 256, 64 outputs (up to 62 species).
 //   warp 0: TMA producer (input tiles, weight chunks in the MMAs' order)
 //   warp 1: TMEM owner and MMA issuer
-//   warps 2-17: epilogue, four warps per TMEM lane quarter (64 columns each; the 64-wide output layer
-//   takes two, 32 columns each): sixteen warps keep enough instructions in flight for a tile's epilogue
+//   warps 2-17: epilogue, four warps per TMEM lane quarter (64 columns each, 16 of the output layer):
+//   sixteen warps keep enough instructions in flight for a tile's epilogue
 //   to take about as long as the other tile's MMAs
 constexpr int kFusedEpiWarps = 16;
 constexpr int kFusedThreads = 64 + 32 * kFusedEpiWarps;
@@ -967,13 +986,20 @@ __device__ __forceinline__ void store_act_bf16(uint32_t chunk_base, int r, int c
 }
 
 __global__ void __launch_bounds__(kFusedThreads, 1)
-    mlp_infer_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ FusedMaps maps, const FusedParams p) {
+    mlp_infer_kernel(const __grid_constant__ CUtensorMap tx, const __grid_constant__ FusedMaps maps,
+                     const __grid_constant__ FusedParams p) {
     extern __shared__ uint8_t dsm[];
     __shared__ uint64_t w_full[kWStages], w_empty[kWStages], x_full[2], acc_full[2], act_ready[2], act_free[2], fin;
     __shared__ uint32_t tmem_s;
     // biases of every layer, the hidden layers' halved: silu(z) = h (1 + tanh h) with h = z / 2 = fma(1/2,
     // acc, b / 2), one FMA where z = acc + b and h = z / 2 took two (the same h: halving is exact)
     __shared__ __align__(16) float sbias[kMaxLayers * kFusedWidth];
+    __shared__ float snorm[128];  // with outputs: their standard deviations and means
+    if (p.n_feat)
+        for (int j = threadIdx.x; j < p.n_feat; j += blockDim.x) {
+            snorm[j] = p.std[j];
+            snorm[64 + j] = p.mean[j];
+        }
     const uint32_t base = (smem_u32(dsm) + 1023u) & ~1023u;
     const uint32_t act0 = base, wring = base + 2 * kActBytes;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1088,9 +1114,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         for (int pr = blockIdx.x; pr < pairs && ok; pr += gridDim.x, pi++) {
             for (int l = 0; l < L && ok; l++) {
                 const int N = p.dims[l + 1];
-                // this warp's columns: a quarter of N in chunks of 32 (N = 64: the first two quarters only)
-                const int cols = N >= 128 ? N / 4 : 32;
-                const int c_begin = quarter * cols < N ? quarter * cols : N;
                 const float* bias = sbias + l * kFusedWidth;  // halved for the hidden layers
                 for (int t = 0; t < 2 && ok; t++) {
                     const int tile = 2 * pr + t;
@@ -1103,12 +1126,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                     umma::fence_after_sync();
                     const uint32_t acc = tmem + (uint32_t)(t * 256) + ((uint32_t)(q * 32) << 16);
                     const uint32_t a_base = act0 + t * kActBytes;
+                    if (l < L - 1) {
 #pragma unroll 1
-                    for (int c = c_begin; c < c_begin + cols && c < N; c += 32) {
-                        float v[32];
-                        umma::tmem_ld32(acc + (uint32_t)c, v);
-                        const float4* b4 = reinterpret_cast<const float4*>(bias + c);  // broadcast reads
-                        if (l < L - 1) {
+                        for (int c = quarter * (N / 4); c < (quarter + 1) * (N / 4); c += 32) {
+                            float v[32];
+                            umma::tmem_ld32(acc + (uint32_t)c, v);
+                            const float4* b4 = reinterpret_cast<const float4*>(bias + c);  // broadcast reads
 #pragma unroll
                             for (int j = 0; j < 8; j++) {
                                 const float4 hb = b4[j];
@@ -1120,10 +1143,29 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
                                 }
                             }
                             store_act_bf16(a_base + (uint32_t)(c >> 6) * kActChunk, r, c, v);
+                        }
+                    } else {  // 64 columns, 16 per warp
+                        float v[16];
+                        const int c = quarter * 16;
+                        umma::tmem_ld16(acc + (uint32_t)c, v);
+                        const float4* b4 = reinterpret_cast<const float4*>(bias + c);
+                        if (p.n_feat) {  // transport properties (outputs_kernel's), a warp's 32 cells per store
+                            const int cell = tile * kBM + r;
+#pragma unroll
+                            for (int j = 0; j < 4; j++) {
+                                const float4 b = b4[j];
+                                const float bb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                                for (int e = 0; e < 4; e++) {
+                                    const int f = c + 4 * j + e;
+                                    if (f < p.n_feat && cell < p.cells)
+                                        p.out[f][cell] = (double)__expf(fmaf(snorm[f], v[4 * j + e] + bb[e], snorm[64 + f]));
+                                }
+                            }
                         } else {
                             float4* dst = reinterpret_cast<float4*>(p.Y + ((size_t)tile * kBM + r) * p.ldY + c);
 #pragma unroll
-                            for (int j = 0; j < 8; j++) {
+                            for (int j = 0; j < 4; j++) {
                                 const float4 b = b4[j];
                                 dst[j] = make_float4(v[4 * j] + b.x, v[4 * j + 1] + b.y, v[4 * j + 2] + b.z, v[4 * j + 3] + b.w);
                             }

@@ -162,6 +162,11 @@ struct FusedParams {
     const float* bias[kMaxLayers];
     float* Y;
     int ldY;
+    // n_feat > 0: instead of Y, the transport properties exp(mean_j + std_j y_j) of `cells` cells (rows beyond are
+    // padding) to out[j]
+    int n_feat, cells;
+    const float* mean; const float* std;
+    double* out[64];
     int* status;
 };
 bool mlp_fused_shape(const int* dims, int L);

@@ -29,6 +29,11 @@ __device__ __forceinline__ const double* const* transport_inputs(const Header& H
     Tn = io.in[1][i];
     return io.in + 2;
 }
+// Output array k of a cell of the first or the second list.
+template <class Args>
+__device__ __forceinline__ double* transport_out(const Args& io, int k, bool second) {
+    return second ? io.out2 + (size_t)k * io.stride2 : io.out[k];
+}
 // Products here are rounded on their own (never fused into the next add, as in the reference's own
 // arithmetic), so that the two kernels cannot differ by where the compiler contracts.
 __device__ __forceinline__ double conductivity_of(double Ac, double Bc, double N, double VT) {
@@ -174,7 +179,7 @@ constexpr int kWarpScratch = 4 * KMAX + 32 * 33;  // doubles per warp: X, v, Y, 
 
 template <int KMAX>
 __device__ void transport_cell_warp(const uint8_t* tab, const TransportArgs<KMAX>& io, size_t i, size_t o,
-                                    double* sh) {
+                                    double* sh, bool second = false) {
     static_assert(2 * KMAX <= 32 * 33, "the viscosity terms reuse the tile");
     const int lane = threadIdx.x & 31;
     const TransportHeader& H = *reinterpret_cast<const TransportHeader*>(tab + kMathBytes);
@@ -224,7 +229,7 @@ __device__ void transport_cell_warp(const uint8_t* tab, const TransportArgs<KMAX
     const double Ac = __shfl_sync(0xffffffffu, acc, 1);
     const double Bc = __shfl_sync(0xffffffffu, acc, 2);
     __syncwarp();  // lanes 0-2 are done with v and Y
-    if (lane == 0) io.out[0][o] = conductivity_of(Ac, Bc, N, VT);
+    if (lane == 0) transport_out(io, 0, second)[o] = conductivity_of(Ac, Bc, N, VT);
     const double MVTN = MN * VT;
 
     // Viscosity: one row of the expanded Wilke sums per lane, each over j in order; the products and
@@ -257,7 +262,7 @@ __device__ void transport_cell_warp(const uint8_t* tab, const TransportArgs<KMAX
         double mu = 0.0;
 #pragma unroll 1
         for (int k = 0; k < K; k++) mu = fma(T[2 * k], T[2 * k + 1], mu);
-        io.out[1][o] = VT * mu;
+        transport_out(io, 1, second)[o] = VT * mu;
     }
     __syncwarp();
 
@@ -300,7 +305,7 @@ __device__ void transport_cell_warp(const uint8_t* tab, const TransportArgs<KMAX
             __syncwarp();
         }
     }
-    for (int k = lane; k < K; k += 32) io.out[2 + k][o] = diffusion_of(MVTN, VT, W[k], X[k], S[k]);
+    for (int k = lane; k < K; k += 32) transport_out(io, 2 + k, second)[o] = diffusion_of(MVTN, VT, W[k], X[k], S[k]);
     __syncwarp();  // the scratch is reused by the warp's next cell
 }
 

@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kTransportXBlock<KMAX>) transport_x_kernel(con
 // One cell per warp, every sum in the thread form's order (transport_cell_warp's division of the work).
 template <int KMAX>
 __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb, const TransportArgs<KMAX>& io, size_t i,
-                                                      size_t o, double* sh) {
+                                                      size_t o, double* sh, bool second) {
     const int lane = threadIdx.x & 31;
     const TransportXHeader& H = *tb.H;
     const int K = H.K;
@@ -277,7 +277,7 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
     const double Ac = __shfl_sync(0xffffffffu, acc, 1);
     const double Bc = __shfl_sync(0xffffffffu, acc, 2);
     __syncwarp();
-    if (lane == 0) io.out[0][o] = conductivity_of(Ac, Bc, N, VT);
+    if (lane == 0) transport_out(io, 0, second)[o] = conductivity_of(Ac, Bc, N, VT);
 
     int my = 0, mz = 0;
     for (int k = lane; k < K; k += 32) {
@@ -325,7 +325,7 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
         for (int k = lane; k < K; k += 2) mu = fma(U[2 * k], U[2 * k + 1], mu);
     }
     mu += __shfl_sync(0xffffffffu, mu, 1);
-    if (lane == 0) io.out[1][o] = VT * mu;
+    if (lane == 0) transport_out(io, 1, second)[o] = VT * mu;
     __syncwarp();
 
     // Diffusion, in tiles of 32 rows by 32 columns of pairs: lanes on consecutive pairs of a row (consecutive table
@@ -375,15 +375,16 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
             __syncwarp();
         }
     }
-    for (int k = lane; k < K; k += 32) io.out[2 + k][o] = diffusion_x(MN, VT, tb.W[k], X[k], S[k]);
+    for (int k = lane; k < K; k += 32) transport_out(io, 2 + k, second)[o] = diffusion_x(MN, VT, tb.W[k], X[k], S[k]);
     return true;
 }
 
 constexpr int kWarpCellWarpsX = 16;  // cells per block, as many as fit in shared memory
 
 template <int KMAX>
-__device__ __noinline__ void transport_cell_f64_warp(const TransportArgs<KMAX>& io, size_t i, size_t o, double* sh) {
-    transport_cell_warp<KMAX>(io.f64_tab, io, i, o, sh);
+__device__ __noinline__ void transport_cell_f64_warp(const TransportArgs<KMAX>& io, size_t i, size_t o, double* sh,
+                                                     bool second) {
+    transport_cell_warp<KMAX>(io.f64_tab, io, i, o, sh, second);
 }
 
 template <int KMAX, bool SMEM>
@@ -400,13 +401,15 @@ __global__ void __launch_bounds__(32 * kWarpCellWarpsX) transport_x_warp_kernel(
     const TransportXTables tb(SMEM ? cb_dsmem : gtab);
     double* sh = reinterpret_cast<double*>(cb_dsmem + warp_table_bytes(SMEM, tab_bytes)) +
                  (size_t)(threadIdx.x >> 5) * kWarpScratch<KMAX>;
-    if (io.count) n = min(n, (size_t)*io.count);
+    if (io.count && !io.index2) n = min(n, (size_t)*io.count);
     const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5);
     for (size_t j = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); j < n; j += warps) {
-        const size_t i = io.index ? (size_t)(io.index[j] & kIndexMask) : j, o = (io.flags & kCompactOut) ? j : i;
-        if (!transport_cell_x_warp<KMAX>(tb, io, i, o, sh)) {
+        const bool second = io.index2 && j >= io.n1;
+        const size_t i = second ? (size_t)(io.index2[j - io.n1] & kIndexMask) : io.index ? (size_t)(io.index[j] & kIndexMask) : j;
+        const size_t o = second ? j - io.n1 : (io.flags & kCompactOut) ? j : i;
+        if (!transport_cell_x_warp<KMAX>(tb, io, i, o, sh, second)) {
             __syncwarp();
-            transport_cell_f64_warp<KMAX>(io, i, o, sh);
+            transport_cell_f64_warp<KMAX>(io, i, o, sh, second);
         }
         __syncwarp();  // the scratch is reused by the warp's next cell
     }
@@ -454,6 +457,9 @@ cudaError_t launch_transport_x(int kmax, const uint8_t* tab, uint32_t tab_bytes,
         return launch_transport_xk<256>(tab, tab_bytes, *static_cast<const TransportArgs<256>*>(args), n, st, status);
     default: return cudaErrorInvalidValue;
     }
+}
+size_t transport_x_warp_cells(int kmax) {
+    return (size_t)sm_count() * (kmax == 16 ? kWarpCellsPerSmX<16> : kmax == 64 ? kWarpCellsPerSmX<64> : kWarpCellsPerSmX<256>);
 }
 template <int KMAX>
 static size_t wave_transport_xk(uint32_t tab_bytes) {

@@ -188,3 +188,35 @@ def test_rates_small_calls_match_large_ones(config, make):
             out[r] = t[:, -48:].cpu().numpy()
         assert np.array_equal(out[1], out[40], equal_nan=True)
         assert np.array_equal(out[1], out[reps], equal_nan=True)
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 257, 39000])
+def test_surrogate_call_sizes(n):
+    """The inference kernel writes the transport properties of every cell of a call and nothing beyond, whatever
+    the call's last tile holds; fallback and audited cells (one launch for both lists when few, two otherwise) keep the
+    plain kernel's bits."""
+    import torch
+    import combustion_gb300 as cb
+    from combustion_gb300 import surrogate as S
+    m = util.mechanism("k10")
+    mech = cb.Mechanism(m)
+    mech.transport_setup(*synthetic.transport_scales(m))
+    s = S.Surrogate(mech, width=256, hidden_layers=2, batch=1024, seed=3)
+    s.generate(1 << 13, S.distribution("k10", seed=2))
+    cells = S.generate_cells(mech, 39000, S.distribution("k10", seed=7))[:, :n].contiguous()
+    cells[2, ::5] = 5000.0  # outside the training range
+    full = torch.full((mech.K + 2, n + 130), -1.0, dtype=torch.float64, device="cuda")
+    s.transport(cells, full[:, :n], gate=False)
+    every = torch.full((mech.K + 2, 39000), -1.0, dtype=torch.float64, device="cuda")
+    s.transport(torch.cat([cells, cells.flip(1).repeat(1, 39000 // n + 1)], 1)[:, :39000].contiguous(), every, gate=False)
+    assert torch.equal(full[:, :n], every[:, :n])
+    assert bool((full[:, n:] == -1.0).all()) and bool((full[:, :n] > 0).all())
+    gated = torch.empty((mech.K + 2, n), dtype=torch.float64, device="cuda")
+    st = s.transport(cells, gated, audit_stride=3)
+    plain = torch.empty_like(gated)
+    rates = torch.empty((mech.A + 2, n), dtype=torch.float64, device="cuda")
+    mech.rates_transport(cells, rates, plain)
+    idx = torch.arange(n, device="cuda")
+    own = (idx % 5 == 0) | (idx % 3 == 7919 % 3)
+    assert st["fallback_cells"] >= int((idx % 5 == 0).sum())
+    assert torch.equal(gated[:, own], plain[:, own])
