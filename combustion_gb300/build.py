@@ -10,7 +10,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libcombustion_gb300.so")
 BUILD = os.path.join(HERE, "_build")
-SOURCES = ["mechanism.cpp", "kernels.cu", "kernels_mixed.cu", "kernels_fixed.cu", "transport_fixed.cu", "fixed_tables.cpp", "capi.cu", "diagnostics.cu", "surrogate.cu",
+SOURCES = ["mechanism.cpp", "kernels.cu", "kernels_mixed.cu", "mixed_warp.cu", "kernels_fixed.cu", "transport_fixed.cu", "fixed_tables.cpp", "capi.cu", "diagnostics.cu", "surrogate.cu",
            "surrogate_kernels.cu", "bdf.cu", "bdf_slice.cu", "bdf_slice_global.cu", "bdf_slice_global_wide.cu",
            "bdf_slice_global_mid.cu",
            "yaml_reader.cpp"]

@@ -108,6 +108,15 @@ int launch_rates_path(cb_mech* m, size_t n, const double* const* in, double* con
                                     m->host.rates_blob.size(), "rates kernel");
 }
 
+int launch_rates_mixed_path(cb_mech* m, size_t n, const double* const* in, double* const* out, uint32_t flags,
+                            cudaStream_t st) {
+    auto launch = [m](int kmax, const uint8_t* tab, uint32_t bytes, const void* args, size_t cells, cudaStream_t s, int* status) {
+        return cbg::launch_rates_mixed(kmax, tab, bytes, args, cells, rates_warp_bytes(m), s, status);
+    };
+    return dispatch<cbg::RatesArgs>(m, n, in, m->host.K + 3, out, m->host.A + 2, flags, st, launch, m->d_rates_mixed,
+                                    m->host.rates_mixed_bytes, "mixed rates kernel");
+}
+
 // The plain transport: the fixed-point kernels, or the FP64 ones.
 struct TransportLaunch {
     cudaError_t (*launch)(int, const uint8_t*, uint32_t, const void*, size_t, cudaStream_t, int*);
@@ -152,15 +161,13 @@ int launch_path(cb_mech* m, Path path, size_t n, const double* const* in, double
                                             t.tab, t.bytes, "transport kernel");
     }
     case Path::RatesMixed:
-        return dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, cbg::launch_rates_mixed,
-                                        m->d_rates_mixed, m->host.rates_mixed_blob.size(), "mixed rates kernel");
+        return launch_rates_mixed_path(m, n, in, out, flags, st);
     case Path::TransportMixed:
         return dispatch<cbg::TransportArgs>(m, n, in, K + 1, out, K + 2, flags, st, cbg::launch_transport_mixed,
                                             m->d_transport_mixed, m->host.transport_mixed_blob.size(),
                                             "mixed transport kernel");
     case Path::FusedMixed: {
-        int rc = dispatch<cbg::RatesArgs>(m, n, in, K + 3, out, A + 2, flags, st, cbg::launch_rates_mixed,
-                                          m->d_rates_mixed, m->host.rates_mixed_blob.size(), "mixed rates kernel");
+        int rc = launch_rates_mixed_path(m, n, in, out, flags, st);
         if (rc) return rc;
         return dispatch<cbg::TransportArgs>(m, n, in, K + 3, out + (A + 2), K + 2, flags | cbg::kFromRates, st,
                                             cbg::launch_transport_mixed, m->d_transport_mixed,
@@ -197,7 +204,7 @@ bool needs_transport(Path p) {
 // each persistent grid the same number of cells, so no SM idles through a chunk's last partial wave.
 size_t path_wave(const cb_mech* m, Path path) {
     const uint32_t rb = (uint32_t)m->host.rates_blob.size(), tb = (uint32_t)m->host.transport_blob.size();
-    const uint32_t rmb = (uint32_t)m->host.rates_mixed_blob.size();
+    const uint32_t rmb = (uint32_t)m->host.rates_mixed_bytes;
     const uint32_t tmb = (uint32_t)m->host.transport_mixed_blob.size();
     const uint32_t rfb = (uint32_t)m->host.rates_fixed_blob.size();
     auto rates_wave = [&] { return m->d_rates_fixed ? cbg::wave_rates_x(m->kmax, rfb) : cbg::wave_rates(m->kmax, rb); };

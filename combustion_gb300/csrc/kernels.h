@@ -144,8 +144,14 @@ size_t wave_transport_x(int kmax, uint32_t tab_bytes);
 size_t transport_x_warp_cells(int kmax);  // most cells of a call that goes one cell per warp
 size_t wave_rates_x(int kmax, uint32_t tab_bytes);
 size_t wave_reaction_rates_x(int kmax, uint32_t tab_bytes);
+// warp_bytes as above: small calls go one cell per warp (mixed_warp.cu); `tab_bytes` is what the kernels stage, the
+// species' reaction lists follow.
 cudaError_t launch_rates_mixed(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
-                               cudaStream_t st, int* status);
+                               size_t warp_bytes, cudaStream_t st, int* status);
+cudaError_t launch_rates_mixed_warp(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
+                                    size_t warp_bytes, cudaStream_t st, int* status);
+cudaError_t launch_transport_mixed_warp(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
+                                        cudaStream_t st, int* status);
 cudaError_t launch_transport_mixed(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                    cudaStream_t st, int* status);
 cudaError_t launch_transport(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,

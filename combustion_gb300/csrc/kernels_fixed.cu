@@ -306,7 +306,7 @@ __device__ __forceinline__ bool rates_cell_warp(const RatesXTables& tb, const Ra
     const RatesXHeader& H = *tb.H;
     const int K = H.K, A = H.A;
     const bool uniform = io.flags & kUniformPressure;
-    const double T = io.in[2][i], V = io.in[3][i];
+    const double T = io.in[2][i], V = io.in[3][i], rcp_pressure_R = uniform ? io.in[1][0] : io.in[1][i];
     CellXW<KMAX> c;
     if (!cell_progress_warp<KMAX>(tb, uniform ? io.in[0][0] : io.in[0][i], T, V, io.in + 4, i, sh, lane, c)) return false;
     double *C = sh, *h = sh + K, *cp = sh + 2 * K, *w = sh + 3 * K, *cR = sh + 4 * K + H.n_eff;
@@ -338,7 +338,7 @@ __device__ __forceinline__ bool rates_cell_warp(const RatesXTables& tb, const Ra
     const double E = __shfl_sync(0xffffffffu, acc, 0), Cp = __shfl_sync(0xffffffffu, acc, 1),
                  dtE = __shfl_sync(0xffffffffu, acc, 2);
     if (lane == 0) {
-        const double dtT_T = div64(-E, Cp), rcp_pressure_R = uniform ? io.in[1][0] : io.in[1][i];
+        const double dtT_T = div64(-E, Cp);
         io.out[0][i] = T * dtT_T;
         io.out[1][i] = V * fma(rcp_pressure_R * T, dtE, dtT_T);
     }
@@ -410,38 +410,12 @@ namespace {
 template <int KMAX>
 constexpr size_t kWarpCellsPerSmR = KMAX == 16 ? 32 : KMAX == 64 ? 150 : 100;
 
-// As many warps as fit beside the tables (or, of a large mechanism, beside the functions' tables).
-template <class KS, class KG, class Args>
-cudaError_t launch_rates_warp(KS ksmem, KG kglobal, const uint8_t* tab, uint32_t tab_bytes, const Args& io, size_t n,
-                              size_t warp_bytes, cudaStream_t st, int* status) {
-    const size_t share = (n + sm_count() - 1) / sm_count();
-    const uint32_t math = kMathBytes + kFixMathBytes;
-    const bool smem = tab_bytes + 2 * warp_bytes <= (size_t)max_table_smem();
-    int warps = share < (size_t)kRatesWarps ? (int)share : kRatesWarps;
-    while (warps > 1 && (smem ? tab_bytes : math) + warps * warp_bytes > (size_t)max_table_smem()) warps--;
-    const size_t bytes = (smem ? tab_bytes : math) + warps * warp_bytes;
-    if (bytes > (size_t)max_table_smem()) return cudaErrorInvalidConfiguration;
-    cudaError_t e = smem ? cudaFuncSetAttribute(ksmem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
-                         : cudaFuncSetAttribute(kglobal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    int per_sm = 1;
-    if (smem) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ksmem, 32 * warps, bytes);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kglobal, 32 * warps, bytes);
-    if (per_sm < 1) per_sm = 1;
-    size_t grid = (size_t)sm_count() * per_sm;
-    const size_t want = (n + warps - 1) / warps;
-    if (want < grid) grid = want;
-    if (smem) ksmem<<<(unsigned)grid, 32 * warps, bytes, st>>>(tab, tab_bytes, io, n, status);
-    else kglobal<<<(unsigned)grid, 32 * warps, bytes, st>>>(tab, tab_bytes, io, n, status);
-    return cudaGetLastError();
-}
-
 template <int KMAX>
 cudaError_t launch_rates_xk(const uint8_t* tab, uint32_t tab_bytes, const RatesArgs<KMAX>& io, size_t n, size_t warp_bytes,
                             cudaStream_t st, int* status) {
     if (n <= (size_t)sm_count() * kWarpCellsPerSmR<KMAX> && 4 * warp_bytes + 32768 <= (size_t)max_table_smem())
-        return launch_rates_warp(rates_x_warp_kernel<KMAX, true>, rates_x_warp_kernel<KMAX, false>, tab, tab_bytes, io, n,
-                                 warp_bytes, st, status);
+        return launch_warp_kernel<kRatesWarps>(rates_x_warp_kernel<KMAX, true>, rates_x_warp_kernel<KMAX, false>, tab, tab_bytes, io, n,
+                                               kMathBytes + kFixMathBytes, warp_bytes, st, status);
     return launch_table_kernel<kRatesXBlock>(rates_x_kernel<KMAX, true>, rates_x_kernel<KMAX, false>, tab, tab_bytes, io, n,
                                              kMathBytes + kFixMathBytes, true, st, status);
 }
@@ -449,8 +423,8 @@ template <int KMAX>
 cudaError_t launch_reaction_rates_xk(const uint8_t* tab, uint32_t tab_bytes, const ReactionRatesArgs<KMAX>& io, size_t n,
                                      size_t warp_bytes, cudaStream_t st, int* status) {
     if (n <= (size_t)sm_count() * kWarpCellsPerSmR<KMAX> && 4 * warp_bytes + 32768 <= (size_t)max_table_smem())
-        return launch_rates_warp(reaction_rates_x_warp_kernel<KMAX, true>, reaction_rates_x_warp_kernel<KMAX, false>, tab,
-                                 tab_bytes, io, n, warp_bytes, st, status);
+        return launch_warp_kernel<kRatesWarps>(reaction_rates_x_warp_kernel<KMAX, true>, reaction_rates_x_warp_kernel<KMAX, false>, tab,
+                                               tab_bytes, io, n, kMathBytes + kFixMathBytes, warp_bytes, st, status);
     return launch_table_kernel<kRatesXBlock>(reaction_rates_x_kernel<KMAX, true>, reaction_rates_x_kernel<KMAX, false>, tab,
                                              tab_bytes, io, n, kMathBytes + kFixMathBytes, true, st, status);
 }

@@ -61,10 +61,10 @@ __device__ void rates_mixed_cell(const RatesMixedTables& tb, const RatesArgs<KMA
     const double T2 = T * T, T3 = T * T2, T4 = T2 * T2;
     double sum = 0.0;
     for (int k = 0; k < K - 1; k++) {
-        c.C[k] = md * max0(io.in[4 + k][i]);
+        c.C[k] = __dmul_rn(md, max0(io.in[4 + k][i]));  // (not fused into the sum: one rounding in every form)
         sum += c.C[k];
     }
-    const double Ctot = pressure_R * rcpT;
+    const double Ctot = __dmul_rn(pressure_R, rcpT);
     c.C[K - 1] = Ctot - sum;
     c.Ctotf = dbl_to_flt(Ctot);
     c.Tf = dbl_to_flt(T);
@@ -274,8 +274,29 @@ __global__ void __launch_bounds__(kTransportMixedBlock) transport_mixed_kernel(c
 }
 
 // ---------------------------------------------------------------------------------------------------
-CB_DISPATCH(launch_rates_mixed, rates_mixed_kernel, RatesArgs, kBlock, kMathBytes, false)
-CB_DISPATCH(launch_transport_mixed, transport_mixed_kernel, TransportArgs, kTransportMixedBlock, kMathBytes, false)
+namespace {
+CB_DISPATCH(launch_rates_mixed_threads, rates_mixed_kernel, RatesArgs, kBlock, kMathBytes, false)
+CB_DISPATCH(launch_transport_mixed_threads, transport_mixed_kernel, TransportArgs, kTransportMixedBlock, kMathBytes, false)
+// Calls and gathered launches of up to this many cells per SM go one cell per warp (mixed_warp.cu). Rates: a thread's
+// cell takes 60, 520 and 6,000 us however few there are (10, 53, 250 species) and a call of one cell per thread 68, 780
+// and 9,900 us at 2,500, 30,000 and 30,000 cells; a warp's takes 42, 67 and 400 us and then 7, 22 and 310 ns per cell.
+// Transport: 12, 44 and 4,400 us (73 and 6,500 at 3,000 and 7,600 cells of 53 and 250 species) against 11, 25 and 700 us
+// and then 10 and 640 ns per cell. Beyond these lines the thread form is the faster.
+size_t rates_warp_cells(int kmax) { return (size_t)sm_count() * (kmax == 16 ? 28 : 192); }
+size_t transport_warp_cells(int kmax) { return (size_t)sm_count() * (kmax == 16 ? 32 : kmax == 64 ? 24 : 60); }
+}  // namespace
+
+cudaError_t launch_rates_mixed(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
+                               size_t warp_bytes, cudaStream_t st, int* status) {
+    if (n <= rates_warp_cells(kmax) && kMathBytes + 4 * warp_bytes <= (size_t)max_table_smem())
+        return launch_rates_mixed_warp(kmax, tab, tab_bytes, args, n, warp_bytes, st, status);
+    return launch_rates_mixed_threads(kmax, tab, tab_bytes, args, n, st, status);
+}
+cudaError_t launch_transport_mixed(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
+                                   cudaStream_t st, int* status) {
+    if (n <= transport_warp_cells(kmax)) return launch_transport_mixed_warp(kmax, tab, tab_bytes, args, n, st, status);
+    return launch_transport_mixed_threads(kmax, tab, tab_bytes, args, n, st, status);
+}
 CB_WAVE(wave_rates_mixed, rates_mixed_kernel, kBlock, kMathBytes)
 CB_WAVE(wave_transport_mixed, transport_mixed_kernel, kTransportMixedBlock, kMathBytes)
 

@@ -60,6 +60,31 @@ cudaError_t launch_table_kernel(KS ksmem, KG kglobal, const uint8_t* tab, uint32
     return cudaGetLastError();
 }
 
+// One cell per warp, up to WARPS of them in a block: as many warps as fit beside the tables (or, of a large mechanism, beside the functions' tables).
+template <int WARPS, class KS, class KG, class Args>
+cudaError_t launch_warp_kernel(KS ksmem, KG kglobal, const uint8_t* tab, uint32_t tab_bytes, const Args& io, size_t n,
+                               uint32_t math, size_t warp_bytes, cudaStream_t st, int* status) {
+    const size_t share = (n + sm_count() - 1) / sm_count();
+    const bool smem = tab_bytes + 2 * warp_bytes <= (size_t)max_table_smem();
+    int warps = share < (size_t)WARPS ? (int)share : WARPS;
+    while (warps > 1 && (smem ? tab_bytes : math) + warps * warp_bytes > (size_t)max_table_smem()) warps--;
+    const size_t bytes = (smem ? tab_bytes : math) + warps * warp_bytes;
+    if (bytes > (size_t)max_table_smem()) return cudaErrorInvalidConfiguration;
+    cudaError_t e = smem ? cudaFuncSetAttribute(ksmem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
+                         : cudaFuncSetAttribute(kglobal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    int per_sm = 1;
+    if (smem) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ksmem, 32 * warps, bytes);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kglobal, 32 * warps, bytes);
+    if (per_sm < 1) per_sm = 1;
+    size_t grid = (size_t)sm_count() * per_sm;
+    const size_t want = (n + warps - 1) / warps;
+    if (want < grid) grid = want ? want : 1;
+    if (smem) ksmem<<<(unsigned)grid, 32 * warps, bytes, st>>>(tab, tab_bytes, io, n, status);
+    else kglobal<<<(unsigned)grid, 32 * warps, bytes, st>>>(tab, tab_bytes, io, n, status);
+    return cudaGetLastError();
+}
+
 template <int BLOCK, class KS, class KG>
 size_t wave_of(KS ksmem, KG kglobal, uint32_t tab_bytes, uint32_t math_bytes) {
     int per_sm = 1;

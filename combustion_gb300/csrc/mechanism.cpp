@@ -591,6 +591,17 @@ int build_mechanism(const cb_mech_desc* d, HostMechanism& m, std::string& err) {
         hm.off_falloff = align_blob(b); append(b, ff.data(), ff.size());
         hm.off_eff = align_blob(b); append(b, efff.data(), efff.size());
         finish_blob(b, hm);
+        m.rates_mixed_bytes = b.size();
+        // behind what the kernels stage: per active species its reactions (grouped order) and net coefficients
+        std::vector<int32_t> start(A + 1, 0), lists;
+        for (int k = 0; k < A; k++) {
+            for (int r = 0; r < R; r++)
+                for (int q = 0; q < rfg[r].n_net; q++)
+                    if (rfg[r].net_k[q] == k) lists.push_back((r << 8) | (rfg[r].net_n[q] & 0xff));
+            start[k + 1] = (int32_t)lists.size();
+        }
+        append(b, start.data(), start.size());
+        append(b, lists.data(), lists.size());
     }
 
     // ---- algorithmic work of reaction.rs:356-391 per cell (the reference's operations) ----------

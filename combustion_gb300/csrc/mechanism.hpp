@@ -23,7 +23,8 @@ struct HostMechanism {
     std::vector<double> rate, k0, troe, sri, eff;  // [R*3], [R*3], [R*4], [R*5], [R*K]
 
     std::vector<uint8_t> rates_blob;
-    std::vector<uint8_t> rates_mixed_blob;  // tables of the mixed-precision form
+    std::vector<uint8_t> rates_mixed_blob;  // tables of the mixed-precision form, then the species' reaction lists
+    size_t rates_mixed_bytes = 0;           // the tables alone
     std::vector<uint8_t> rates_fixed_blob;  // fixed-point tables of the plain form (empty: out of their range)
     Work rates_work;
 

@@ -220,3 +220,36 @@ def test_surrogate_call_sizes(n):
     own = (idx % 5 == 0) | (idx % 3 == 7919 % 3)
     assert st["fallback_cells"] >= int((idx % 5 == 0).sum())
     assert torch.equal(gated[:, own], plain[:, own])
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+def test_mixed_small_calls_match_large_ones(config):
+    """The mixed-precision form: a cell has the same bits in calls of 1, 47, 480 and more cells than go one per warp."""
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = shapes_mechanism(config)
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    mech.transport_setup(*synthetic.transport_scales(m))
+    cells = edge_temperatures(config, 48)
+    x = np.array(o.rates_inputs(cells))
+    x[4, 20], x[2, 22], x[3, 23] = np.nan, np.nan, 0.0
+    reps = 640 * 152 // 48 + 1
+    large = None
+    for n in (48 * reps, 480, 47, 1):
+        xin = torch.tensor(np.tile(x, (1, n // 48 + 1))[:, :n].copy(), dtype=torch.float64, device="cuda")
+        r = torch.full((mech.A + 2, n), float("nan"), dtype=torch.float64, device="cuda")
+        t = torch.full((mech.K + 2, n), float("nan"), dtype=torch.float64, device="cuda")
+        mech.rates_transport(xin, r, t, mixed=True)
+        mech.synchronize()
+        both = torch.cat([r, t]).cpu().numpy()
+        if large is None:
+            large = both[:, -48:]
+        assert np.array_equal(both, np.tile(large, (1, n // 48 + 1))[:, :n], equal_nan=True)
+    xin = torch.tensor(x, dtype=torch.float64, device="cuda")
+    uniform, split = torch.empty_like(r[:, :1]).expand(-1, 48).clone(), torch.empty_like(r[:, :1]).expand(-1, 48).clone()
+    mech.rates([xin[0, :1], xin[1, :1]] + list(xin[2:]), uniform, uniform_pressure=True, mixed=True)
+    xin[:2] = xin[:2, :1].clone()
+    mech.rates(xin, split, mixed=True)
+    mech.synchronize()
+    assert torch.equal(uniform.nan_to_num(7.0), split.nan_to_num(7.0))
