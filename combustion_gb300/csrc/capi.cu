@@ -12,6 +12,7 @@
 #include "../../include/combustion_gb300.h"
 #include "capi_internal.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "mechanism.hpp"
 #include "tables.h"
 
@@ -129,6 +130,33 @@ TransportLaunch transport_launch(const cb_mech* m) {
     return {cbg::launch_transport, m->d_transport, m->host.transport_blob.size()};
 }
 
+// kOverlap where the transport of a fused call may run beside its rates: its outputs touch neither the cells nor the
+// rates' outputs (ends of the whole range they span, so rows laid out in between count as touched).
+// The two kernels then fill what the other leaves idle: the SMs a small call does not reach, the last wave, the pipe
+// the other waits for. Rates and transport after / beside each other, us: 53 species 1 cell 107 / 75, 10,100 cells
+// 645 / 590, 160,000 cells 4,310 / 3,580; 250 species 1 cell 1,117 / 783, 60,000 cells 39,500 / 33,100 (mixed precision
+// 23,300 / 15,000). Not so for a few cells per SM of the small and the large tables, where both blocks land on one SM
+// and share its L1: 10 species, 3 to 11 cells per SM 60 / 71; 250 species, 4 to 16 (mixed precision 60) per SM 1,143 /
+// 3,220 at worst; nor for many waves of the small ones (10 species, 2^22 cells: 5,563 / 5,611).
+uint32_t overlap_flag(int kmax, bool mixed, size_t n, const double* const* in, int ni, double* const* rates, int nr,
+                      double* const* transport, int nt) {
+    const size_t per_sm = (n + cbg::sm_count() - 1) / cbg::sm_count();
+    if (kmax == 16 && ((per_sm > 2 && per_sm <= 11) || per_sm > 16384)) return 0;
+    if (kmax == 256 && per_sm > 3 && per_sm <= (mixed ? 60 : 16)) return 0;
+    uintptr_t lo = UINTPTR_MAX, hi = 0;
+    const size_t bytes = n * sizeof(double);
+    for (int q = 0; q < nt; q++) {
+        lo = std::min(lo, (uintptr_t)transport[q]);
+        hi = std::max(hi, (uintptr_t)transport[q] + bytes);
+    }
+    auto apart = [&](const double* p) { return (uintptr_t)p + bytes <= lo || (uintptr_t)p >= hi; };
+    for (int q = 0; q < ni; q++)
+        if (!apart(in[q])) return 0;
+    for (int q = 0; q < nr; q++)
+        if (!apart(rates[q])) return 0;
+    return cbg::kOverlap;
+}
+
 // One call on device pointers (pointer arrays already resolved).
 int launch_path(cb_mech* m, Path path, size_t n, const double* const* in, double* const* out, uint32_t flags,
                 cudaStream_t st) {
@@ -157,7 +185,8 @@ int launch_path(cb_mech* m, Path path, size_t n, const double* const* in, double
     case Path::Fused: {
         int rc = launch_rates_path(m, n, in, out, flags, st);
         if (rc) return rc;
-        return dispatch<cbg::TransportArgs>(m, n, in, K + 3, out + (A + 2), K + 2, flags | cbg::kFromRates, st, t.launch,
+        flags |= overlap_flag(m->kmax, false, n, in, K + 3, out, A + 2, out + (A + 2), K + 2) | cbg::kFromRates;
+        return dispatch<cbg::TransportArgs>(m, n, in, K + 3, out + (A + 2), K + 2, flags, st, t.launch,
                                             t.tab, t.bytes, "transport kernel");
     }
     case Path::RatesMixed:
@@ -169,7 +198,8 @@ int launch_path(cb_mech* m, Path path, size_t n, const double* const* in, double
     case Path::FusedMixed: {
         int rc = launch_rates_mixed_path(m, n, in, out, flags, st);
         if (rc) return rc;
-        return dispatch<cbg::TransportArgs>(m, n, in, K + 3, out + (A + 2), K + 2, flags | cbg::kFromRates, st,
+        flags |= overlap_flag(m->kmax, true, n, in, K + 3, out, A + 2, out + (A + 2), K + 2) | cbg::kFromRates;
+        return dispatch<cbg::TransportArgs>(m, n, in, K + 3, out + (A + 2), K + 2, flags, st,
                                             cbg::launch_transport_mixed, m->d_transport_mixed,
                                             m->host.transport_mixed_blob.size(), "mixed transport kernel");
     }

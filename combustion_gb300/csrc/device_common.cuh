@@ -74,4 +74,11 @@ __device__ __forceinline__ double min_pos(double c, double x) { return bits(x) >
 // max(0, x) as f64::max(0., x): negative values (and negative zero) give +0.
 __device__ __forceinline__ double max0(double x) { return bits(x) < 0 ? 0.0 : x; }
 
+// Overlap of two kernels of a call (programmatic dependent launch). The first lets the second start as soon as all of
+// its blocks run; the second needs nothing of the first, but ends after it: whatever follows on the stream follows both.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+struct EndAfterPrevious {
+    __device__ __forceinline__ ~EndAfterPrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+};
+
 }  // namespace cbg

@@ -21,6 +21,7 @@ template <int KMAX, bool SMEM>
 __global__ void __launch_bounds__(kBlock) rates_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                                       const __grid_constant__ RatesArgs<KMAX> io, size_t n,
                                                       int* status) {
+    let_next_start();
     __shared__ uint64_t bar;
     const uint8_t* tab = gtab;
     if (SMEM) {  // the whole blob, math tables first, into dynamic shared memory
@@ -55,6 +56,7 @@ template <int KMAX, bool SMEM>
 __global__ void __launch_bounds__(kTransportBlock) transport_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                                           const __grid_constant__ TransportArgs<KMAX> io,
                                                           size_t n, int* status) {
+    const EndAfterPrevious last;
     __shared__ uint64_t bar;
     const uint8_t* tab = gtab;
     if (SMEM) {  // the whole blob, math tables first, into dynamic shared memory
@@ -75,6 +77,7 @@ __global__ void __launch_bounds__(32 * kWarpCellWarps) transport_warp_kernel(con
                                                                            uint32_t tab_bytes,
                                                                            const __grid_constant__ TransportArgs<KMAX> io,
                                                                            size_t n, int* status) {
+    const EndAfterPrevious last;
     __shared__ uint64_t bar;
     const uint8_t* tab = gtab;
     if (SMEM) {

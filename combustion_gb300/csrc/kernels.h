@@ -51,6 +51,8 @@ constexpr uint32_t kFromRates = 4u;
 // Gathered cells (the transport surrogate's fallback and audit): cell j of the launch is input cell
 // index[j] & kIndexMask, its outputs go to that cell too or, with kCompactOut, to position j.
 constexpr uint32_t kCompactOut = 8u;
+// The launch may start while the kernel before it on the stream still runs (device_common.cuh).
+constexpr uint32_t kOverlap = 16u;
 constexpr uint32_t kIndexMask = 0x7fffffffu;
 
 template <int KMAX>

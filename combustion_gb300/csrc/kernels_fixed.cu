@@ -186,6 +186,7 @@ template <int KMAX, bool SMEM>
 __global__ void __launch_bounds__(kRatesXBlock) rates_x_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                                         const __grid_constant__ RatesArgs<KMAX> io, size_t n,
                                                         int* status) {
+    let_next_start();
     __shared__ uint64_t bar;
     if (!stage_x<SMEM>(gtab, tab_bytes, &bar, status)) return;
     const RatesXTables tb(SMEM ? cb_dsmem : gtab);
@@ -386,6 +387,7 @@ template <int KMAX, bool SMEM>
 __global__ void __launch_bounds__(32 * kRatesWarps) rates_x_warp_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                                                       const __grid_constant__ RatesArgs<KMAX> io, size_t n,
                                                                       int* status) {
+    let_next_start();
     warp_cells<SMEM>(
         gtab, tab_bytes, n, status,
         [&](const RatesXTables& tb, size_t i, double* sh, int lane) { return rates_cell_warp<KMAX>(tb, io, i, sh, lane); },

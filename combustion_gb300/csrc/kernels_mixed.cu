@@ -131,6 +131,7 @@ template <int KMAX, bool SMEM>
 __global__ void __launch_bounds__(kBlock, 2) rates_mixed_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                                             const __grid_constant__ RatesArgs<KMAX> io, size_t n,
                                                             int* status) {
+    let_next_start();
     __shared__ uint64_t bar;
     const uint8_t* tab = gtab;
     if (SMEM) {  // the whole blob, math tables first, into dynamic shared memory
@@ -258,6 +259,7 @@ __global__ void __launch_bounds__(kTransportMixedBlock) transport_mixed_kernel(c
                                                                          uint32_t tab_bytes,
                                                                          const __grid_constant__ TransportArgs<KMAX> io,
                                                                          size_t n, int* status) {
+    const EndAfterPrevious last;
     __shared__ uint64_t bar;
     const uint8_t* tab = gtab;
     if (SMEM) {  // the whole blob, math tables first, into dynamic shared memory

@@ -23,6 +23,27 @@ bool gathered(const Args&) { return false; }
 template <int KMAX>
 bool gathered(const TransportArgs<KMAX>& io) { return io.index != nullptr; }
 
+template <class Args>
+bool overlapped(const Args&) { return false; }
+template <int KMAX>
+bool overlapped(const TransportArgs<KMAX>& io) { return io.flags & kOverlap; }
+
+template <class K, class Args>
+cudaError_t launch_one(K kernel, size_t grid, int block, size_t bytes, cudaStream_t st, const uint8_t* tab, uint32_t tab_bytes,
+                       const Args& io, size_t n, int* status) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlapped(io) ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, tab, tab_bytes, io, n, status);
+}
+
 // Persistent grid: as many blocks as fit on the GPU at once (each stages the tables once). A call of at most
 // two waves takes smaller blocks, so that every SM gets the same share of each wave and small calls spread
 // over all of them: blocks of 768 left 10,100 cells on 14 SMs. (Beyond two waves the last one weighs less
@@ -55,9 +76,8 @@ cudaError_t launch_table_kernel(KS ksmem, KG kglobal, const uint8_t* tab, uint32
     }
     const size_t want = (n + block - 1) / block;
     if (want < grid) grid = want ? want : 1;
-    if (smem) ksmem<<<(unsigned)grid, block, tab_bytes, st>>>(tab, tab_bytes, io, n, status);
-    else kglobal<<<(unsigned)grid, block, math_bytes, st>>>(tab, tab_bytes, io, n, status);
-    return cudaGetLastError();
+    return smem ? launch_one(ksmem, grid, block, tab_bytes, st, tab, tab_bytes, io, n, status)
+                : launch_one(kglobal, grid, block, math_bytes, st, tab, tab_bytes, io, n, status);
 }
 
 // One cell per warp, up to WARPS of them in a block: as many warps as fit beside the tables (or, of a large mechanism, beside the functions' tables).
@@ -80,9 +100,8 @@ cudaError_t launch_warp_kernel(KS ksmem, KG kglobal, const uint8_t* tab, uint32_
     size_t grid = (size_t)sm_count() * per_sm;
     const size_t want = (n + warps - 1) / warps;
     if (want < grid) grid = want ? want : 1;
-    if (smem) ksmem<<<(unsigned)grid, 32 * warps, bytes, st>>>(tab, tab_bytes, io, n, status);
-    else kglobal<<<(unsigned)grid, 32 * warps, bytes, st>>>(tab, tab_bytes, io, n, status);
-    return cudaGetLastError();
+    return smem ? launch_one(ksmem, grid, 32 * warps, bytes, st, tab, tab_bytes, io, n, status)
+                : launch_one(kglobal, grid, 32 * warps, bytes, st, tab, tab_bytes, io, n, status);
 }
 
 template <int BLOCK, class KS, class KG>

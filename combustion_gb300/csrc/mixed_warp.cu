@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(32 * kMixedWarps) rates_mixed_warp_kernel(cons
                                                                             uint32_t tab_bytes,
                                                                             const __grid_constant__ RatesArgs<KMAX> io,
                                                                             size_t n, int* status) {
+    let_next_start();
     __shared__ uint64_t bar;
     if (!stage_m<SMEM>(gtab, tab_bytes, &bar, status)) return;
     const RatesMixedTables tb(SMEM ? cb_dsmem : gtab);
@@ -256,6 +257,7 @@ template <int KMAX, bool SMEM>
 __global__ void __launch_bounds__(32 * kMixedWarps)
     transport_mixed_warp_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                 const __grid_constant__ TransportArgs<KMAX> io, size_t n, int* status) {
+    const EndAfterPrevious last;
     __shared__ uint64_t bar;
     if (!stage_m<SMEM>(gtab, tab_bytes, &bar, status)) return;
     const uint8_t* tab = SMEM ? cb_dsmem : gtab;

@@ -207,6 +207,7 @@ template <int KMAX, bool SMEM>
 __global__ void __launch_bounds__(kTransportXBlock<KMAX>) transport_x_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                                                      const __grid_constant__ TransportArgs<KMAX> io,
                                                                      size_t n, int* status) {
+    const EndAfterPrevious last;
     __shared__ uint64_t bar;
     if (SMEM) {
         if (!stage_to_shared(cb_dsmem, gtab, tab_bytes, &bar, status)) return;
@@ -392,6 +393,7 @@ __global__ void __launch_bounds__(32 * kWarpCellWarpsX) transport_x_warp_kernel(
                                                                              uint32_t tab_bytes,
                                                                              const __grid_constant__ TransportArgs<KMAX> io,
                                                                              size_t n, int* status) {
+    const EndAfterPrevious last;
     __shared__ uint64_t bar;
     if (SMEM) {
         if (!stage_to_shared(cb_dsmem, gtab, tab_bytes, &bar, status)) return;
@@ -440,8 +442,7 @@ cudaError_t launch_transport_xk(const uint8_t* tab, uint32_t tab_bytes, const Tr
         size_t grid = (size_t)sm_count() * per_sm;
         const size_t want = (n + warps - 1) / warps;
         if (want < grid) grid = want ? want : 1;
-        kern<<<(unsigned)grid, 32 * warps, bytes, st>>>(tab, tab_bytes, io, n, status);
-        return cudaGetLastError();
+        return launch_one(kern, grid, 32 * warps, bytes, st, tab, tab_bytes, io, n, status);
     }
     return launch_table_kernel<kTransportXBlock<KMAX>>(transport_x_kernel<KMAX, true>, transport_x_kernel<KMAX, false>, tab,
                                                  tab_bytes, io, n, kMathBytes, false, st, status);

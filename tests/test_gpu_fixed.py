@@ -253,3 +253,38 @@ def test_mixed_small_calls_match_large_ones(config):
     mech.rates(xin, split, mixed=True)
     mech.synchronize()
     assert torch.equal(uniform.nan_to_num(7.0), split.nan_to_num(7.0))
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_fused_call_beside_and_after(config, mixed):
+    """Rates and transport of one call, running beside each other or one after the other, give what two calls give;
+    where their outputs share memory the transport's are the last written; and the call can be captured."""
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = util.mechanism(config)
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    mech.transport_setup(*synthetic.transport_scales(m))
+    sizes = {"k10": (1, 300, 1000, 5000, 70001), "k53": (1, 300, 10100, 70001), "k250": (1, 456, 1000, 3000, 12001)}[config]
+    for n in sizes:
+        cells = synthetic.generate_cells(m.K, n, config, seed=7)
+        x = torch.tensor(np.array(o.rates_inputs(cells)), dtype=torch.float64, device="cuda")
+        new = lambda rows: torch.full((rows, n), float("nan"), dtype=torch.float64, device="cuda")  # noqa: E731
+        r, t, alone, shared = new(mech.A + 2), new(mech.K + 2), new(mech.A + 2), new(mech.K + 2)
+        mech.rates(x, alone, mixed=mixed)
+        mech.rates_transport(x, r, t, mixed=mixed)
+        mech.rates_transport(x, shared[:mech.A + 2], shared, mixed=mixed)
+        mech.synchronize()
+        assert torch.isfinite(r).all() and torch.isfinite(t).all()
+        assert torch.equal(r, alone) and torch.equal(shared, t)
+        if n == 300:
+            r2, t2 = new(mech.A + 2), new(mech.K + 2)
+            graph = torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph):
+                mech.rates_transport(x, r2, t2, mixed=mixed)
+            for _ in range(3):
+                graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(r2, r) and torch.equal(t2, t)
