@@ -60,7 +60,7 @@ __device__ __forceinline__ double wilke_rcp(long long s1, long long s2, long lon
 __device__ __forceinline__ double diffusion_x(double MN, double VT, double W, double X, double S) {
     return __dmul_rn(__dmul_rn(fma(-W, X, MN), VT), rcp64(S));
 }
-// The three sums' accumulators to values in one unit (four bits finer than the hi-hi products').
+// The three sums' accumulators to values in one unit (one bit finer than the hi-hi products').
 __device__ __forceinline__ long long mix_value(long long s1, long long s2) {
     return (s1 << 1) + ((s2 + (1ll << (kLo - 2))) >> (kLo - 1));
 }
