@@ -81,4 +81,19 @@ struct EndAfterPrevious {
     __device__ __forceinline__ ~EndAfterPrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 };
 
+// TEAM warps that share a cell: one, or all of the block.
+template <int TEAM>
+__device__ __forceinline__ void team_sync() {
+    if (TEAM == 1) __syncwarp();
+    else __syncthreads();
+}
+// The first lane's value on all; slot: shared memory that nothing uses until the next team_sync.
+template <int TEAM>
+__device__ __forceinline__ double team_value(double v, double* slot, int lane) {
+    if (TEAM == 1) return __shfl_sync(0xffffffffu, v, 0);
+    if (lane == 0) *slot = v;
+    __syncthreads();
+    return *slot;
+}
+
 }  // namespace cbg

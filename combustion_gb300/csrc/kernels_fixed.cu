@@ -215,6 +215,7 @@ __global__ void __launch_bounds__(kRatesXBlock) reaction_rates_x_kernel(const ui
 // One cell per warp, for calls too small to fill the GPU with one per thread: lanes share out species, third-body
 // rows and reactions; every FP64 sum runs on one lane in the thread form's order (the integer sums are exact), so that
 // a cell has the same bits in both forms.
+// TEAM warps (a block of its own) share a cell in calls of at most a cell per SM, 1 otherwise.
 constexpr int kRatesWarps = 16;  // cells per block at most
 
 template <int KMAX>
@@ -228,11 +229,13 @@ struct CellXW {
 };
 
 // The cell's rates of progress into cR [R] (grouped order); the concentrations stay in sh, followed by two free arrays
-// of K doubles and the species rates'. False where the cell needs the FP64 form (warp-uniform).
-template <int KMAX>
+// of K doubles and the species rates'. False where the cell needs the FP64 form (the same for all
+// its lanes). lane: of all of the cell's.
+template <int TEAM, int KMAX>
 __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, double pressure_R, double T, double V,
                                                    const double* const* amounts, size_t i, double* sh, int lane,
                                                    CellXW<KMAX>& c) {
+    constexpr int kStep = 32 * TEAM;
     const RatesXHeader& H = *tb.H;
     const int K = H.K, A = H.A;
     if (!(T >= kFixTmin && T < kFixTmax)) return false;
@@ -243,44 +246,48 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
     double* cR = M + H.n_eff;
     const double md = __drcp_rn(V);
     c.rcpT = __drcp_rn(T);
-    for (int k = lane; k < K - 1; k += 32) C[k] = __dmul_rn(md, max0(amounts[k][i]));
-    __syncwarp();
+    for (int k = lane; k < K - 1; k += kStep) C[k] = __dmul_rn(md, max0(amounts[k][i]));
+    team_sync<TEAM>();
     double sum = 0.0;
     if (lane == 0) {
 #pragma unroll 4
         for (int k = 0; k < K - 1; k++) sum += C[k];
     }
-    sum = __shfl_sync(0xffffffffu, sum, 0);
+    sum = team_value<TEAM>(sum, sh + 3 * K, lane);
     c.Ctot = __dmul_rn(pressure_R, c.rcpT);
     const double S = sum > c.Ctot ? sum : c.Ctot;
     if (!(S > 1e-200 && S < 1e200 && c.Ctot > 0.0)) return false;
     if (lane == 0) C[K - 1] = c.Ctot - sum;
-    __syncwarp();
+    team_sync<TEAM>();
     const int ex = exponent_above_x(S);
     c.m_q = H.eff_shift + 6 - ex;
     c.ctot = dbl_to_fix(c.Ctot, c.m_q);
     c.t = make_temps(H, T, c.rcpT);
     c.C = C;
     c.g = g;
-    for (int k = lane; k < K; k += 32) {
+    for (int k = lane; k < K; k += kStep) {
         const Word2 w = split_word(dbl_to_fix(C[k], kCq + kLo - ex));
         cw[k] = __hiloint2double(w.hi, w.lo);
         if (k < A && (tb.species[k].need_exp | tb.species[k].need_exp_neg)) g[k] = gibbs_log2(tb.species[k], c.t);
     }
-    __syncwarp();
-    for (int e = lane; e < H.n_eff; e += 32) {
+    team_sync<TEAM>();
+    for (int e = lane; e < H.n_eff; e += kStep) {
         const Word2* E = tb.eff + (size_t)e * K;
         long long s1 = 0, s2 = 0;
 #pragma unroll 4
         for (int k = 0; k < K; k++) dot_term(E[k], Word2{__double2hiint(cw[k]), __double2loint(cw[k])}, s1, s2);
         M[e] = third_body(c, s1, s2);
     }
-    __syncwarp();
+    team_sync<TEAM>();
     const int first = H.group_end[1];
+    int turn = 0;  // the warp that takes the model's first 32 reactions
 #pragma unroll 1
     for (int m = 0; m < 6; m++) {  // one model's program at a time
+        const int begin = m ? H.group_end[m - 1] : 0;
+        const int mine = TEAM == 1 ? 0 : ((lane >> 5) - turn + TEAM) % TEAM;
+        if (TEAM > 1) turn = (turn + (H.group_end[m] - begin + 31) / 32) % TEAM;
 #pragma unroll 1
-        for (int r = (m ? H.group_end[m - 1] : 0) + lane; r < H.group_end[m]; r += 32) {
+        for (int r = begin + 32 * mine + (lane & 31); r < H.group_end[m]; r += kStep) {
             auto store = [&](int, double v) { cR[r] = v; };
             if (m == 1) {
                 reaction_x<false, false>(tb, r, c, nullptr, [&](const ArrheniusX& k) { return rate_constant(k, c.t); }, store);
@@ -297,21 +304,22 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
             }
         }
     }
-    __syncwarp();
+    team_sync<TEAM>();
     return true;
 }
 
-template <int KMAX>
+template <int TEAM, int KMAX>
 __device__ __forceinline__ bool rates_cell_warp(const RatesXTables& tb, const RatesArgs<KMAX>& io, size_t i, double* sh,
                                                 int lane) {
+    constexpr int kStep = 32 * TEAM;
     const RatesXHeader& H = *tb.H;
     const int K = H.K, A = H.A;
     const bool uniform = io.flags & kUniformPressure;
     const double T = io.in[2][i], V = io.in[3][i], rcp_pressure_R = uniform ? io.in[1][0] : io.in[1][i];
     CellXW<KMAX> c;
-    if (!cell_progress_warp<KMAX>(tb, uniform ? io.in[0][0] : io.in[0][i], T, V, io.in + 4, i, sh, lane, c)) return false;
+    if (!cell_progress_warp<TEAM, KMAX>(tb, uniform ? io.in[0][0] : io.in[0][i], T, V, io.in + 4, i, sh, lane, c)) return false;
     double *C = sh, *h = sh + K, *cp = sh + 2 * K, *w = sh + 3 * K, *cR = sh + 4 * K + H.n_eff;
-    for (int k = lane; k < K; k += 32) {
+    for (int k = lane; k < K; k += kStep) {
         if (k < A) {
             double v = 0.0;
             const int end = tb.csr_start[k + 1];
@@ -328,7 +336,7 @@ __device__ __forceinline__ bool rates_cell_warp(const RatesXTables& tb, const Ra
         if (k < A) h[k] = enthalpy_x(s, set, c.t);
         cp[k] = heat_capacity_x(s, set, c.t);
     }
-    __syncwarp();
+    team_sync<TEAM>();
     double acc = 0.0;  // E, Cp and dtE on lanes 0, 1, 2
     if (lane < 3) {
         const int n = lane == 1 ? K : A;
@@ -343,29 +351,37 @@ __device__ __forceinline__ bool rates_cell_warp(const RatesXTables& tb, const Ra
         io.out[0][i] = T * dtT_T;
         io.out[1][i] = V * fma(rcp_pressure_R * T, dtE, dtT_T);
     }
-    __syncwarp();  // the scratch is the warp's next cell's
+    team_sync<TEAM>();  // the scratch is the warp's next cell's
     return true;
 }
 
-template <int KMAX>
+template <int TEAM, int KMAX>
 __device__ __forceinline__ bool reaction_rates_cell_warp(const RatesXTables& tb, const ReactionRatesArgs<KMAX>& io, size_t i,
                                                          double* sh, int lane) {
+    constexpr int kStep = 32 * TEAM;
     CellXW<KMAX> c;
-    if (!cell_progress_warp<KMAX>(tb, io.in[0][i], io.in[1][i], io.in[2][i], io.in + 3, i, sh, lane, c)) return false;
+    if (!cell_progress_warp<TEAM, KMAX>(tb, io.in[0][i], io.in[1][i], io.in[2][i], io.in + 3, i, sh, lane, c)) return false;
     const double* cR = sh + 4 * tb.H->K + tb.H->n_eff;
-    for (int r = lane; r < tb.H->R; r += 32) io.out[tb.reactions[r].orig][i] = cR[r];
-    __syncwarp();
+    for (int r = lane; r < tb.H->R; r += kStep) io.out[tb.reactions[r].orig][i] = cR[r];
+    team_sync<TEAM>();
     return true;
 }
 
 // The warp's cells; those that need the FP64 form are put off until there are 32, one per lane.
-template <bool SMEM, class Cell, class F64>
+template <bool SMEM, int TEAM, class Cell, class F64>
 __device__ __forceinline__ void warp_cells(const uint8_t* gtab, uint32_t tab_bytes, size_t n, int* status, Cell cell, F64 f64) {
     __shared__ uint64_t bar;
     if (!stage_x<SMEM>(gtab, tab_bytes, &bar, status)) return;
     const RatesXTables tb(SMEM ? cb_dsmem : gtab);
-    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const uint32_t tables = SMEM ? tab_bytes : (uint32_t)(kMathBytes + kFixMathBytes);
+    if (TEAM > 1) {
+        for (size_t i = blockIdx.x; i < n; i += gridDim.x) {
+            if (!cell(tb, i, reinterpret_cast<double*>(cb_dsmem + tables), (int)threadIdx.x) && threadIdx.x == 0) f64(i);
+            __syncthreads();
+        }
+        return;
+    }
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     double* sh = reinterpret_cast<double*>(cb_dsmem + tables) +
                  (size_t)(threadIdx.x >> 5) * (4 * tb.H->K + tb.H->n_eff + tb.H->R);  // rates_warp_bytes
     size_t later = 0;
@@ -383,29 +399,31 @@ __device__ __forceinline__ void warp_cells(const uint8_t* gtab, uint32_t tab_byt
     if (lane < put_off) f64(later);
 }
 
-template <int KMAX, bool SMEM>
-__global__ void __launch_bounds__(32 * kRatesWarps) rates_x_warp_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
+template <int KMAX, bool SMEM, int TEAM>
+__global__ void __launch_bounds__(32 * (TEAM > 1 ? TEAM : kRatesWarps)) rates_x_warp_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                                                       const __grid_constant__ RatesArgs<KMAX> io, size_t n,
                                                                       int* status) {
     let_next_start();
-    warp_cells<SMEM>(
+    warp_cells<SMEM, TEAM>(
         gtab, tab_bytes, n, status,
-        [&](const RatesXTables& tb, size_t i, double* sh, int lane) { return rates_cell_warp<KMAX>(tb, io, i, sh, lane); },
+        [&](const RatesXTables& tb, size_t i, double* sh, int lane) { return rates_cell_warp<TEAM, KMAX>(tb, io, i, sh, lane); },
         [&](size_t i) { rates_cell_f64<KMAX>(io, i); });
 }
-template <int KMAX, bool SMEM>
-__global__ void __launch_bounds__(32 * kRatesWarps)
+template <int KMAX, bool SMEM, int TEAM>
+__global__ void __launch_bounds__(32 * (TEAM > 1 ? TEAM : kRatesWarps))
     reaction_rates_x_warp_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                  const __grid_constant__ ReactionRatesArgs<KMAX> io, size_t n, int* status) {
-    warp_cells<SMEM>(
+    warp_cells<SMEM, TEAM>(
         gtab, tab_bytes, n, status,
         [&](const RatesXTables& tb, size_t i, double* sh, int lane) {
-            return reaction_rates_cell_warp<KMAX>(tb, io, i, sh, lane);
+            return reaction_rates_cell_warp<TEAM, KMAX>(tb, io, i, sh, lane);
         },
         [&](size_t i) { reaction_rates_cell_f64<KMAX>(io, i); });
 }
 
 namespace {
+// Calls of up to a cell per SM go one cell per block of eight warps (one state: 10 species 34 -> 25 us, 53 species 35 ->
+// 23, 250 species 391 -> 138: the reactions' eleven (48) rounds become two (six); the FP64 sums stay on one lane).
 // Calls of up to this many cells per SM go one cell per warp. A thread's cell takes 60, 500 and 5,000 us however few
 // there are (10, 53, 250 species), a warp's 34, 66 and 410 us and then 12, 24 and 360 ns per cell (bound by the FP64
 // chains that run on one lane); beyond these lines the thread form is the faster.
@@ -415,8 +433,12 @@ constexpr size_t kWarpCellsPerSmR = KMAX == 16 ? 32 : KMAX == 64 ? 150 : 100;
 template <int KMAX>
 cudaError_t launch_rates_xk(const uint8_t* tab, uint32_t tab_bytes, const RatesArgs<KMAX>& io, size_t n, size_t warp_bytes,
                             cudaStream_t st, int* status) {
-    if (n <= (size_t)sm_count() * kWarpCellsPerSmR<KMAX> && 4 * warp_bytes + 32768 <= (size_t)max_table_smem())
-        return launch_warp_kernel<kRatesWarps>(rates_x_warp_kernel<KMAX, true>, rates_x_warp_kernel<KMAX, false>, tab, tab_bytes, io, n,
+    const bool fits = 4 * warp_bytes + 32768 <= (size_t)max_table_smem();
+    if (n <= (size_t)sm_count() && fits)
+        return launch_team_kernel<kTeamWarps>(rates_x_warp_kernel<KMAX, true, kTeamWarps>, rates_x_warp_kernel<KMAX, false, kTeamWarps>,
+                                              tab, tab_bytes, io, n, kMathBytes + kFixMathBytes, warp_bytes, st, status);
+    if (n <= (size_t)sm_count() * kWarpCellsPerSmR<KMAX> && fits)
+        return launch_warp_kernel<kRatesWarps>(rates_x_warp_kernel<KMAX, true, 1>, rates_x_warp_kernel<KMAX, false, 1>, tab, tab_bytes, io, n,
                                                kMathBytes + kFixMathBytes, warp_bytes, st, status);
     return launch_table_kernel<kRatesXBlock>(rates_x_kernel<KMAX, true>, rates_x_kernel<KMAX, false>, tab, tab_bytes, io, n,
                                              kMathBytes + kFixMathBytes, true, st, status);
@@ -424,8 +446,13 @@ cudaError_t launch_rates_xk(const uint8_t* tab, uint32_t tab_bytes, const RatesA
 template <int KMAX>
 cudaError_t launch_reaction_rates_xk(const uint8_t* tab, uint32_t tab_bytes, const ReactionRatesArgs<KMAX>& io, size_t n,
                                      size_t warp_bytes, cudaStream_t st, int* status) {
-    if (n <= (size_t)sm_count() * kWarpCellsPerSmR<KMAX> && 4 * warp_bytes + 32768 <= (size_t)max_table_smem())
-        return launch_warp_kernel<kRatesWarps>(reaction_rates_x_warp_kernel<KMAX, true>, reaction_rates_x_warp_kernel<KMAX, false>, tab,
+    const bool fits = 4 * warp_bytes + 32768 <= (size_t)max_table_smem();
+    if (n <= (size_t)sm_count() && fits)
+        return launch_team_kernel<kTeamWarps>(reaction_rates_x_warp_kernel<KMAX, true, kTeamWarps>,
+                                              reaction_rates_x_warp_kernel<KMAX, false, kTeamWarps>, tab, tab_bytes, io, n,
+                                              kMathBytes + kFixMathBytes, warp_bytes, st, status);
+    if (n <= (size_t)sm_count() * kWarpCellsPerSmR<KMAX> && fits)
+        return launch_warp_kernel<kRatesWarps>(reaction_rates_x_warp_kernel<KMAX, true, 1>, reaction_rates_x_warp_kernel<KMAX, false, 1>, tab,
                                                tab_bytes, io, n, kMathBytes + kFixMathBytes, warp_bytes, st, status);
     return launch_table_kernel<kRatesXBlock>(reaction_rates_x_kernel<KMAX, true>, reaction_rates_x_kernel<KMAX, false>, tab,
                                              tab_bytes, io, n, kMathBytes + kFixMathBytes, true, st, status);

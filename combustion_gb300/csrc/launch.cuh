@@ -104,6 +104,20 @@ cudaError_t launch_warp_kernel(KS ksmem, KG kglobal, const uint8_t* tab, uint32_
                 : launch_one(kglobal, grid, 32 * warps, bytes, st, tab, tab_bytes, io, n, status);
 }
 
+// One cell per block of TEAM warps, for calls of at most a cell per SM.
+constexpr int kTeamWarps = 8;
+template <int TEAM, class KS, class KG, class Args>
+cudaError_t launch_team_kernel(KS ksmem, KG kglobal, const uint8_t* tab, uint32_t tab_bytes, const Args& io, size_t n,
+                               uint32_t math, size_t cell_bytes, cudaStream_t st, int* status) {
+    const bool smem = tab_bytes + cell_bytes <= (size_t)max_table_smem();
+    const size_t bytes = (smem ? tab_bytes : math) + cell_bytes, grid = n ? n : 1;
+    cudaError_t e = smem ? cudaFuncSetAttribute(ksmem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
+                         : cudaFuncSetAttribute(kglobal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    return smem ? launch_one(ksmem, grid, 32 * TEAM, bytes, st, tab, tab_bytes, io, n, status)
+                : launch_one(kglobal, grid, 32 * TEAM, bytes, st, tab, tab_bytes, io, n, status);
+}
+
 template <int BLOCK, class KS, class KG>
 size_t wave_of(KS ksmem, KG kglobal, uint32_t tab_bytes, uint32_t math_bytes) {
     int per_sm = 1;
