@@ -227,10 +227,15 @@ __global__ void __launch_bounds__(kTransportXBlock<KMAX>) transport_x_kernel(con
 
 // ---------------------------------------------------------------------------------------------------
 // One cell per warp, every sum in the thread form's order (transport_cell_warp's division of the work).
+// TEAM warps (a block of its own) share the cell in calls of at most a cell per SM, 1 otherwise.
 template <int KMAX>
+constexpr size_t kTeamScratch = 4 * KMAX + 32 * (KMAX + 1) > kWarpScratch<KMAX> ? 4 * KMAX + 32 * (KMAX + 1) : kWarpScratch<KMAX>;
+
+template <int TEAM, int KMAX>
 __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb, const TransportArgs<KMAX>& io, size_t i,
                                                       size_t o, double* sh, bool second) {
-    const int lane = threadIdx.x & 31;
+    constexpr int kStep = 32 * TEAM;
+    const int lane = TEAM == 1 ? threadIdx.x & 31 : threadIdx.x, lane32 = threadIdx.x & 31;
     const TransportXHeader& H = *tb.H;
     const int K = H.K;
     double N, Tn;
@@ -242,11 +247,11 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
     double* Z = sh + 3 * KMAX;
     double* T = sh + 4 * KMAX;
     int mx = 0;
-    for (int k = lane; k < K - 1; k += 32) {
+    for (int k = lane; k < K - 1; k += kStep) {
         X[k] = amounts[k][i];
         mx = max(mx, __double2hiint(X[k]) & 0x7fffffff);
     }
-    __syncwarp();
+    team_sync<TEAM>();
     double xb = 0.0;
     if (lane == 0) {
         double s = 0.0;
@@ -255,18 +260,20 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
         X[K - 1] = xb;
         mx = max(mx, __double2hiint(xb) & 0x7fffffff);
     }
-    __syncwarp();
+    team_sync<TEAM>();
+    if (TEAM > 1)  // every warp over all species
+        for (int k = lane32; k < K; k += 32) mx = max(mx, __double2hiint(X[k]) & 0x7fffffff);
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (mx < 0x20ca2fe7 || mx >= 0x5f138d35 || !(N - N == 0.0)) return false;
     const PowersX L = log_powers(H, Tn);
     const double VT = sqrt(Tn);
-    for (int k = lane; k < K; k += 32) {
+    for (int k = lane; k < K; k += kStep) {
         const PolyX P = tb.cond[k];
         const long long d = poly_x(P, L);
         v[k] = fix_to_dbl(d, kDq - P.sp);
         Y[k] = rcp_fixed(d, P.rcp_bias);
     }
-    __syncwarp();
+    team_sync<TEAM>();
     double acc = 0.0;  // lanes 0-2: the even species of the three sums, lanes 3-5: the odd ones
     if (lane < 6) {
         const double* src = lane % 3 == 0 ? tb.W : lane % 3 == 1 ? v : Y;
@@ -274,14 +281,14 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
         for (int k = lane / 3; k < K; k += 2) acc = fma(src[k], X[k], acc);
     }
     acc += __shfl_sync(0xffffffffu, acc, (lane + 3) & 31);  // used by lanes 0-2
-    const double MN = __shfl_sync(0xffffffffu, acc, 0);
+    const double MN = team_value<TEAM>(acc, T, lane);
     const double Ac = __shfl_sync(0xffffffffu, acc, 1);
     const double Bc = __shfl_sync(0xffffffffu, acc, 2);
-    __syncwarp();
+    team_sync<TEAM>();
     if (lane == 0) transport_out(io, 0, second)[o] = conductivity_of(Ac, Bc, N, VT);
 
     int my = 0, mz = 0;
-    for (int k = lane; k < K; k += 32) {
+    for (int k = lane; k < K; k += kStep) {
         const PolyX P = tb.visc[k];
         v[k] = rcp_fixed(poly_x(P, L), P.rcp_bias);  // 1 / v'
         Y[k] = __dmul_rn(X[k], v[k]);
@@ -289,23 +296,31 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
         my = max(my, __double2hiint(Y[k]) & 0x7fffffff);
         mz = max(mz, __double2hiint(Z[k]) & 0x7fffffff);
     }
+    if (TEAM > 1) {
+        __syncthreads();
+        for (int k = lane32; k < K; k += 32) {
+            my = max(my, __double2hiint(Y[k]) & 0x7fffffff);
+            mz = max(mz, __double2hiint(Z[k]) & 0x7fffffff);
+        }
+        __syncthreads();
+    }
     my = __reduce_max_sync(0xffffffffu, my);
     mz = __reduce_max_sync(0xffffffffu, mz);
     const int qx = kMixXq<KMAX> - exponent_above(mx), qy = kMixXq<KMAX> - exponent_above(my),
               qz = kMixXq<KMAX> - exponent_above(mz);
     double* Xw = T;  // the tile holds X's words and the viscosity terms until the diffusion
     double* U = T + KMAX;
-    for (int k = lane; k < K; k += 32) {
+    for (int k = lane; k < K; k += kStep) {
         const Word2 x = split_word(dbl_to_fix(X[k], qx)), y = split_word(dbl_to_fix(Y[k], qy)),
                     z = split_word(dbl_to_fix(Z[k], qz));
         Xw[k] = __hiloint2double(x.hi, x.lo);
         Y[k] = __hiloint2double(y.hi, y.lo);
         Z[k] = __hiloint2double(z.hi, z.lo);
     }
-    __syncwarp();
+    team_sync<TEAM>();
     const int unit = H.a_shift + 1 - 2 * kLo;
 #pragma unroll 1
-    for (int k = lane; k < K; k += 32) {
+    for (int k = lane; k < K; k += kStep) {
         const Word2* a = tb.A2 + k;
         long long s[3] = {0, 0, 0}, t[3] = {0, 0, 0};
 #pragma unroll 2
@@ -319,7 +334,7 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
         U[2 * k + 1] = wilke_rcp(mix_value(s[0], t[0]), mix_value(s[1], t[1]), mix_value(s[2], t[2]), unit + qx, unit + qy,
                                  unit + qz, v[k]);
     }
-    __syncwarp();
+    team_sync<TEAM>();
     double mu = 0.0;
     if (lane < 2) {
 #pragma unroll 4
@@ -327,11 +342,55 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
     }
     mu += __shfl_sync(0xffffffffu, mu, 1);
     if (lane == 0) transport_out(io, 1, second)[o] = VT * mu;
-    __syncwarp();
+    team_sync<TEAM>();
 
     // Diffusion, in tiles of 32 rows by 32 columns of pairs: lanes on consecutive pairs of a row (consecutive table
     // records) leave the reciprocals in the tile, then lanes on rows add theirs, then lanes on columns.
     double* S = Y;
+    if (TEAM > 1) {  // bands of 32 rows: all warps evaluate the pairs, one adds the rows' sums, the others the columns'
+        constexpr int LD = KMAX + 1;
+        for (int base = 0; base < K; base += 32) {
+            const int rows = min(32, K - base);
+            for (int q = lane >> 5; q < rows; q += TEAM) {
+                const int k = base + q;
+                const PolyX* P = tb.diff + (size_t)k * (k - 1) / 2;
+#pragma unroll 2
+                for (int c = lane32; c < k; c += 32) {
+                    const PolyX p = P[c];
+                    T[q * LD + c] = rcp_fixed(poly_x(p, L), p.rcp_bias);
+                }
+            }
+            __syncthreads();
+            if (lane < 32) {
+                if (lane < rows) {
+                    const int k = base + lane;
+                    const double* Trow = T + lane * LD;
+                    double sa = 0.0, sb = 0.0;
+                    int c = 0;
+#pragma unroll 4
+                    for (; c + 1 < k; c += 2) {
+                        sa = fma(X[c], Trow[c], sa);
+                        sb = fma(X[c + 1], Trow[c + 1], sb);
+                    }
+                    if (c < k) sa = fma(X[c], Trow[c], sa);
+                    double s1 = sa + sb;
+                    for (int q = lane + 1; q < rows; q++) s1 = fma(X[base + q], T[q * LD + k], s1);
+                    S[k] = s1;
+                }
+            } else {
+                for (int c = lane - 32; c < base; c += kStep - 32) {
+                    double s1 = S[c];
+#pragma unroll 4
+                    for (int q = 0; q < rows; q++) s1 = fma(X[base + q], T[q * LD + c], s1);
+                    S[c] = s1;
+                }
+            }
+            __syncthreads();
+        }
+        for (int k = lane; k < K; k += kStep)
+            transport_out(io, 2 + k, second)[o] = diffusion_x(MN, VT, tb.W[k], X[k], S[k]);
+        return true;
+    }
 #pragma unroll 1
     for (int b = 0; 32 * b < K; b++) {
         const int r = 32 * b + lane, rows = min(32, K - 32 * b);
@@ -409,7 +468,7 @@ __global__ void __launch_bounds__(32 * kWarpCellWarpsX) transport_x_warp_kernel(
         const bool second = io.index2 && j >= io.n1;
         const size_t i = second ? (size_t)(io.index2[j - io.n1] & kIndexMask) : io.index ? (size_t)(io.index[j] & kIndexMask) : j;
         const size_t o = second ? j - io.n1 : (io.flags & kCompactOut) ? j : i;
-        if (!transport_cell_x_warp<KMAX>(tb, io, i, o, sh, second)) {
+        if (!transport_cell_x_warp<1, KMAX>(tb, io, i, o, sh, second)) {
             __syncwarp();
             transport_cell_f64_warp<KMAX>(io, i, o, sh, second);
         }
@@ -417,7 +476,35 @@ __global__ void __launch_bounds__(32 * kWarpCellWarpsX) transport_x_warp_kernel(
     }
 }
 
+template <int KMAX, bool SMEM>
+__global__ void __launch_bounds__(32 * kTeamWarps) transport_x_team_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
+                                                                           const __grid_constant__ TransportArgs<KMAX> io,
+                                                                           size_t n, int* status) {
+    const EndAfterPrevious last;
+    __shared__ uint64_t bar;
+    if (SMEM) {
+        if (!stage_to_shared(cb_dsmem, gtab, tab_bytes, &bar, status)) return;
+    } else {
+        load_math(gtab);
+    }
+    const TransportXTables tb(SMEM ? cb_dsmem : gtab);
+    double* sh = reinterpret_cast<double*>(cb_dsmem + warp_table_bytes(SMEM, tab_bytes));
+    if (io.count && !io.index2) n = min(n, (size_t)*io.count);
+    for (size_t j = blockIdx.x; j < n; j += gridDim.x) {
+        const bool second = io.index2 && j >= io.n1;
+        const size_t i = second ? (size_t)(io.index2[j - io.n1] & kIndexMask) : io.index ? (size_t)(io.index[j] & kIndexMask) : j;
+        const size_t o = second ? j - io.n1 : (io.flags & kCompactOut) ? j : i;
+        const bool done = transport_cell_x_warp<kTeamWarps, KMAX>(tb, io, i, o, sh, second);
+        __syncthreads();
+        if (!done && threadIdx.x < 32) transport_cell_f64_warp<KMAX>(io, i, o, sh, second);
+        __syncthreads();  // the scratch is reused by the block's next cell
+    }
+}
+
 namespace {
+// Calls and gathered launches of up to a cell per SM go one cell per block of eight warps: one state 27, 70 -> 53 and
+// 700 -> 205 us (10, 53, 250 species), where Wilke's rows and the pairs of a band of rows take all lanes at once; the
+// sums keep their lanes and order.
 // Calls and gathered launches of up to this many cells per SM go one cell per warp: a thread's cell takes 55, 460 and
 // 18,000 us however few there are (10, 53, 250 species), a warp's 30, 70 and 660 us and then 9, 34 and 480 ns per
 // cell; beyond these lines the thread form is the faster.
@@ -427,6 +514,15 @@ constexpr size_t kWarpCellsPerSmX = KMAX == 16 ? 24 : KMAX == 64 ? 96 : 256;
 template <int KMAX>
 cudaError_t launch_transport_xk(const uint8_t* tab, uint32_t tab_bytes, const TransportArgs<KMAX>& io, size_t n,
                                 cudaStream_t st, int* status) {
+    if (n <= (size_t)sm_count()) {
+        const size_t scratch = kTeamScratch<KMAX> * sizeof(double);
+        const bool smem = warp_table_bytes(true, tab_bytes) + scratch <= (size_t)max_table_smem();
+        const size_t bytes = warp_table_bytes(smem, tab_bytes) + scratch;
+        auto kern = smem ? transport_x_team_kernel<KMAX, true> : transport_x_team_kernel<KMAX, false>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+        return launch_one(kern, n, 32 * kTeamWarps, bytes, st, tab, tab_bytes, io, n, status);
+    }
     if (n <= (size_t)sm_count() * kWarpCellsPerSmX<KMAX>) {
         const size_t share = (n + sm_count() - 1) / sm_count(), scratch = kWarpScratch<KMAX> * sizeof(double);
         const bool smem = warp_table_bytes(true, tab_bytes) + 4 * scratch <= (size_t)max_table_smem();
