@@ -27,17 +27,22 @@ struct CellMW {
 template <>
 constexpr bool kBatchLoads<CellMW> = true;
 
-template <int MODEL>
+// turn: the warp that takes the model's first 32 reactions.
+template <int TEAM, int MODEL>
 __device__ __forceinline__ void progress_group_m(const RatesMixedTables& tb, const CellMW& c, const float* Mf, double* cR,
-                                                 int lane) {
-    for (int r = (MODEL ? tb.H->group_end[MODEL - 1] : 0) + lane; r < tb.H->group_end[MODEL]; r += 32) {
+                                                 int lane, int& turn) {
+    const int begin = MODEL ? tb.H->group_end[MODEL - 1] : 0, end = tb.H->group_end[MODEL];
+    const int mine = TEAM == 1 ? 0 : ((lane >> 5) - turn + TEAM) % TEAM;
+    if (TEAM > 1) turn = (turn + (end - begin + 31) / 32) % TEAM;
+    for (int r = begin + 32 * mine + (lane & 31); r < end; r += 32 * TEAM) {
         const ReactionF& x = tb.reactions[r];
         cR[r] = reaction_rate_m<MODEL>(tb, x, c, MODEL >= 2 ? Mf[x.eff_row] : 0.f);
     }
 }
 
 // rates_mixed_cell. sh: rates_warp_bytes of scratch. csr: per species its reactions and net coefficients in order.
-template <int KMAX>
+// TEAM warps (a block of its own) share the cell in calls of at most a cell per SM, 1 otherwise.
+template <int TEAM, int KMAX>
 __device__ void rates_mixed_cell_warp(const RatesMixedTables& tb, const int* csr_start, const int* csr,
                                       const RatesArgs<KMAX>& io, size_t i, double* sh, int lane) {
     const RatesMixedHeader& H = *tb.H;
@@ -50,11 +55,13 @@ __device__ void rates_mixed_cell_warp(const RatesMixedTables& tb, const int* csr
     float* Mf = reinterpret_cast<float*>(sh + 4 * K);
     const double md = rcp64(V), rcpT = rcp64(T), lnT = log64(T);
     const double T2 = T * T, T3 = T * T2, T4 = T2 * T2;
-    for (int k = lane; k < K - 1; k += 32) C[k] = __dmul_rn(md, max0(io.in[4 + k][i]));
-    __syncwarp();
+    for (int k = lane; k < K - 1; k += 32 * TEAM) C[k] = __dmul_rn(md, max0(io.in[4 + k][i]));
+    team_sync<TEAM>();
     double sum = 0.0;
+    if (lane < 32) {
 #pragma unroll 4
-    for (int k = 0; k < K - 1; k++) sum += C[k];
+        for (int k = 0; k < K - 1; k++) sum += C[k];
+    }
     const double Ctot = __dmul_rn(pressure_R, rcpT);
     CellMW c;
     c.Ctotf = dbl_to_flt(Ctot);
@@ -68,31 +75,32 @@ __device__ void rates_mixed_cell_warp(const RatesMixedTables& tb, const int* csr
     c.ex = ex;
     c.exn = exn;
     if (lane == 0) C[K - 1] = Ctot - sum;
-    for (int k = lane; k < A; k += 32) {
+    for (int k = lane; k < A; k += 32 * TEAM) {
         const SpeciesF& s = tb.species[k];
         if (!(s.need_exp | s.need_exp_neg)) continue;
         const double* g = s.g[piece_of_m(s.split, T)];
         const double x = fma(g[6], rcpT, fma(g[5], T4, fma(g[4], T3, fma(g[3], T2, fma(g[2], T, fma(g[1], lnT, g[0]))))));
         gibbs_exps(x, s.need_exp, s.need_exp_neg, H.M3, H.cbrt_max, c.C0, c.rcpC0, ex[k], exn[k]);
     }
-    __syncwarp();
-    for (int e = lane; e < H.n_eff; e += 32) {
+    team_sync<TEAM>();
+    for (int e = lane; e < H.n_eff; e += 32 * TEAM) {
         const float* E = tb.eff + (size_t)e * K;
         float s = 0.f;
 #pragma unroll 4
         for (int k = 0; k < K; k++) s = fmaf(E[k], dbl_to_flt(C[k]), s);
         Mf[e] = c.Ctotf + s;
     }
-    __syncwarp();
-    progress_group_m<0>(tb, c, Mf, cR, lane);
-    progress_group_m<1>(tb, c, Mf, cR, lane);
-    progress_group_m<2>(tb, c, Mf, cR, lane);
-    progress_group_m<3>(tb, c, Mf, cR, lane);
-    progress_group_m<4>(tb, c, Mf, cR, lane);
-    progress_group_m<5>(tb, c, Mf, cR, lane);
-    __syncwarp();
+    team_sync<TEAM>();
+    int turn = 0;
+    progress_group_m<TEAM, 0>(tb, c, Mf, cR, lane, turn);
+    progress_group_m<TEAM, 1>(tb, c, Mf, cR, lane, turn);
+    progress_group_m<TEAM, 2>(tb, c, Mf, cR, lane, turn);
+    progress_group_m<TEAM, 3>(tb, c, Mf, cR, lane, turn);
+    progress_group_m<TEAM, 4>(tb, c, Mf, cR, lane, turn);
+    progress_group_m<TEAM, 5>(tb, c, Mf, cR, lane, turn);
+    team_sync<TEAM>();
     double *hk = ex, *cpk = exn;
-    for (int k = lane; k < K; k += 32) {
+    for (int k = lane; k < K; k += 32 * TEAM) {
         const SpeciesF& s = tb.species[k];
         const int p = piece_of_m(s.split, T);
         const float Tf = c.Tf, *cp = s.cp[p], *h = s.h[p];
@@ -106,7 +114,7 @@ __device__ void rates_mixed_cell_warp(const RatesMixedTables& tb, const int* csr
         w[k] = wk;
         io.out[2 + k][i] = wk;
     }
-    __syncwarp();
+    team_sync<TEAM>();
     double acc = 0.0;  // E, Cp and dtE on lanes 0, 1, 2
     if (lane < 3) {
         const int n = lane == 1 ? K : A;
@@ -121,7 +129,7 @@ __device__ void rates_mixed_cell_warp(const RatesMixedTables& tb, const int* csr
         io.out[0][i] = T * dtT_T;
         io.out[1][i] = V * fma(rcp_pressure_R * T, dtE, dtT_T);
     }
-    __syncwarp();  // the scratch is the warp's next cell's
+    team_sync<TEAM>();  // the scratch is the warp's next cell's
 }
 
 // The tables into shared memory, or only the functions' (the rest is then read through L1).
@@ -134,8 +142,8 @@ __device__ __forceinline__ bool stage_m(const uint8_t* gtab, uint32_t tab_bytes,
 
 constexpr int kMixedWarps = 16;  // cells per block at most
 
-template <int KMAX, bool SMEM>
-__global__ void __launch_bounds__(32 * kMixedWarps) rates_mixed_warp_kernel(const uint8_t* __restrict__ gtab,
+template <int KMAX, bool SMEM, int TEAM>
+__global__ void __launch_bounds__(32 * (TEAM > 1 ? TEAM : kMixedWarps)) rates_mixed_warp_kernel(const uint8_t* __restrict__ gtab,
                                                                             uint32_t tab_bytes,
                                                                             const __grid_constant__ RatesArgs<KMAX> io,
                                                                             size_t n, int* status) {
@@ -144,16 +152,18 @@ __global__ void __launch_bounds__(32 * kMixedWarps) rates_mixed_warp_kernel(cons
     if (!stage_m<SMEM>(gtab, tab_bytes, &bar, status)) return;
     const RatesMixedTables tb(SMEM ? cb_dsmem : gtab);
     const int *csr_start = reinterpret_cast<const int*>(gtab + tb.H->total_bytes), *csr = csr_start + tb.H->A + 1;
-    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    // the block's cells: as many as it has warps, or one
+    const int lane = TEAM > 1 ? threadIdx.x : threadIdx.x & 31, slot = TEAM > 1 ? 0 : threadIdx.x >> 5;
+    const int cells = TEAM > 1 ? 1 : blockDim.x >> 5;
     double* sh = reinterpret_cast<double*>(cb_dsmem + (SMEM ? tab_bytes : (uint32_t)kMathBytes)) +
-                 (size_t)(threadIdx.x >> 5) * (4 * tb.H->K + tb.H->n_eff + tb.H->R);  // rates_warp_bytes
-    for (size_t i = (size_t)blockIdx.x * warps + (threadIdx.x >> 5); i < n; i += (size_t)gridDim.x * warps)
-        rates_mixed_cell_warp<KMAX>(tb, csr_start, csr, io, i, sh, lane);
+                 (size_t)slot * (4 * tb.H->K + tb.H->n_eff + tb.H->R);  // rates_warp_bytes
+    for (size_t i = (size_t)blockIdx.x * cells + slot; i < n; i += (size_t)gridDim.x * cells)
+        rates_mixed_cell_warp<TEAM, KMAX>(tb, csr_start, csr, io, i, sh, lane);
 }
 
 // ---------------------------------------------------------------------------------------------------
 // transport_mixed_cell, in six arrays of K floats.
-template <int KMAX>
+template <int TEAM, int KMAX>
 __device__ void transport_mixed_cell_warp(const uint8_t* tab, const TransportArgs<KMAX>& io, size_t i, size_t o, float* sh,
                                           int lane) {
     const TransportMixedHeader& H = *reinterpret_cast<const TransportMixedHeader*>(tab + kMathBytes);
@@ -179,14 +189,14 @@ __device__ void transport_mixed_cell_warp(const uint8_t* tab, const TransportArg
     const float L1 = logf(Tn), L2 = L1 * L1, L3 = L2 * L1, L4 = L3 * L1;
     auto poly = [&](const float* P) { return fmaf(P[4], L4, fmaf(P[3], L3, fmaf(P[2], L2, fmaf(P[1], L1, P[0])))); };
     float *X = sh, *v = sh + K, *Y = sh + 2 * K, *Z = sh + 3 * K, *a = sh + 4 * K, *b = sh + 5 * K;
-    for (int k = lane; k < K; k += 32) {
+    for (int k = lane; k < K; k += 32 * TEAM) {
         if (k < K - 1) X[k] = dbl_to_flt(amounts[k][i]);
         const float c = poly(cond + 5 * k);
         a[k] = c;
         b[k] = rcp_f32(c);
         v[k] = poly(visc + 5 * k);
     }
-    __syncwarp();
+    team_sync<TEAM>();
     float s = 0.f, comp = 0.f;
 #pragma unroll 4
     for (int k = 0; k < K - 1; k++) {
@@ -194,25 +204,25 @@ __device__ void transport_mixed_cell_warp(const uint8_t* tab, const TransportArg
         comp = (t - s) - y;
         s = t;
     }
-    __syncwarp();
+    team_sync<TEAM>();
     if (lane == 0) X[K - 1] = (N - s) + comp;
-    __syncwarp();
-    for (int k = lane; k < K; k += 32) {
+    team_sync<TEAM>();
+    for (int k = lane; k < K; k += 32 * TEAM) {
         const float r = rcp_f32(v[k]), y = X[k] * r;
         Y[k] = y;
         Z[k] = y * r;
     }
     const float VT = sqrtf(Tn);
-    const float* q = lane == 1 ? a : lane == 2 ? b : W;  // sums over X: molar mass, conductivities, their reciprocals
+    const float* q = (lane & 31) == 1 ? a : (lane & 31) == 2 ? b : W;  // sums over X: molar mass, conductivities, their reciprocals
     float acc = 0.f;
 #pragma unroll 4
     for (int k = 0; k < K; k++) acc = fmaf(X[k], q[k], acc);
     const float MN = __shfl_sync(0xffffffffu, acc, 0), Ac = __shfl_sync(0xffffffffu, acc, 1),
                 Bc = __shfl_sync(0xffffffffu, acc, 2);
     const float MVTN = MN * VT;
-    __syncwarp();
+    team_sync<TEAM>();
     if (lane == 0) io.out[0][o] = flt_to_dbl((__fdividef(Ac, N) + __fdividef(N, Bc)) * VT);
-    for (int k = lane; k < K; k += 32) {  // Wilke, a row per lane
+    for (int k = lane; k < K; k += 32 * TEAM) {  // Wilke, a row per lane
         const float4* w = wil + (size_t)k * K;
         float s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll 4
@@ -225,14 +235,14 @@ __device__ void transport_mixed_cell_warp(const uint8_t* tab, const TransportArg
         a[k] = X[k] * (v[k] * v[k]);
         b[k] = rcp_f32(fmaf(v[k], fmaf(v[k], s3, s2), s1));
     }
-    __syncwarp();
+    team_sync<TEAM>();
     float mu = 0.f;
 #pragma unroll 4
     for (int k = 0; k < K; k++) mu = fmaf(a[k], b[k], mu);
     if (lane == 0) io.out[1][o] = flt_to_dbl(VT * mu);
     // Mixture diffusion, a species k per lane: even and odd j < k apart, then j > k in order. Each pair is evaluated for
     // both of its species (4 FMAs and a reciprocal; the pairs of 250 species would take 124 KB per warp).
-    for (int k = lane; k < K; k += 32) {
+    for (int k = lane; k < K; k += 32 * TEAM) {
         const float4* row = diff + (size_t)k * (k - 1);  // pairs (k, 0), two float4 each
         float sa = 0.f, sb = 0.f, S = 0.f;
 #pragma unroll 4
@@ -250,11 +260,11 @@ __device__ void transport_mixed_cell_warp(const uint8_t* tab, const TransportArg
         }
         io.out[2 + k][o] = flt_to_dbl(__fdividef(fmaf(-(VT * W[k]), X[k], MVTN), S));
     }
-    __syncwarp();  // the scratch is the warp's next cell's
+    team_sync<TEAM>();  // the scratch is the warp's next cell's
 }
 
-template <int KMAX, bool SMEM>
-__global__ void __launch_bounds__(32 * kMixedWarps)
+template <int KMAX, bool SMEM, int TEAM>
+__global__ void __launch_bounds__(32 * (TEAM > 1 ? TEAM : kMixedWarps))
     transport_mixed_warp_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                 const __grid_constant__ TransportArgs<KMAX> io, size_t n, int* status) {
     const EndAfterPrevious last;
@@ -262,40 +272,42 @@ __global__ void __launch_bounds__(32 * kMixedWarps)
     if (!stage_m<SMEM>(gtab, tab_bytes, &bar, status)) return;
     const uint8_t* tab = SMEM ? cb_dsmem : gtab;
     if (io.count) n = min(n, (size_t)*io.count);  // gathered cells: the count is known on the device only
-    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    float* sh = reinterpret_cast<float*>(cb_dsmem + (SMEM ? tab_bytes : (uint32_t)kMathBytes)) +
-                (size_t)(threadIdx.x >> 5) * (6 * KMAX);
-    for (size_t j = (size_t)blockIdx.x * warps + (threadIdx.x >> 5); j < n; j += (size_t)gridDim.x * warps) {
+    const int lane = TEAM > 1 ? threadIdx.x : threadIdx.x & 31, slot = TEAM > 1 ? 0 : threadIdx.x >> 5;
+    const int cells = TEAM > 1 ? 1 : blockDim.x >> 5;
+    float* sh = reinterpret_cast<float*>(cb_dsmem + (SMEM ? tab_bytes : (uint32_t)kMathBytes)) + (size_t)slot * (6 * KMAX);
+    for (size_t j = (size_t)blockIdx.x * cells + slot; j < n; j += (size_t)gridDim.x * cells) {
         const size_t i = io.index ? (size_t)(io.index[j] & kIndexMask) : j;
-        transport_mixed_cell_warp<KMAX>(tab, io, i, (io.flags & kCompactOut) ? j : i, sh, lane);
+        transport_mixed_cell_warp<TEAM, KMAX>(tab, io, i, (io.flags & kCompactOut) ? j : i, sh, lane);
     }
 }
 
+// A cell per block of eight warps up to a cell per SM, a cell per warp beyond.
+#define CB_LAUNCH(KERNEL, KM, ARGS, SCRATCH)                                                                             \
+    case KM: {                                                                                                           \
+        const auto& io = *static_cast<const ARGS<KM>*>(args);                                                            \
+        if (n <= (size_t)sm_count())                                                                                     \
+            return launch_team_kernel<kTeamWarps>(KERNEL<KM, true, kTeamWarps>, KERNEL<KM, false, kTeamWarps>, tab, tab_bytes, \
+                                                  io, n, kMathBytes, SCRATCH, st, status);                               \
+        return launch_warp_kernel<kMixedWarps>(KERNEL<KM, true, 1>, KERNEL<KM, false, 1>, tab, tab_bytes, io, n, kMathBytes, \
+                                               SCRATCH, st, status);                                                     \
+    }
 cudaError_t launch_rates_mixed_warp(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                     size_t warp_bytes, cudaStream_t st, int* status) {
-#define CB_ONE(KM)                                                                                                        \
-    case KM:                                                                                                              \
-        return launch_warp_kernel<kMixedWarps>(rates_mixed_warp_kernel<KM, true>, rates_mixed_warp_kernel<KM, false>, tab, \
-                                               tab_bytes, *static_cast<const RatesArgs<KM>*>(args), n, kMathBytes, warp_bytes, \
-                                               st, status);
     switch (kmax) {
-        CB_ONE(16) CB_ONE(64) CB_ONE(256)
+        CB_LAUNCH(rates_mixed_warp_kernel, 16, RatesArgs, warp_bytes)
+        CB_LAUNCH(rates_mixed_warp_kernel, 64, RatesArgs, warp_bytes)
+        CB_LAUNCH(rates_mixed_warp_kernel, 256, RatesArgs, warp_bytes)
     default: return cudaErrorInvalidValue;
     }
-#undef CB_ONE
 }
 cudaError_t launch_transport_mixed_warp(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                         cudaStream_t st, int* status) {
-#define CB_ONE(KM)                                                                                                       \
-    case KM:                                                                                                             \
-        return launch_warp_kernel<kMixedWarps>(transport_mixed_warp_kernel<KM, true>, transport_mixed_warp_kernel<KM, false>, \
-                                               tab, tab_bytes, *static_cast<const TransportArgs<KM>*>(args), n, kMathBytes,  \
-                                               6 * KM * sizeof(float), st, status);
     switch (kmax) {
-        CB_ONE(16) CB_ONE(64) CB_ONE(256)
+        CB_LAUNCH(transport_mixed_warp_kernel, 16, TransportArgs, 6 * 16 * sizeof(float))
+        CB_LAUNCH(transport_mixed_warp_kernel, 64, TransportArgs, 6 * 64 * sizeof(float))
+        CB_LAUNCH(transport_mixed_warp_kernel, 256, TransportArgs, 6 * 256 * sizeof(float))
     default: return cudaErrorInvalidValue;
     }
-#undef CB_ONE
 }
 
 }  // namespace cbg
