@@ -1,6 +1,7 @@
 // The mixed-precision kernels, one cell per warp, for calls too small to fill the GPU with one cell per thread
 // (kernels_mixed.cu): there a call takes as long as one thread needs for its cell, 520 us at 53 species, where a
-// warp needs 67 (10,100 cells: 1,105 -> 315 us; with transport 1,375 -> 394).
+// warp needs 67 (10,100 cells: 1,105 -> 315 us; with transport 1,375 -> 394), and a block of eight warps, for calls
+// of at most a cell per SM, 51 (250 species, rates and transport: 10,400 -> 748 -> 145).
 // The lanes share a cell's species, third-body rows, reactions and rows of the mixture rules; every sum runs in
 // the order of the thread's program, so a cell has the same bits in both forms. What is left is latency: the FP64
 // sums over the species in that order (a quarter of the FP64 pipe's time on one lane each) and eleven rounds of
