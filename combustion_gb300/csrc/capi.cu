@@ -133,8 +133,8 @@ TransportLaunch transport_launch(const cb_mech* m) {
 // kOverlap where the transport of a fused call may run beside its rates: its outputs touch neither the cells nor the
 // rates' outputs (ends of the whole range they span, so rows laid out in between count as touched).
 // The two kernels then fill what the other leaves idle: the SMs a small call does not reach, the last wave, the pipe
-// the other waits for. Rates and transport after / beside each other, us: 53 species 1 cell 107 / 75, 10,100 cells
-// 645 / 590, 160,000 cells 4,310 / 3,580; 250 species 1 cell 1,117 / 783, 60,000 cells 39,500 / 33,100 (mixed precision
+// the other waits for. Rates and transport after / beside each other, us: 53 species 5,000 cells 387 / 328, 10,100 cells
+// 645 / 590, 160,000 cells 4,310 / 3,580; 250 species 300 cells 1,180 / 834, 60,000 cells 39,500 / 33,100 (mixed precision
 // 23,300 / 15,000). Not so for a few cells per SM of the small and the large tables, where both blocks land on one SM
 // and share its L1: 10 species, 3 to 11 cells per SM 60 / 71; 250 species, 4 to 16 (mixed precision 60) per SM 1,143 /
 // 3,220 at worst; nor for many waves of the small ones (10 species, 2^22 cells: 5,563 / 5,611).
