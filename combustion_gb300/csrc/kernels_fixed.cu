@@ -32,6 +32,12 @@ struct CellX {
 // e with S < 2^e, S positive and normal.
 __device__ __forceinline__ int exponent_above_x(double S) { return ((__double2hiint(S) >> 20) & 0x7ff) - 1022; }
 
+// The larger total S is a positive normal number well inside the exponent range and the other one not negative: every
+// concentration is finite and at most S. (False for a NaN sum, of a NaN amount, and for a negative one, of a negative volume.)
+__device__ __forceinline__ bool totals_in_range(double sum, double Ctot, double S) {
+    return sum >= 0.0 && Ctot > 0.0 && S > 1e-200 && S < 1e200;
+}
+
 // Prologue of reaction.rs:362-373; false where the cell needs the FP64 form.
 template <int KMAX>
 __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pressure_R, double T, double V,
@@ -49,9 +55,8 @@ __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pres
         sum += c.C[k];
     }
     c.Ctot = __dmul_rn(pressure_R, c.rcpT);
-    // the larger total must be a positive normal number well inside the exponent range, and the other finite
     const double S = sum > c.Ctot ? sum : c.Ctot;
-    if (!(S > 1e-200 && S < 1e200 && c.Ctot > 0.0)) return false;
+    if (!totals_in_range(sum, c.Ctot, S)) return false;
     c.C[K - 1] = c.Ctot - sum;
     const int ex = exponent_above_x(S);
     c.m_q = H.eff_shift + 6 - ex;
@@ -256,7 +261,7 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
     sum = team_value<TEAM>(sum, sh + 3 * K, lane);
     c.Ctot = __dmul_rn(pressure_R, c.rcpT);
     const double S = sum > c.Ctot ? sum : c.Ctot;
-    if (!(S > 1e-200 && S < 1e200 && c.Ctot > 0.0)) return false;
+    if (!totals_in_range(sum, c.Ctot, S)) return false;
     if (lane == 0) C[K - 1] = c.Ctot - sum;
     team_sync<TEAM>();
     const int ex = exponent_above_x(S);
