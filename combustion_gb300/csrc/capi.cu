@@ -130,8 +130,10 @@ TransportLaunch transport_launch(const cb_mech* m) {
     return {cbg::launch_transport, m->d_transport, m->host.transport_blob.size()};
 }
 
-// kOverlap where the transport of a fused call may run beside its rates: its outputs touch neither the cells nor the
-// rates' outputs (ends of the whole range they span, so rows laid out in between count as touched).
+// kOverlap where the transport of a fused call may run beside its rates: no array that one of the kernels writes touches
+// one that the other reads or writes (the cells, the rates' outputs, the transport's; ends of the whole range that the
+// written arrays span, so rows laid out in between count as touched). Otherwise the transport follows the rates, and
+// reads a cell that the rates' outputs have overwritten as they left it.
 // The two kernels then fill what the other leaves idle: the SMs a small call does not reach, the last wave, the pipe
 // the other waits for. Rates and transport after / beside each other, us: 53 species 5,000 cells 387 / 328, 10,100 cells
 // 645 / 590, 160,000 cells 4,310 / 3,580; 250 species 300 cells 1,180 / 834, 60,000 cells 39,500 / 33,100 (mixed precision
@@ -143,17 +145,19 @@ uint32_t overlap_flag(int kmax, bool mixed, size_t n, const double* const* in, i
     const size_t per_sm = (n + cbg::sm_count() - 1) / cbg::sm_count();
     if (kmax == 16 && ((per_sm > 2 && per_sm <= 11) || per_sm > 16384)) return 0;
     if (kmax == 256 && per_sm > 3 && per_sm <= (mixed ? 60 : 16)) return 0;
-    uintptr_t lo = UINTPTR_MAX, hi = 0;
     const size_t bytes = n * sizeof(double);
-    for (int q = 0; q < nt; q++) {
-        lo = std::min(lo, (uintptr_t)transport[q]);
-        hi = std::max(hi, (uintptr_t)transport[q] + bytes);
-    }
-    auto apart = [&](const double* p) { return (uintptr_t)p + bytes <= lo || (uintptr_t)p >= hi; };
-    for (int q = 0; q < ni; q++)
-        if (!apart(in[q])) return 0;
-    for (int q = 0; q < nr; q++)
-        if (!apart(rates[q])) return 0;
+    // no row of a touches the range that the rows of b span
+    auto apart = [&](const double* const* a, int na, double* const* b, int nb) {
+        uintptr_t lo = UINTPTR_MAX, hi = 0;
+        for (int q = 0; q < nb; q++) {
+            lo = std::min(lo, (uintptr_t)b[q]);
+            hi = std::max(hi, (uintptr_t)b[q] + bytes);
+        }
+        for (int q = 0; q < na; q++)
+            if ((uintptr_t)a[q] + bytes > lo && (uintptr_t)a[q] < hi) return false;
+        return true;
+    };
+    if (!apart(in, ni, transport, nt) || !apart(rates, nr, transport, nt) || !apart(in, ni, rates, nr)) return 0;
     return cbg::kOverlap;
 }
 

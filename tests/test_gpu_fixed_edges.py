@@ -75,3 +75,32 @@ def test_states_of_the_fp64_form(config):
                                       equal_nan=True), what
             both = np.isfinite(a) & np.isfinite(sc)
             assert (util.cond_err(a, b, sc)[both] <= util.PLAIN_TOL).all()
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_fused_call_with_rates_over_the_cells(config, mixed):
+    """A fused call whose species rates overwrite the cells' amounts: the transport is of the overwritten cells, as in two
+    calls one after the other, at sizes where the two kernels otherwise run beside each other."""
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = util.mechanism(config)
+    mech = cb.Mechanism(m)
+    mech.transport_setup(*synthetic.transport_scales(m))
+    assert m.active() == m.K - 1
+    for n in {"k10": (1, 300, 5000, 70001), "k53": (1, 300, 10100, 70001), "k250": (1, 456, 12001)}[config]:
+        x = dev(oracle.Oracle(m).rates_inputs(synthetic.generate_cells(m.K, n, config, seed=7)))
+        got = []
+        for fused in (True, False):
+            y, d = x.clone(), torch.empty((2, n), dtype=torch.float64, device="cuda")
+            r = list(d) + list(y[4:])
+            t = torch.full((m.K + 2, n), 7.0, dtype=torch.float64, device="cuda")
+            if fused:
+                mech.rates_transport(y, r, t, mixed=mixed)
+            else:
+                mech.rates(y, r, mixed=mixed)
+                mech.rates_transport(y, torch.empty((mech.A + 2, n), dtype=torch.float64, device="cuda"), t, mixed=mixed)
+            mech.synchronize()
+            got.append(torch.cat([y, d, t]).nan_to_num(-3.0))
+        assert torch.equal(*got)
