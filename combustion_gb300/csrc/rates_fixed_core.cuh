@@ -73,6 +73,14 @@ __device__ __forceinline__ int piece_x(double split, double T) {
     return bits(T) <= bits(split) && (bits(split) >> 52) < 0x7ff ? 0 : __double2hiint(T) < (1023 + 11) << 20 ? 1 : 2;
 }
 
+// The cross products of two dot products with word positions a (Qy) and b (3 bits below) as a number in Qy. Each of four
+// terms of b is below 2^58 + 2^58 (a coefficient's high word is below 2^30, a power's at most 2^30, low words at most
+// 2^28), so their sum, below 2^61, is not shifted up; a's two terms are below 2^60.2 together. (The high words' sums may
+// wrap on their way: the total is in range.)
+__device__ __forceinline__ long long low_words(long long a2, long long b2) {
+    return (b2 + (a2 >> 3) + (1ll << (kLo - 4))) >> (kLo - 3);
+}
+
 // Gibbs energy over RT (reaction.rs:75-110) in base-2 units, Qy.
 __device__ __forceinline__ long long gibbs_log2(const SpeciesX& s, const TempsX& t) {
     const int set = piece_x(s.split, t.T);
@@ -83,7 +91,7 @@ __device__ __forceinline__ long long gibbs_log2(const SpeciesX& s, const TempsX&
 #pragma unroll
     for (int i = 0; i < 4; i++) dot_term(g[2 + i], t.p[i], b1, b2);  // Q(kGq + kPq), 3 bits below Qy
     static_assert(kGq + kPq == kYq - 3 && kBq + kLq == kYq && kEq + kRq == kYq, "word positions");
-    return a1 + (b1 << 3) + ((a2 + (b2 << 3) + (1ll << (kLo - 1))) >> kLo);
+    return a1 + (b1 << 3) + low_words(a2, b2);
 }
 
 // h / RT and cp / R of a species.
@@ -93,14 +101,14 @@ __device__ __forceinline__ double enthalpy_x(const ThermoX& s, int set, const Te
     dot_term(h[4], t.r, a1, a2);
 #pragma unroll
     for (int i = 0; i < 4; i++) dot_term(h[i], t.p[i], b1, b2);
-    return fix_to_dbl(a1 + (b1 << 3) + ((a2 + (b2 << 3) + (1ll << (kLo - 1))) >> kLo), kYq);
+    return fix_to_dbl(a1 + (b1 << 3) + low_words(a2, b2), kYq);
 }
 __device__ __forceinline__ double heat_capacity_x(const ThermoX& s, int set, const TempsX& t) {
     const Word2* c = s.cp[set];
     long long b1 = 0, b2 = 0;
 #pragma unroll
     for (int i = 0; i < 4; i++) dot_term(c[i], t.p[i], b1, b2);
-    return fix_to_dbl(s.cp0[set] + (b1 << 3) + (((b2 << 3) + (1ll << (kLo - 1))) >> kLo), kYq);
+    return fix_to_dbl(s.cp0[set] + (b1 << 3) + low_words(0, b2), kYq);
 }
 
 // The Troe forward coefficient in the general case (reaction.rs:160-193).

@@ -104,3 +104,59 @@ def test_fused_call_with_rates_over_the_cells(config, mixed):
             mech.synchronize()
             got.append(torch.cat([y, d, t]).nan_to_num(-3.0))
         assert torch.equal(*got)
+
+
+def _words(v, low):
+    """v = hi 2^low + lo, lo balanced, of Python integers."""
+    hi = (v + (1 << (low - 1))) >> low
+    return hi, v - (hi << low)
+
+
+@pytest.mark.parametrize("power", [11, 13])
+@pytest.mark.parametrize("kind", ["gibbs", "enthalpy", "heat-capacity"])
+def test_low_words_at_their_end(kind, power):
+    """Polynomials whose coefficients' low words are all close to -2^28, just below the end of a piece's temperatures (T /
+    2^11 or T / 2^13 close to 1): the sum of their cross products is then as large as any mechanism's."""
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    LD = np.longdouble
+    m = copy.deepcopy(util.mechanism("k10"))
+    T = 2.0 ** power * (1.0 - 2.0 ** -31)
+    L = 29
+    target = -(1 << 28) + 256
+    log2e = 1 / np.log(LD(2))
+    # (coefficient index, factor to the polynomial's own, bits below the binary point of its two words, power of T)
+    poly = {"gibbs": [(0, -1.0, 53, 0), (5, log2e, 43, -1), (1, -log2e / 2, 47, 1), (2, -log2e / 6, 47, 2),
+                      (3, -log2e / 12, 47, 3), (4, -log2e / 20, 47, 4)],
+            "enthalpy": [(5, 1.0, 43, -1), (1, 0.5, 47, 1), (2, LD(1) / 3, 47, 2), (3, 0.25, 47, 3), (4, LD(1) / 5, 47, 4)],
+            "heat-capacity": [(1, 1.0, 47, 1), (2, 1.0, 47, 2), (3, 1.0, 47, 3), (4, 1.0, 47, 4)]}[kind]
+    largest = 0
+    for k in range(m.K):
+        a2 = b2 = 0
+        for i, factor, bits, n in poly:
+            scale = LD(factor) * LD(2) ** (power * max(n, 0) + bits)
+            hi, _ = _words(int(np.rint(LD(m.nasa7[k, 1, i]) * scale)), L)
+            m.nasa7[k, 1, i] = float((LD(hi) * 2 ** L + target) / scale)
+            w = _words(int(np.rint(LD(m.nasa7[k, 1, i]) * scale)), L)
+            t = {0: np.log2(LD(T)) * LD(2) ** 56, -1: LD(2) ** 66 / LD(T)}.get(n, LD(2.0 ** -power * T) ** n * LD(2) ** 59)
+            t = _words(int(np.rint(t)), L)
+            term = w[0] * t[1] + w[1] * t[0]
+            if n > 0:
+                b2 += term
+            else:
+                a2 += term
+        largest = max(largest, abs(a2 + 8 * b2))
+    assert largest > 1 << 63  # (what a 64-bit sum in units of the smaller words does not hold)
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    cells = synthetic.generate_cells(m.K, 64, "k10", seed=41)
+    cells.amounts *= cells.temperature / T
+    cells.temperature[:] = T
+    rin = o.rates_inputs(cells)
+    out = torch.empty((mech.A + 2, cells.n), dtype=torch.float64, device="cuda")
+    mech.rates(dev(rin), out)
+    mech.synchronize()
+    ref, sc = o.rates(rin, scale=True)
+    e = util.cond_err(out.cpu().numpy(), ref, sc)
+    print(f"{kind}, T / 2^{power}: max cond err {e.max():.2e}")
+    assert e.max() <= util.PLAIN_TOL
