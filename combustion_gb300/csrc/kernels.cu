@@ -176,7 +176,7 @@ cudaError_t launch_transport_k(const uint8_t* tab, uint32_t tab_bytes, const Tra
             const bool smem = warp_table_bytes(true, tab_bytes) + scratch <= (size_t)max_table_smem();
             const size_t bytes = warp_table_bytes(smem, tab_bytes) + scratch;
             auto kern = smem ? transport_warp_kernel<KMAX, true> : transport_warp_kernel<KMAX, false>;
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            const cudaError_t e = allow_shared(kern);
             if (e != cudaSuccess) return e;
             int per_sm = 1;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarpCellWarps, bytes);

@@ -92,6 +92,13 @@ struct CountArgs {
 };
 cudaError_t launch_count_nonfinite(const CountArgs& args, size_t n, unsigned long long* count, cudaStream_t st);
 
+// A kernel's limit of dynamic shared memory, raised to the device's. The limit belongs to the process: with what a call
+// needs in its place, a call of another host thread could lower it between this one's setting and its launch.
+template <class K>
+cudaError_t allow_shared(K kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_table_smem());
+}
+
 // Blocks of a persistent table kernel resident per SM, the tables in shared memory (smem: the variant
 // ksmem, whose dynamic shared memory limit is raised first) or read from global memory (kglobal, only
 // the math tables in shared memory).
@@ -100,7 +107,7 @@ cudaError_t table_kernel_occupancy(KS ksmem, KG kglobal, int block, uint32_t tab
                                    bool smem, int* per_sm) {
     *per_sm = 1;
     if (smem) {
-        cudaError_t e = cudaFuncSetAttribute(ksmem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab_bytes);
+        const cudaError_t e = allow_shared(ksmem);
         if (e != cudaSuccess) return e;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, ksmem, block, tab_bytes);
     } else {

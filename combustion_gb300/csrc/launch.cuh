@@ -90,8 +90,7 @@ cudaError_t launch_warp_kernel(KS ksmem, KG kglobal, const uint8_t* tab, uint32_
     while (warps > 1 && (smem ? tab_bytes : math) + warps * warp_bytes > (size_t)max_table_smem()) warps--;
     const size_t bytes = (smem ? tab_bytes : math) + warps * warp_bytes;
     if (bytes > (size_t)max_table_smem()) return cudaErrorInvalidConfiguration;
-    cudaError_t e = smem ? cudaFuncSetAttribute(ksmem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
-                         : cudaFuncSetAttribute(kglobal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    const cudaError_t e = smem ? allow_shared(ksmem) : allow_shared(kglobal);
     if (e != cudaSuccess) return e;
     int per_sm = 1;
     if (smem) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ksmem, 32 * warps, bytes);
@@ -111,8 +110,7 @@ cudaError_t launch_team_kernel(KS ksmem, KG kglobal, const uint8_t* tab, uint32_
                                uint32_t math, size_t cell_bytes, cudaStream_t st, int* status) {
     const bool smem = tab_bytes + cell_bytes <= (size_t)max_table_smem();
     const size_t bytes = (smem ? tab_bytes : math) + cell_bytes, grid = n ? n : 1;
-    cudaError_t e = smem ? cudaFuncSetAttribute(ksmem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
-                         : cudaFuncSetAttribute(kglobal, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    const cudaError_t e = smem ? allow_shared(ksmem) : allow_shared(kglobal);
     if (e != cudaSuccess) return e;
     return smem ? launch_one(ksmem, grid, 32 * TEAM, bytes, st, tab, tab_bytes, io, n, status)
                 : launch_one(kglobal, grid, 32 * TEAM, bytes, st, tab, tab_bytes, io, n, status);

@@ -519,7 +519,7 @@ cudaError_t launch_transport_xk(const uint8_t* tab, uint32_t tab_bytes, const Tr
         const bool smem = warp_table_bytes(true, tab_bytes) + scratch <= (size_t)max_table_smem();
         const size_t bytes = warp_table_bytes(smem, tab_bytes) + scratch;
         auto kern = smem ? transport_x_team_kernel<KMAX, true> : transport_x_team_kernel<KMAX, false>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        const cudaError_t e = allow_shared(kern);
         if (e != cudaSuccess) return e;
         return launch_one(kern, n, 32 * kTeamWarps, bytes, st, tab, tab_bytes, io, n, status);
     }
@@ -530,7 +530,7 @@ cudaError_t launch_transport_xk(const uint8_t* tab, uint32_t tab_bytes, const Tr
         while (warps > 1 && warp_table_bytes(smem, tab_bytes) + warps * scratch > (size_t)max_table_smem()) warps--;
         const size_t bytes = warp_table_bytes(smem, tab_bytes) + warps * scratch;
         auto kern = smem ? transport_x_warp_kernel<KMAX, true> : transport_x_warp_kernel<KMAX, false>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        const cudaError_t e = allow_shared(kern);
         if (e != cudaSuccess) return e;
         int per_sm = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, bytes);

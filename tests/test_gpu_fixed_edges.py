@@ -160,3 +160,49 @@ def test_low_words_at_their_end(kind, power):
     e = util.cond_err(out.cpu().numpy(), ref, sc)
     print(f"{kind}, T / 2^{power}: max cond err {e.max():.2e}")
     assert e.max() <= util.PLAIN_TOL
+
+
+def test_calls_of_two_threads():
+    """Two host threads, each with a handle and a stream of its own, whose calls take different amounts of shared memory
+    from the same kernels (16 and 2 cells per block of one per warp; 8 warps per cell): every launch is accepted and
+    every call gives what it gives alone."""
+    import threading
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = util.mechanism("k10")
+    x = dev(oracle.Oracle(m).rates_inputs(synthetic.generate_cells(m.K, 4000, "k10", seed=3)))
+    errors = []
+
+    def new(mech, n):
+        return (torch.empty((mech.A + 2, n), dtype=torch.float64, device="cuda"),
+                torch.empty((mech.K + 2, n), dtype=torch.float64, device="cuda"))
+
+    def work(sizes, gate):
+        try:
+            mech, stream = cb.Mechanism(m), torch.cuda.Stream()
+            mech.transport_setup(*synthetic.transport_scales(m))
+            cells, outs = [x[:, :n].contiguous() for n in sizes], [new(mech, n) for n in sizes]
+            alone = [new(mech, n) for n in sizes]
+            for c, o in zip(cells, alone):
+                mech.rates_transport(c, *o)
+            torch.cuda.synchronize()
+            gate.wait()
+            for _ in range(1500):
+                for c, (r, t) in zip(cells, outs):
+                    mech.rates_transport(c, r, t, stream=stream)
+                    mech.rates(c, r, stream=stream, mixed=True)
+                    mech.rates(c, r, stream=stream)
+            mech.synchronize(stream.cuda_stream)
+            assert all(torch.equal(a, b) for p, q in zip(outs, alone) for a, b in zip(p, q))
+        except Exception as e:  # noqa: BLE001
+            errors.append(repr(e))
+            gate.abort()
+
+    gate = threading.Barrier(2)
+    threads = [threading.Thread(target=work, args=(sizes, gate)) for sizes in ((2400, 1), (200, 400))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
