@@ -107,7 +107,10 @@ cudaError_t table_kernel_occupancy(KS ksmem, KG kglobal, int block, uint32_t tab
                                    bool smem, int* per_sm) {
     *per_sm = 1;
     if (smem) {
-        const cudaError_t e = allow_shared(ksmem);
+        cudaError_t e = allow_shared(ksmem);
+        // the split of shared memory and L1 that an earlier call asked for (set_carveout) is not this call's
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(ksmem, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutDefault);
         if (e != cudaSuccess) return e;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, ksmem, block, tab_bytes);
     } else {
@@ -118,7 +121,8 @@ cudaError_t table_kernel_occupancy(KS ksmem, KG kglobal, int block, uint32_t tab
 }
 
 // Shared memory (of an SM's 256 KB, shared with L1) for `per_sm` resident blocks of a table kernel, whatever
-// block size a launch takes.
+// block size a launch takes. The preference stays with the kernel: table_kernel_occupancy takes it back for the next
+// call (left from a call of a smaller mechanism, 2^20 cells of mixed rates at 53 species took 11.5 ms, 9.4 without).
 template <class K>
 cudaError_t set_carveout(K kernel, int per_sm, uint32_t bytes) {
     const int most = max_table_smem() + 1024, want = per_sm * (int)(bytes + 2048);

@@ -206,3 +206,38 @@ def test_calls_of_two_threads():
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_large_call_after_small_ones():
+    """A large call is as fast after a small call of another mechanism of the same capacity as before it (the split of
+    shared memory and L1 that a small call prefers ends with it)."""
+    import torch
+    import combustion_gb300 as cb
+    from combustion_gb300 import surrogate as S
+    m = util.mechanism("k53")
+    small = copy.deepcopy(m)  # the same species with a sixth of the reactions: smaller tables
+    keep = np.arange(0, m.R) < m.K - 1  # (the generator's first K - 1 reactions change every species but the last)
+    for name in ("reactants", "products", "model", "rate", "k0", "troe", "sri", "efficiencies"):
+        setattr(small, name, getattr(m, name)[keep])
+    mech, other = cb.Mechanism(m), cb.Mechanism(small)
+    n = 1 << 20
+    x = S.generate_cells(mech, n, S.distribution("k53", seed=5))
+    out = torch.empty((mech.A + 2, n), dtype=torch.float64, device="cuda")
+
+    def timed(mixed):
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            mech.rates(x, out, mixed=mixed)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return float(np.median(times))
+
+    for mixed in (True, False):
+        before = timed(mixed)
+        other.rates(x[:, :50000], out[:, :50000], mixed=mixed)
+        after = timed(mixed)
+        print(f"mixed {mixed}: {before:.2f} ms, after a small call {after:.2f} ms")
+        assert after < 1.1 * before
