@@ -147,7 +147,8 @@ bool build_rates_fixed(HostMechanism& m) {
     std::vector<Reaction> rx(R);
     std::vector<ReactionX> fx(R);
     const int third = H.group_end[1];  // models 2-5 follow
-    std::vector<FalloffX> ff(R > third ? R - third : 0);
+    std::vector<FalloffX> ff(R > third ? (R - third + 3) / 4 * 4 : 0);
+    if (!ff.empty()) std::memset(ff.data(), 0, ff.size() * sizeof(FalloffX));
     for (int r = 0; r < R; r++) {
         at(H.off_reactions, r, sizeof(Reaction), &rx[r]);
         const Reaction& x = rx[r];
@@ -202,7 +203,6 @@ bool build_rates_fixed(HostMechanism& m) {
         }
         if (r >= third) {
             FalloffX& g = ff[r - third];
-            std::memset(&g, 0, sizeof g);
             if (x.falloff >= 0) {
                 if (!arrhenius_fix(fo.k0, g.k0, bound)) return false;
                 g.ainf = fo.ainf;
@@ -225,17 +225,29 @@ bool build_rates_fixed(HostMechanism& m) {
         }
     }
 
-    // third-body efficiencies minus one, rows padded to a multiple of 4 like the FP64 table's
+    // third-body efficiencies minus one, rows padded to a multiple of 4 like the FP64 table's, a unit of its own each
     const size_t n_e = (size_t)(H.n_eff + 3) / 4 * 4 * K;
     std::vector<double> eff(n_e);
     if (n_e) std::memcpy(eff.data(), blob + H.off_eff, n_e * sizeof(double));
-    double largest = 0.;
-    for (double e : eff) largest = std::max(largest, std::fabs(e));
-    if (!(largest < 256.)) return false;
-    X.eff_shift = kEffBits;
-    while (std::ldexp(largest, X.eff_shift) >= std::ldexp(1.0, kEffBits)) X.eff_shift--;
     std::vector<Word2> ef(n_e);
-    for (size_t i = 0; i < n_e; i++) ef[i] = words((int64_t)std::llround(std::ldexp((long double)eff[i], X.eff_shift)));
+    for (size_t row = 0; row < n_e / K; row++) {
+        const double* e = &eff[row * K];
+        long double largest = 0.0L, sum = 0.0L;
+        for (int k = 0; k < K; k++) {
+            largest = std::max(largest, std::fabs((long double)e[k]));
+            sum += std::fabs((long double)e[k]);
+        }
+        if (!(largest < 256.0L)) return false;
+        int q = 29;
+        while (std::ldexp(largest, q) > 2147483646.0L || std::ldexp(sum, q) + K > std::ldexp(1.0L, 33)) q--;
+        for (int k = 0; k < K; k++)
+            ef[row * K + k] = words((int64_t)std::llround(std::ldexp((long double)e[k], q + kThirdLo)), kThirdLo);
+        // the sum, at most 1 + 2 largest, below 2^60 in its unit (2^62 where the high words leave no bits below)
+        int top = 0;
+        while (std::ldexp(1.0L, top) < 1.0L + 2.0L * largest) top++;
+        ff[row].m_up = std::min(std::max(59 - top - q - 30, 0), kThirdLo - 1);
+        ff[row].m_q = q + 30 + ff[row].m_up;
+    }
 
     std::vector<uint8_t>& b = m.rates_fixed_blob;
     b.insert(b.end(), blob, blob + kMathBytes);  // the FP64 functions' tables, then the fixed-point ones

@@ -22,10 +22,10 @@ template <int KMAX>
 struct CellX {
     TempsX t;
     double rcpT, Ctot;
-    long long ctot;    // Ctot in the third-body sums' unit
-    int m_q;           // and the position of its point
+    long long ctot;    // Ctot over S, Q60
+    int ex;            // S = 2^ex
     double C[KMAX];    // concentrations, bulk last
-    Word2 cw[KMAX];    // the same over S
+    Word2 cw[KMAX];    // the same over S, Q60
     long long g[KMAX];  // Gibbs energies over RT, base 2, Qy
 };
 
@@ -58,11 +58,10 @@ __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pres
     const double S = sum > c.Ctot ? sum : c.Ctot;
     if (!totals_in_range(sum, c.Ctot, S)) return false;
     c.C[K - 1] = c.Ctot - sum;
-    const int ex = exponent_above_x(S);
-    c.m_q = H.eff_shift + 6 - ex;
-    c.ctot = dbl_to_fix(c.Ctot, c.m_q);
+    c.ex = exponent_above_x(S);
+    c.ctot = dbl_to_fix(c.Ctot, 60 - c.ex);
     if (H.n_eff)
-        for (int k = 0; k < K; k++) c.cw[k] = split_word(dbl_to_fix(c.C[k], kCq + kLo - ex));
+        for (int k = 0; k < K; k++) c.cw[k] = split_word<kThirdLo>(dbl_to_fix(c.C[k], 60 - c.ex));
     c.t = make_temps(H, T, c.rcpT);
     for (int k = 0; k < A; k++) {
         const SpeciesX& s = tb.species[k];
@@ -82,8 +81,10 @@ __device__ __forceinline__ void plain_group_x(const RatesXTables& tb, const Cell
 
 // Third-body concentration of a row from its two partial sums (reaction.rs:141-145): Ctot + sum (e - 1) C.
 template <class CellT>
-__device__ __forceinline__ double third_body(const CellT& c, long long s1, long long s2) {
-    return fix_to_dbl(c.ctot + (s1 << 6) + ((s2 + (1ll << (kLo - 7))) >> (kLo - 6)), c.m_q);
+__device__ __forceinline__ double third_body(const CellT& c, const FalloffX& row, long long s1, long long s2) {
+    const int up = row.m_up, down = kThirdLo - up, q = row.m_q;  // down >= 1, q <= 59
+    const long long ctot = (c.ctot + (1ll << (59 - q))) >> (60 - q);
+    return fix_to_dbl(ctot + (s1 << up) + ((s2 + (1ll << (down - 1))) >> down), q - c.ex);
 }
 
 // Models 2-5: the third-body sums of four consecutive rows in one pass over the concentrations (three
@@ -100,8 +101,9 @@ __device__ __forceinline__ void third_body_groups_x(const RatesXTables& tb, cons
 #pragma unroll
             for (int q = 0; q < 4; q++) dot_term(E[q * K + k], ck, s1[q], s2[q]);
         }
-        const double M0 = third_body(c, s1[0], s2[0]), M1 = third_body(c, s1[1], s2[1]);
-        const double M2 = third_body(c, s1[2], s2[2]), M3 = third_body(c, s1[3], s2[3]);
+        const FalloffX* row = tb.falloff + (r0 - r_begin);
+        const double M0 = third_body(c, row[0], s1[0], s2[0]), M1 = third_body(c, row[1], s1[1], s2[1]);
+        const double M2 = third_body(c, row[2], s1[2], s2[2]), M3 = third_body(c, row[3], s1[3], s2[3]);
         const int rq = min(r_end - r0, 4);
 #pragma unroll 1
         for (int q = 0; q < rq; q++) {
@@ -228,7 +230,7 @@ struct CellXW {
     TempsX t;
     double rcpT, Ctot;
     long long ctot;
-    int m_q;
+    int ex;
     const double* C;
     const long long* g;
 };
@@ -264,14 +266,13 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
     if (!totals_in_range(sum, c.Ctot, S)) return false;
     if (lane == 0) C[K - 1] = c.Ctot - sum;
     team_sync<TEAM>();
-    const int ex = exponent_above_x(S);
-    c.m_q = H.eff_shift + 6 - ex;
-    c.ctot = dbl_to_fix(c.Ctot, c.m_q);
+    c.ex = exponent_above_x(S);
+    c.ctot = dbl_to_fix(c.Ctot, 60 - c.ex);
     c.t = make_temps(H, T, c.rcpT);
     c.C = C;
     c.g = g;
     for (int k = lane; k < K; k += kStep) {
-        const Word2 w = split_word(dbl_to_fix(C[k], kCq + kLo - ex));
+        const Word2 w = split_word<kThirdLo>(dbl_to_fix(C[k], 60 - c.ex));
         cw[k] = __hiloint2double(w.hi, w.lo);
         if (k < A && (tb.species[k].need_exp | tb.species[k].need_exp_neg)) g[k] = gibbs_log2(tb.species[k], c.t);
     }
@@ -281,7 +282,7 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
         long long s1 = 0, s2 = 0;
 #pragma unroll 4
         for (int k = 0; k < K; k++) dot_term(E[k], Word2{__double2hiint(cw[k]), __double2loint(cw[k])}, s1, s2);
-        M[e] = third_body(c, s1, s2);
+        M[e] = third_body(c, tb.falloff[e], s1, s2);
     }
     team_sync<TEAM>();
     const int first = H.group_end[1];

@@ -32,8 +32,12 @@ constexpr int kRq = 37;    // 1 / T, hi word (1/T <= 1/200)
 constexpr int kEq = 14;    // its factor, |.| < 2^17
 constexpr int kPq = 30;    // (T / 2^p)^i, hi word, p = 11 below 2048 K and 13 above
 constexpr int kGq = 18;    // its factor, |.| < 4096
-constexpr int kCq = 29;    // C_k / S, hi word (S a power of two above every sum of concentrations)
-constexpr int kEffBits = 55;  // |efficiency - 1| 2^eff_shift < 2^kEffBits
+// Third-body sums: C_k / S (S a power of two above both totals) in 60 bits, efficiencies - 1 of a row in units of
+// 2^-(q + kThirdLo), q the largest (at most 29) that keeps the row's high words below 2^31 and their sum below 2^33: then
+// the cross products' sum stays below 2^63. The dropped products of low words are below 2^-(q + 32) S each; the sum's
+// error is below that of FP64 FMAs (an efficiency of 256 beside 52 of 0.5 to 3: largest 4.4e-16 of M, FP64 9.5e-16; with
+// one unit for the whole mechanism and 29-bit low words it was 2.1e-14).
+constexpr int kThirdLo = 30;
 
 struct Word2 {
     int32_t hi, lo;
@@ -66,14 +70,15 @@ struct ReactionX {  // 64 bytes
 };
 static_assert(sizeof(ReactionX) == 64, "four 16-byte loads");
 
-// One per reaction of models 2-5, in reaction order (three-body entries unused). Exponents and
-// logarithms in base 2.
+// One per reaction of models 2-5, in reaction order, padded to a multiple of 4 (of a three-body reaction the
+// efficiencies' unit only). Exponents and logarithms in base 2.
 struct FalloffX {
     ArrheniusX k0;
     double ainf, c1mA, cA, c3, c1, cmT2, l2_fcent;
     int64_t lainf;          // log2(ainf), Qy
     int32_t flags, sri_flags;
     double sA, smB, smrC, sD, sE;
+    int32_t m_up, m_q;      // the third-body sum's unit is 2^-m_q S, 2^m_up below that of its high words' products
 };
 
 // Gibbs energy over RT in base-2 units: piece 0 for T <= split, else 1 below kFixTmid and 2 above (the
@@ -98,8 +103,6 @@ struct RatesXHeader {
     int32_t off_csr_start, off_csr;  // per species the reactions that change it, in order: [K + 1]; r << 8 | nu
     int32_t group_end[6];
     int64_t lM3, lcbrt, lC0;  // log2 of the Gibbs exponentials' caps and of P0 / R, Qy
-    int32_t eff_shift;        // efficiency words are (e - 1) 2^eff_shift, eff_shift <= kEffBits
-    int32_t pad;
     double l10_04, l10_075;   // 0.4 and 0.75 log2(10)
 };
 

@@ -241,3 +241,56 @@ def test_large_call_after_small_ones():
         after = timed(mixed)
         print(f"mixed {mixed}: {before:.2f} ms, after a small call {after:.2f} ms")
         assert after < 1.1 * before
+
+
+def concentrations(m, cells):
+    """Ctot, S = 2^ex above it and every sum, and C of unit volumes, as every form computes them."""
+    Ctot = cells.pressure_R * (1.0 / cells.temperature)
+    total = np.zeros(cells.n)
+    for k in range(m.K - 1):
+        total = total + cells.amounts[k]
+    return Ctot, np.frexp(np.maximum(total, Ctot))[1], np.vstack([cells.amounts, Ctot - total])
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+@pytest.mark.parametrize("largest", [12.0, 17.0, 61.0, 256.5])
+def test_third_body_sums(config, largest):
+    """Third-body concentrations against long double, one species far more efficient than the others: the error is that
+    of the words (sums in fixed point) and two roundings, below that of a chain of FP64 FMAs."""
+    import torch
+    import combustion_gb300 as cb
+    LD = np.longdouble
+    m = copy.deepcopy(util.mechanism(config))
+    K, (s, p) = m.K, (0, 1)
+    rows = np.flatnonzero(m.model == synthetic.THREE_BODY)
+    rng = np.random.default_rng(5)
+    for i, r in enumerate(rows):  # 1 M C_s, and nothing back where species p is absent
+        m.reactants[r], m.products[r], m.rate[r] = 0, 0, (1.0, 0.0, 0.0)
+        m.reactants[r, s] = m.products[r, p] = 1
+        m.efficiencies[r] = rng.uniform(0.5, 3.0, K)
+        m.efficiencies[r, 2 + i % (K - 2)] = largest
+    assert m.active() == K - 1
+    mech = cb.Mechanism(m)
+    cells = synthetic.generate_cells(K, 512, config, seed=43)
+    cells.amounts[p] = 0.0
+    Ctot, ex, C = concentrations(m, cells)
+    x = np.vstack([cells.pressure_R, cells.temperature, cells.volume, cells.amounts])
+    out = torch.empty((m.R, cells.n), dtype=torch.float64, device="cuda")
+    mech.reaction_rates(dev(x), out)
+    mech.synchronize()
+    out = out.cpu().numpy()
+    worst = ratio = 0.0
+    for r in rows:
+        e = m.efficiencies[r].astype(LD) - 1
+        M = Ctot + (e[:, None] * C).sum(0)
+        size = np.abs(m.efficiencies[r] - 1.0)
+        q = 29
+        while size.max() * 2.0 ** q > 2.0 ** 31 - 2 or size.sum() * 2.0 ** q + K > 2.0 ** 33:
+            q -= 1
+        # words of C (2^-61 S) and of e - 1 (2^-(q + 31), times at most 2 S), dropped products, the sum's unit
+        words = size.sum() * 2.0 ** -61 + 2.0 ** -(q + 30) + K * 2.0 ** -(q + 32) + 2.0 ** -(q + 30)
+        bound = words * np.ldexp(1.0, ex) / np.abs(M) + 2.0 ** -52
+        err = np.abs((out[r] - M * C[s]) / (M * C[s])).astype(np.float64)
+        worst, ratio = max(worst, err.max()), max(ratio, (err / bound).max())
+    print(f"{config}, largest efficiency {largest}: max error {worst:.2e}, {ratio:.2f} of the bound")
+    assert ratio <= 1.0
