@@ -32,12 +32,18 @@ bool to_words(long double x, int q_hi, long double limit, Word2& w, int lo = kLo
 }
 
 // k = exp(x) or the constant A (times a power of T), as log2 k; `bound` receives the largest |log2 k| over
-// the fixed-point temperature range.
-bool arrhenius_fix(const Arrhenius& a, ArrheniusX& f, long double& bound) {
+// the fixed-point temperature range. The constant itself unless `logarithm` (a Troe reaction adds logarithms).
+bool arrhenius_fix(const Arrhenius& a, ArrheniusX& f, long double& bound, bool logarithm) {
     static const int power[] = {0, -2, -1, 4, 3, 2, 1};  // Factor
     const long double beta = a.has_x ? (long double)a.beta : (long double)power[a.factor];
     const long double e = a.has_x ? (long double)a.mEa * kLog2e : 0.0L;
     if (!a.has_x && !(a.A > 0. && std::isfinite(a.A))) return false;
+    if (!a.has_x && !logarithm) {
+        f.b = {a.factor, 0};
+        f.e = {kExactRate, 0};
+        std::memcpy(&f.a, &a.A, sizeof f.a);
+        return true;
+    }
     const long double l = a.has_x ? (long double)a.lnA * kLog2e : std::log2((long double)a.A);
     bound = std::fabs(l) + std::fabs(beta) * 13.0L + std::fabs(e) / (long double)kFixTmin;
     return to_words(beta, kBq, 64.0L, f.b) && to_words(e, kEq, 131000.0L, f.e) && to_fix(l, kYq, 4000.0L, f.a) &&
@@ -195,7 +201,7 @@ bool build_rates_fixed(HostMechanism& m) {
         Falloff fo;
         if (x.falloff >= 0) at(H.off_falloff, x.falloff, sizeof fo, &fo);
         const bool const_k = x.model == 4 && (fo.flags & kKinfConst);
-        if (!const_k && !arrhenius_fix(x.k, f.k, bound)) return false;
+        if (!const_k && !arrhenius_fix(x.k, f.k, bound, x.model == 4)) return false;
         if (x.model != 1) {  // the equilibrium constant's logarithm stays in range
             long double b = 2.0L * (30.0L + 13.0L);
             for (int i = 0; i < x.n_net; i++) b += std::abs((int)x.net_n[i]) * g_bound[x.net_k[i]];
@@ -204,7 +210,7 @@ bool build_rates_fixed(HostMechanism& m) {
         if (r >= third) {
             FalloffX& g = ff[r - third];
             if (x.falloff >= 0) {
-                if (!arrhenius_fix(fo.k0, g.k0, bound)) return false;
+                if (!arrhenius_fix(fo.k0, g.k0, bound, x.model == 4)) return false;
                 g.ainf = fo.ainf;
                 if (x.model == 4 && (!(fo.ainf > 0.) || !to_fix(std::log2((long double)fo.ainf), kYq, 1000.0L, g.lainf)))
                     return false;
@@ -215,6 +221,12 @@ bool build_rates_fixed(HostMechanism& m) {
                 g.cmT2 = (double)((long double)fo.cmT2 * kLog2e);
                 g.l2_fcent = (double)((long double)fo.ln_fcent * kLog2e);
                 g.flags = fo.flags;
+                if (x.model == 4 && !fo.k0.has_x && (const_k || !x.k.has_x)) {
+                    g.flags |= kTroeExact;
+                    g.a0 = fo.k0.A;
+                    g.power0 = fo.k0.factor;
+                    g.power_inf = const_k ? (int)kNone : x.k.factor;
+                }
                 g.sri_flags = fo.sri_flags;
                 g.sA = fo.sA;
                 g.smB = (double)((long double)fo.smB * kLog2e);

@@ -21,7 +21,7 @@ namespace cbg {
 template <int KMAX>
 struct CellX {
     TempsX t;
-    double rcpT, Ctot;
+    double Ctot;
     long long ctot;    // Ctot over S, Q60
     int ex;            // S = 2^ex
     double C[KMAX];    // concentrations, bulk last
@@ -47,14 +47,13 @@ __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pres
     if (!(T >= kFixTmin && T < kFixTmax)) return false;
     // both reciprocals and the products rounded as the reference's: the bulk concentration is a difference of
     // totals, whose last bits it magnifies
-    const double md = __drcp_rn(V);
-    c.rcpT = __drcp_rn(T);
+    const double md = __drcp_rn(V), rcpT = __drcp_rn(T);
     double sum = 0.0;
     for (int k = 0; k < K - 1; k++) {
         c.C[k] = __dmul_rn(md, max0(amounts[k][i]));
         sum += c.C[k];
     }
-    c.Ctot = __dmul_rn(pressure_R, c.rcpT);
+    c.Ctot = __dmul_rn(pressure_R, rcpT);
     const double S = sum > c.Ctot ? sum : c.Ctot;
     if (!totals_in_range(sum, c.Ctot, S)) return false;
     c.C[K - 1] = c.Ctot - sum;
@@ -62,7 +61,7 @@ __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pres
     c.ctot = dbl_to_fix(c.Ctot, 60 - c.ex);
     if (H.n_eff)
         for (int k = 0; k < K; k++) c.cw[k] = split_word<kThirdLo>(dbl_to_fix(c.C[k], 60 - c.ex));
-    c.t = make_temps(H, T, c.rcpT);
+    c.t = make_temps(H, T, rcpT);
     for (int k = 0; k < A; k++) {
         const SpeciesX& s = tb.species[k];
         if (!(s.need_exp | s.need_exp_neg)) continue;
@@ -111,10 +110,10 @@ __device__ __forceinline__ void third_body_groups_x(const RatesXTables& tb, cons
             const double M = q == 0 ? M0 : q == 1 ? M1 : q == 2 ? M2 : M3;
             const FalloffX* f = tb.falloff + (r - r_begin);
             auto forward = [&](const ArrheniusX& k) {
-                if (r < H.group_end[2]) return forward_x<2>(H, k, f, c.t, c.rcpT, M);
-                if (r < H.group_end[3]) return forward_x<3>(H, k, f, c.t, c.rcpT, M);
-                if (r < H.group_end[4]) return forward_x<4>(H, k, f, c.t, c.rcpT, M);
-                return forward_x<5>(H, k, f, c.t, c.rcpT, M);
+                if (r < H.group_end[2]) return forward_x<2>(H, k, f, c.t, M);
+                if (r < H.group_end[3]) return forward_x<3>(H, k, f, c.t, M);
+                if (r < H.group_end[4]) return forward_x<4>(H, k, f, c.t, M);
+                return forward_x<5>(H, k, f, c.t, M);
             };
             reaction_x<true, SUM>(tb, r, c, w, forward, emit);
         }
@@ -228,7 +227,7 @@ constexpr int kRatesWarps = 16;  // cells per block at most
 template <int KMAX>
 struct CellXW {
     TempsX t;
-    double rcpT, Ctot;
+    double Ctot;
     long long ctot;
     int ex;
     const double* C;
@@ -251,8 +250,7 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
     long long* g = reinterpret_cast<long long*>(sh + 2 * K);
     double* M = sh + 4 * K;
     double* cR = M + H.n_eff;
-    const double md = __drcp_rn(V);
-    c.rcpT = __drcp_rn(T);
+    const double md = __drcp_rn(V), rcpT = __drcp_rn(T);
     for (int k = lane; k < K - 1; k += kStep) C[k] = __dmul_rn(md, max0(amounts[k][i]));
     team_sync<TEAM>();
     double sum = 0.0;
@@ -261,14 +259,14 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
         for (int k = 0; k < K - 1; k++) sum += C[k];
     }
     sum = team_value<TEAM>(sum, sh + 3 * K, lane);
-    c.Ctot = __dmul_rn(pressure_R, c.rcpT);
+    c.Ctot = __dmul_rn(pressure_R, rcpT);
     const double S = sum > c.Ctot ? sum : c.Ctot;
     if (!totals_in_range(sum, c.Ctot, S)) return false;
     if (lane == 0) C[K - 1] = c.Ctot - sum;
     team_sync<TEAM>();
     c.ex = exponent_above_x(S);
     c.ctot = dbl_to_fix(c.Ctot, 60 - c.ex);
-    c.t = make_temps(H, T, c.rcpT);
+    c.t = make_temps(H, T, rcpT);
     c.C = C;
     c.g = g;
     for (int k = lane; k < K; k += kStep) {
@@ -301,10 +299,10 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
                 auto forward = [&](const ArrheniusX& k) {
                     if (m == 0) return rate_constant(k, c.t);
                     const FalloffX* f = tb.falloff + (r - first);
-                    if (m == 2) return forward_x<2>(H, k, f, c.t, c.rcpT, M[r - first]);
-                    if (m == 3) return forward_x<3>(H, k, f, c.t, c.rcpT, M[r - first]);
-                    if (m == 4) return forward_x<4>(H, k, f, c.t, c.rcpT, M[r - first]);
-                    return forward_x<5>(H, k, f, c.t, c.rcpT, M[r - first]);
+                    if (m == 2) return forward_x<2>(H, k, f, c.t, M[r - first]);
+                    if (m == 3) return forward_x<3>(H, k, f, c.t, M[r - first]);
+                    if (m == 4) return forward_x<4>(H, k, f, c.t, M[r - first]);
+                    return forward_x<5>(H, k, f, c.t, M[r - first]);
                 };
                 reaction_x<true, false>(tb, r, c, nullptr, forward, store);
             }

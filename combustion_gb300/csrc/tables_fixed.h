@@ -43,11 +43,14 @@ struct Word2 {
     int32_t hi, lo;
 };
 
-// log2 of k = exp(beta ln T + mEa / T + ln A).
+// log2 of k = exp(beta ln T + mEa / T + ln A). A constant and a constant times a whole power of T keep their FP64 form
+// (exact, or two roundings, where a logarithm's last bit is 1.5e-16 of k): e.hi = kExactRate, b.hi the power (Factor) and
+// `a` the bits of A.
 struct ArrheniusX {
     Word2 b, e;  // factors of log2 T and 1 / T
     int64_t a;   // Qy
 };
+constexpr int32_t kExactRate = INT32_MIN;  // beyond any factor of 1 / T
 
 // Shape flags of a reaction (ReactionX::shape).
 enum Shape : uint32_t {
@@ -72,12 +75,15 @@ static_assert(sizeof(ReactionX) == 64, "four 16-byte loads");
 
 // One per reaction of models 2-5, in reaction order, padded to a multiple of 4 (of a three-body reaction the
 // efficiencies' unit only). Exponents and logarithms in base 2.
+constexpr int32_t kTroeExact = 1 << 16;  // beside the FP64 tables' flags
 struct FalloffX {
     ArrheniusX k0;
     double ainf, c1mA, cA, c3, c1, cmT2, l2_fcent;
     int64_t lainf;          // log2(ainf), Qy
     int32_t flags, sri_flags;
     double sA, smB, smrC, sD, sE;
+    double a0;                  // kTroeExact: both coefficients of a Troe reaction are constants times whole powers of T,
+    int32_t power0, power_inf;  // k0 = a0 T^.. and T^.. (1 with kKinfConst)
     int32_t m_up, m_q;      // the third-body sum's unit is 2^-m_q S, 2^m_up below that of its high words' products
 };
 

@@ -294,3 +294,55 @@ def test_third_body_sums(config, largest):
         worst, ratio = max(worst, err.max()), max(ratio, (err / bound).max())
     print(f"{config}, largest efficiency {largest}: max error {worst:.2e}, {ratio:.2f} of the bound")
     assert ratio <= 1.0
+
+
+@pytest.mark.parametrize("config", ["k10", "k53"])
+def test_exact_rate_constants(config):
+    """Constants and constants times a whole power of T have the bits of their FP64 products, in calls of every size; a
+    Troe reaction of such coefficients is as close to long double as its dozen FP64 roundings."""
+    import torch
+    import combustion_gb300 as cb
+    LD = np.longdouble
+    m = copy.deepcopy(util.mechanism(config))
+    rows = np.flatnonzero(m.model == synthetic.ELEMENTARY)[:8]
+    powers = [0.0, -2.0, -1.0, 1.0, 2.0, 3.0, 4.0, 0.0]
+    for r, b in zip(rows, powers):
+        m.model[r] = synthetic.IRREVERSIBLE
+        m.rate[r] = (m.rate[r, 0], b, 0.0)
+        s = int(np.flatnonzero(m.reactants[r])[0])
+        m.reactants[r] = 0
+        m.reactants[r, s] = 1
+    m.rate[rows[-1], 0] = 1e300  # capped at the largest 32-bit number
+    troe = np.flatnonzero(m.model == synthetic.TROE)[:2]
+    for r, b in zip(troe, (0.0, 2.0)):
+        m.rate[r], m.k0[r] = (1e3, b, 0.0), (1e4, 1.0, 0.0)
+        m.reactants[r], m.products[r] = 0, 0  # one reactant, and a product that is absent
+        m.reactants[r, 2] = m.products[r, 3] = 1
+    assert m.active() == m.K - 1
+    mech = cb.Mechanism(m)
+    cells = synthetic.generate_cells(m.K, 64, config, seed=47)
+    cells.amounts[3] = 0.0
+    Ctot, _, C = concentrations(m, cells)
+    T = cells.temperature
+    x = np.vstack([cells.pressure_R, T, cells.volume, cells.amounts])
+    factor = {0.0: 1.0, -2.0: (1 / T) * (1 / T), -1.0: 1 / T, 1.0: T, 2.0: T * T, 3.0: T * (T * T), 4.0: (T * T) * (T * T)}
+    for reps in (1, 20, 152 * 400 // 64 + 1):
+        out = torch.empty((m.R, 64 * reps), dtype=torch.float64, device="cuda")
+        mech.reaction_rates(dev(np.tile(x, (1, reps))), out)
+        mech.synchronize()
+        out = out[:, -64:].cpu().numpy()
+        for r, b in zip(rows, powers):
+            k = np.minimum(factor[b] * m.rate[r, 0], float(np.finfo(np.float32).max))
+            assert np.array_equal(out[r], k * C[int(np.flatnonzero(m.reactants[r])[0])]), (b, reps)
+        for r, b in zip(troe, (0, 2)):
+            M = Ctot + ((m.efficiencies[r].astype(LD) - 1)[:, None] * C).sum(0)
+            ki = LD(1) if b == 0 else T.astype(LD) ** 2
+            Pr = M * LD(m.k0[r, 0] / m.rate[r, 0]) * T / ki
+            a, T3, T1 = (LD(v) for v in m.troe[r, :3])
+            lF = np.log((1 - a) * np.exp(-T / T3) + a * np.exp(-T / T1))
+            y = np.log(Pr) - LD(67) / 100 * lF - LD(4) / 10 * np.log(LD(10))
+            f1 = y / (-LD(14) / 100 * y - LD(127) / 100 * lF + LD(75) / 100 * np.log(LD(10)))
+            ref = np.exp(lF / (f1 * f1 + 1)) * m.rate[r, 0] * ki * Pr / (Pr + 1) * C[2]
+            err = np.abs((out[r] - ref) / ref).astype(np.float64).max()
+            print(f"{config} Troe, T^{b}: max error {err:.2e}")
+            assert err <= 4e-15
