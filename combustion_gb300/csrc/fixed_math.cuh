@@ -100,8 +100,9 @@ __device__ __forceinline__ double exp2_fix(long long y) {
     if ((unsigned)((int)(y >> 32) + (1021 << 19)) >= (2044u << 19)) return exp2_slow_fix(y);
     return exp2_core(y);
 }
-// min(f32::MAX, 2^y) (reaction.rs:138); from 128 - 2^-18 on out of line.
+// min(f32::MAX, 2^y) (reaction.rs:138), or of the constant that y stands for (kConstRate); from 128 - 2^-18 on out of line.
 static __device__ __noinline__ double rate_slow(long long y) {
+    if (y >= kConstRateMin) return min_pos(kF32Max, __longlong_as_double(y - kConstRate));
     if (y >= (128ll << kYq)) return kF32Max;
     return min_pos(kF32Max, exp2((double)y * 0x1p-51));
 }

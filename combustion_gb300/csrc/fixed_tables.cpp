@@ -31,23 +31,23 @@ bool to_words(long double x, int q_hi, long double limit, Word2& w, int lo = kLo
     return true;
 }
 
-// k = exp(x) or the constant A (times a power of T), as log2 k; `bound` receives the largest |log2 k| over
-// the fixed-point temperature range. The constant itself unless `logarithm` (a Troe reaction adds logarithms).
-bool arrhenius_fix(const Arrhenius& a, ArrheniusX& f, long double& bound, bool logarithm) {
+// k = exp(x) or A times a power of T, as log2 k; `bound` receives the largest |log2 k| over the fixed-point temperature
+// range. `constant`: a constant as itself (kConstRate).
+bool arrhenius_fix(const Arrhenius& a, ArrheniusX& f, long double& bound, bool constant) {
     static const int power[] = {0, -2, -1, 4, 3, 2, 1};  // Factor
     const long double beta = a.has_x ? (long double)a.beta : (long double)power[a.factor];
     const long double e = a.has_x ? (long double)a.mEa * kLog2e : 0.0L;
-    if (!a.has_x && !(a.A > 0. && std::isfinite(a.A))) return false;
-    if (!a.has_x && !logarithm) {
-        f.b = {a.factor, 0};
-        f.e = {kExactRate, 0};
+    if (!a.has_x && !(a.A >= std::ldexp(1.0, -500) && a.A < std::ldexp(1.0, 500))) return false;
+    if (!a.has_x && a.factor == kNone && constant) {
+        f.b = f.e = {0, 0};
         std::memcpy(&f.a, &a.A, sizeof f.a);
+        f.a += kConstRate;
         return true;
     }
     const long double l = a.has_x ? (long double)a.lnA * kLog2e : std::log2((long double)a.A);
     bound = std::fabs(l) + std::fabs(beta) * 13.0L + std::fabs(e) / (long double)kFixTmin;
     return to_words(beta, kBq, 64.0L, f.b) && to_words(e, kEq, 131000.0L, f.e) && to_fix(l, kYq, 4000.0L, f.a) &&
-           bound < 4000.0L;
+           bound < (long double)kMaxRate;
 }
 
 template <class T>
@@ -153,8 +153,7 @@ bool build_rates_fixed(HostMechanism& m) {
     std::vector<Reaction> rx(R);
     std::vector<ReactionX> fx(R);
     const int third = H.group_end[1];  // models 2-5 follow
-    std::vector<FalloffX> ff(R > third ? (R - third + 3) / 4 * 4 : 0);
-    if (!ff.empty()) std::memset(ff.data(), 0, ff.size() * sizeof(FalloffX));
+    std::vector<FalloffX> ff(R > third ? R - third : 0);
     for (int r = 0; r < R; r++) {
         at(H.off_reactions, r, sizeof(Reaction), &rx[r]);
         const Reaction& x = rx[r];
@@ -167,6 +166,8 @@ bool build_rates_fixed(HostMechanism& m) {
         for (int i = 0; i < x.n_p; i++) factors_p += x.p_n[i];
         for (int i = 0; i < x.n_net; i++) small &= std::abs((int)x.net_n[i]) <= 2;
         small &= factors_r <= 2 && (x.model == 1 || factors_p <= 2);
+        const bool power = x.model <= 1 && !x.k.has_x && x.k.factor != kNone;  // A T^n
+        small &= !power;
         f.shape = (uint32_t)(x.minus_sigma_net + 2) * kShapeMsn;
         if (x.model == 1 && (x.minus_sigma_net < -2 || x.minus_sigma_net > 5)) f.shape = 0;  // unused there
         if (small) {
@@ -201,7 +202,12 @@ bool build_rates_fixed(HostMechanism& m) {
         Falloff fo;
         if (x.falloff >= 0) at(H.off_falloff, x.falloff, sizeof fo, &fo);
         const bool const_k = x.model == 4 && (fo.flags & kKinfConst);
-        if (!const_k && !arrhenius_fix(x.k, f.k, bound, x.model == 4)) return false;
+        if (!const_k && !arrhenius_fix(x.k, f.k, bound, true)) return false;
+        if (power) {
+            f.k.b = {0, x.k.factor};
+            f.k.e = {0, kExactRate};
+            std::memcpy(&f.k.a, &x.k.A, sizeof f.k.a);
+        }
         if (x.model != 1) {  // the equilibrium constant's logarithm stays in range
             long double b = 2.0L * (30.0L + 13.0L);
             for (int i = 0; i < x.n_net; i++) b += std::abs((int)x.net_n[i]) * g_bound[x.net_k[i]];
@@ -209,8 +215,10 @@ bool build_rates_fixed(HostMechanism& m) {
         }
         if (r >= third) {
             FalloffX& g = ff[r - third];
+            std::memset(&g, 0, sizeof g);
             if (x.falloff >= 0) {
-                if (!arrhenius_fix(fo.k0, g.k0, bound, x.model == 4)) return false;
+                // (of a Troe reaction when k_inf is a constant too: otherwise their logarithms are added)
+                if (!arrhenius_fix(fo.k0, g.k0, bound, x.model != 4 || const_k)) return false;
                 g.ainf = fo.ainf;
                 if (x.model == 4 && (!(fo.ainf > 0.) || !to_fix(std::log2((long double)fo.ainf), kYq, 1000.0L, g.lainf)))
                     return false;
@@ -221,12 +229,6 @@ bool build_rates_fixed(HostMechanism& m) {
                 g.cmT2 = (double)((long double)fo.cmT2 * kLog2e);
                 g.l2_fcent = (double)((long double)fo.ln_fcent * kLog2e);
                 g.flags = fo.flags;
-                if (x.model == 4 && !fo.k0.has_x && (const_k || !x.k.has_x)) {
-                    g.flags |= kTroeExact;
-                    g.a0 = fo.k0.A;
-                    g.power0 = fo.k0.factor;
-                    g.power_inf = const_k ? (int)kNone : x.k.factor;
-                }
                 g.sri_flags = fo.sri_flags;
                 g.sA = fo.sA;
                 g.smB = (double)((long double)fo.smB * kLog2e);
@@ -237,28 +239,29 @@ bool build_rates_fixed(HostMechanism& m) {
         }
     }
 
-    // third-body efficiencies minus one, rows padded to a multiple of 4 like the FP64 table's, a unit of its own each
+    // third-body efficiencies minus one, rows padded to a multiple of 4 like the FP64 table's, a unit for every four
     const size_t n_e = (size_t)(H.n_eff + 3) / 4 * 4 * K;
     std::vector<double> eff(n_e);
     if (n_e) std::memcpy(eff.data(), blob + H.off_eff, n_e * sizeof(double));
     std::vector<Word2> ef(n_e);
-    for (size_t row = 0; row < n_e / K; row++) {
-        const double* e = &eff[row * K];
+    std::vector<int32_t> eq(n_e / K / 4);
+    for (size_t g = 0; g < eq.size(); g++) {
+        const double* e = &eff[4 * g * K];
         long double largest = 0.0L, sum = 0.0L;
-        for (int k = 0; k < K; k++) {
-            largest = std::max(largest, std::fabs((long double)e[k]));
-            sum += std::fabs((long double)e[k]);
+        for (int row = 0; row < 4; row++) {
+            long double s = 0.0L;
+            for (int k = 0; k < K; k++) {
+                largest = std::max(largest, std::fabs((long double)e[row * K + k]));
+                s += std::fabs((long double)e[row * K + k]);
+            }
+            sum = std::max(sum, s);
         }
-        if (!(largest < 256.0L)) return false;
+        if (!(largest < (long double)kMaxEff)) return false;
         int q = 29;
         while (std::ldexp(largest, q) > 2147483646.0L || std::ldexp(sum, q) + K > std::ldexp(1.0L, 33)) q--;
-        for (int k = 0; k < K; k++)
-            ef[row * K + k] = words((int64_t)std::llround(std::ldexp((long double)e[k], q + kThirdLo)), kThirdLo);
-        // the sum, at most 1 + 2 largest, below 2^60 in its unit (2^62 where the high words leave no bits below)
-        int top = 0;
-        while (std::ldexp(1.0L, top) < 1.0L + 2.0L * largest) top++;
-        ff[row].m_up = std::min(std::max(59 - top - q - 30, 0), kThirdLo - 1);
-        ff[row].m_q = q + 30 + ff[row].m_up;
+        for (int i = 0; i < 4 * K; i++)
+            ef[4 * g * K + i] = words((int64_t)std::llround(std::ldexp((long double)e[i], q + kThirdLo)), kThirdLo);
+        eq[g] = q;
     }
 
     std::vector<uint8_t>& b = m.rates_fixed_blob;
@@ -272,6 +275,7 @@ bool build_rates_fixed(HostMechanism& m) {
     X.off_reactions = put(b, fx.data(), fx.size());
     X.off_falloff = put(b, ff.data(), ff.size());
     X.off_eff = put(b, ef.data(), ef.size());
+    X.off_eff_q = put(b, eq.data(), eq.size());
     std::vector<int32_t> start(K + 1, 0), lists;
     for (int k = 0; k < K; k++) {
         for (int r = 0; r < R; r++)

@@ -21,7 +21,7 @@ namespace cbg {
 template <int KMAX>
 struct CellX {
     TempsX t;
-    double Ctot;
+    double rcpT, Ctot;
     long long ctot;    // Ctot over S, Q60
     int ex;            // S = 2^ex
     double C[KMAX];    // concentrations, bulk last
@@ -47,13 +47,14 @@ __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pres
     if (!(T >= kFixTmin && T < kFixTmax)) return false;
     // both reciprocals and the products rounded as the reference's: the bulk concentration is a difference of
     // totals, whose last bits it magnifies
-    const double md = __drcp_rn(V), rcpT = __drcp_rn(T);
+    const double md = __drcp_rn(V);
+    c.rcpT = __drcp_rn(T);
     double sum = 0.0;
     for (int k = 0; k < K - 1; k++) {
         c.C[k] = __dmul_rn(md, max0(amounts[k][i]));
         sum += c.C[k];
     }
-    c.Ctot = __dmul_rn(pressure_R, rcpT);
+    c.Ctot = __dmul_rn(pressure_R, c.rcpT);
     const double S = sum > c.Ctot ? sum : c.Ctot;
     if (!totals_in_range(sum, c.Ctot, S)) return false;
     c.C[K - 1] = c.Ctot - sum;
@@ -61,7 +62,7 @@ __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pres
     c.ctot = dbl_to_fix(c.Ctot, 60 - c.ex);
     if (H.n_eff)
         for (int k = 0; k < K; k++) c.cw[k] = split_word<kThirdLo>(dbl_to_fix(c.C[k], 60 - c.ex));
-    c.t = make_temps(H, T, rcpT);
+    c.t = make_temps(H, T, c.rcpT);
     for (int k = 0; k < A; k++) {
         const SpeciesX& s = tb.species[k];
         if (!(s.need_exp | s.need_exp_neg)) continue;
@@ -78,12 +79,11 @@ __device__ __forceinline__ void plain_group_x(const RatesXTables& tb, const Cell
             tb, r, c, w, [&](const ArrheniusX& k) { return rate_constant(k, c.t); }, emit);
 }
 
-// Third-body concentration of a row from its two partial sums (reaction.rs:141-145): Ctot + sum (e - 1) C.
-template <class CellT>
-__device__ __forceinline__ double third_body(const CellT& c, const FalloffX& row, long long s1, long long s2) {
-    const int up = row.m_up, down = kThirdLo - up, q = row.m_q;  // down >= 1, q <= 59
-    const long long ctot = (c.ctot + (1ll << (59 - q))) >> (60 - q);
-    return fix_to_dbl(ctot + (s1 << up) + ((s2 + (1ll << (down - 1))) >> down), q - c.ex);
+// Third-body concentration of a row from its two partial sums (reaction.rs:141-145): Ctot + sum (e - 1) C, in the unit of
+// its four rows, 2^-(q + 30) S.
+__device__ __forceinline__ long long third_body_total(long long ctot, int q) { return (ctot + (1ll << (29 - q))) >> (30 - q); }
+__device__ __forceinline__ double third_body(long long total, int unit, long long s1, long long s2) {
+    return fix_to_dbl(total + s1 + ((s2 + (1ll << (kThirdLo - 1))) >> kThirdLo), unit);
 }
 
 // Models 2-5: the third-body sums of four consecutive rows in one pass over the concentrations (three
@@ -100,9 +100,10 @@ __device__ __forceinline__ void third_body_groups_x(const RatesXTables& tb, cons
 #pragma unroll
             for (int q = 0; q < 4; q++) dot_term(E[q * K + k], ck, s1[q], s2[q]);
         }
-        const FalloffX* row = tb.falloff + (r0 - r_begin);
-        const double M0 = third_body(c, row[0], s1[0], s2[0]), M1 = third_body(c, row[1], s1[1], s2[1]);
-        const double M2 = third_body(c, row[2], s1[2], s2[2]), M3 = third_body(c, row[3], s1[3], s2[3]);
+        const int eq = tb.eff_q[(r0 - r_begin) >> 2], unit = eq + 30 - c.ex;
+        const long long total = third_body_total(c.ctot, eq);
+        const double M0 = third_body(total, unit, s1[0], s2[0]), M1 = third_body(total, unit, s1[1], s2[1]);
+        const double M2 = third_body(total, unit, s1[2], s2[2]), M3 = third_body(total, unit, s1[3], s2[3]);
         const int rq = min(r_end - r0, 4);
 #pragma unroll 1
         for (int q = 0; q < rq; q++) {
@@ -110,10 +111,10 @@ __device__ __forceinline__ void third_body_groups_x(const RatesXTables& tb, cons
             const double M = q == 0 ? M0 : q == 1 ? M1 : q == 2 ? M2 : M3;
             const FalloffX* f = tb.falloff + (r - r_begin);
             auto forward = [&](const ArrheniusX& k) {
-                if (r < H.group_end[2]) return forward_x<2>(H, k, f, c.t, M);
-                if (r < H.group_end[3]) return forward_x<3>(H, k, f, c.t, M);
-                if (r < H.group_end[4]) return forward_x<4>(H, k, f, c.t, M);
-                return forward_x<5>(H, k, f, c.t, M);
+                if (r < H.group_end[2]) return forward_x<2>(H, k, f, c.t, c.rcpT, M);
+                if (r < H.group_end[3]) return forward_x<3>(H, k, f, c.t, c.rcpT, M);
+                if (r < H.group_end[4]) return forward_x<4>(H, k, f, c.t, c.rcpT, M);
+                return forward_x<5>(H, k, f, c.t, c.rcpT, M);
             };
             reaction_x<true, SUM>(tb, r, c, w, forward, emit);
         }
@@ -227,7 +228,7 @@ constexpr int kRatesWarps = 16;  // cells per block at most
 template <int KMAX>
 struct CellXW {
     TempsX t;
-    double Ctot;
+    double rcpT, Ctot;
     long long ctot;
     int ex;
     const double* C;
@@ -250,7 +251,8 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
     long long* g = reinterpret_cast<long long*>(sh + 2 * K);
     double* M = sh + 4 * K;
     double* cR = M + H.n_eff;
-    const double md = __drcp_rn(V), rcpT = __drcp_rn(T);
+    const double md = __drcp_rn(V);
+    c.rcpT = __drcp_rn(T);
     for (int k = lane; k < K - 1; k += kStep) C[k] = __dmul_rn(md, max0(amounts[k][i]));
     team_sync<TEAM>();
     double sum = 0.0;
@@ -259,14 +261,14 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
         for (int k = 0; k < K - 1; k++) sum += C[k];
     }
     sum = team_value<TEAM>(sum, sh + 3 * K, lane);
-    c.Ctot = __dmul_rn(pressure_R, rcpT);
+    c.Ctot = __dmul_rn(pressure_R, c.rcpT);
     const double S = sum > c.Ctot ? sum : c.Ctot;
     if (!totals_in_range(sum, c.Ctot, S)) return false;
     if (lane == 0) C[K - 1] = c.Ctot - sum;
     team_sync<TEAM>();
     c.ex = exponent_above_x(S);
     c.ctot = dbl_to_fix(c.Ctot, 60 - c.ex);
-    c.t = make_temps(H, T, rcpT);
+    c.t = make_temps(H, T, c.rcpT);
     c.C = C;
     c.g = g;
     for (int k = lane; k < K; k += kStep) {
@@ -280,7 +282,8 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
         long long s1 = 0, s2 = 0;
 #pragma unroll 4
         for (int k = 0; k < K; k++) dot_term(E[k], Word2{__double2hiint(cw[k]), __double2loint(cw[k])}, s1, s2);
-        M[e] = third_body(c, tb.falloff[e], s1, s2);
+        const int eq = tb.eff_q[e >> 2];
+        M[e] = third_body(third_body_total(c.ctot, eq), eq + 30 - c.ex, s1, s2);
     }
     team_sync<TEAM>();
     const int first = H.group_end[1];
@@ -299,10 +302,10 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
                 auto forward = [&](const ArrheniusX& k) {
                     if (m == 0) return rate_constant(k, c.t);
                     const FalloffX* f = tb.falloff + (r - first);
-                    if (m == 2) return forward_x<2>(H, k, f, c.t, M[r - first]);
-                    if (m == 3) return forward_x<3>(H, k, f, c.t, M[r - first]);
-                    if (m == 4) return forward_x<4>(H, k, f, c.t, M[r - first]);
-                    return forward_x<5>(H, k, f, c.t, M[r - first]);
+                    if (m == 2) return forward_x<2>(H, k, f, c.t, c.rcpT, M[r - first]);
+                    if (m == 3) return forward_x<3>(H, k, f, c.t, c.rcpT, M[r - first]);
+                    if (m == 4) return forward_x<4>(H, k, f, c.t, c.rcpT, M[r - first]);
+                    return forward_x<5>(H, k, f, c.t, c.rcpT, M[r - first]);
                 };
                 reaction_x<true, false>(tb, r, c, nullptr, forward, store);
             }

@@ -19,6 +19,7 @@ struct RatesXTables {
     const ReactionX* reactions;
     const FalloffX* falloff;
     const Word2* eff;
+    const int32_t* eff_q;
     const int32_t *csr_start, *csr;
     __device__ explicit RatesXTables(const uint8_t* tab)
         : H(reinterpret_cast<const RatesXHeader*>(tab + kMathBytes + kFixMathBytes)),
@@ -27,13 +28,14 @@ struct RatesXTables {
           reactions(reinterpret_cast<const ReactionX*>(tab + H->off_reactions)),
           falloff(reinterpret_cast<const FalloffX*>(tab + H->off_falloff)),
           eff(reinterpret_cast<const Word2*>(tab + H->off_eff)),
+          eff_q(reinterpret_cast<const int32_t*>(tab + H->off_eff_q)),
           csr_start(reinterpret_cast<const int32_t*>(tab + H->off_csr_start)),
           csr(reinterpret_cast<const int32_t*>(tab + H->off_csr)) {}
 };
 
 // A cell's temperature in fixed point.
 struct TempsX {
-    double T, rcpT;
+    double T;
     Word2 l, r, p[4];   // log2 T, 1/T, (T / 2^pw)^i with pw = 11 below kFixTmid, else 13
     long long lc0;      // log2(P0 / (R T)), Qy
 };
@@ -41,7 +43,6 @@ struct TempsX {
 __device__ __forceinline__ TempsX make_temps(const RatesXHeader& H, double T, double rcpT) {
     TempsX t;
     t.T = T;
-    t.rcpT = rcpT;
     int e;
     const long long f = log2_frac(T, e);
     t.l = split_word(((long long)e << (kLq + kLo)) + ((f + 32) >> 6));
@@ -65,8 +66,8 @@ __device__ __forceinline__ long long arrhenius_log2(const ArrheniusX& a, const T
     return dot_value(s1, s2);
 }
 // min(f32::MAX, A T^power), as the FP64 form's arrhenius.
-static __device__ __noinline__ double rate_exact(int power, double A, double T, double rcpT) {
-    const double T2 = T * T;
+static __device__ __noinline__ double rate_exact(int power, double A, double T) {
+    const double T2 = T * T, rcpT = __drcp_rn(T);
     double f = 1.0;
     switch (power) {
     case kRcpT2: f = rcpT * rcpT; break;
@@ -80,7 +81,6 @@ static __device__ __noinline__ double rate_exact(int power, double A, double T, 
 }
 // min(f32::MAX, k) of reaction.rs:138.
 __device__ __forceinline__ double rate_constant(const ArrheniusX& a, const TempsX& t) {
-    if (a.e.hi == kExactRate) return rate_exact(a.b.hi, __longlong_as_double(a.a), t.T, t.rcpT);
     return rate_fix(arrhenius_log2(a, t));
 }
 
@@ -129,15 +129,14 @@ __device__ __forceinline__ double heat_capacity_x(const ThermoX& s, int set, con
 
 // The Troe forward coefficient in the general case (reaction.rs:160-193).
 static __device__ __noinline__ double troe_general(const RatesXHeader& H, const FalloffX& f, long long y0, long long yi,
-                                                   double lF, double M, double T, double rcpT) {
-    const bool exact = f.flags & kTroeExact;
-    const double k0 = exact ? rate_exact(f.power0, f.a0, T, rcpT) : rate_fix(y0);
+                                                   double lF, double M) {
+    const double k0 = rate_fix(y0);
     double Pr, kinf;
     if (f.flags & kKinfConst) {
         Pr = M * k0;
         kinf = f.ainf;
     } else {
-        const double ki = exact ? rate_exact(f.power_inf, 1.0, T, rcpT) : rate_fix(yi);
+        const double ki = rate_fix(yi);
         Pr = div64(M * k0, ki + kF32MinPos);
         kinf = f.ainf * ki;
     }
@@ -152,7 +151,7 @@ static __device__ __noinline__ double troe_general(const RatesXHeader& H, const 
 // Forward coefficient of one reaction: k, k M, or the falloff-blended value (reaction.rs:149-203).
 template <int MODEL>
 __device__ __forceinline__ double forward_x(const RatesXHeader& H, const ArrheniusX& k, const FalloffX* fo,
-                                            const TempsX& t, double M) {
+                                            const TempsX& t, double rcpT, double M) {
     if constexpr (MODEL == 4) {  // Troe (reaction.rs:160-193), logarithms in base 2
         const FalloffX& f = *fo;
         double lF;
@@ -163,23 +162,23 @@ __device__ __forceinline__ double forward_x(const RatesXHeader& H, const Arrheni
             if (f.flags & kTermT3) F = f.c1mA * exp2_dbl(t.T * f.c3);
             if (f.flags & kTermT1) F += f.cA * exp2_dbl(t.T * f.c1);
             if (f.flags & kTermAConst) F += f.cA;
-            if (f.flags & kTermT2) F += exp2_dbl(f.cmT2 * t.rcpT);
+            if (f.flags & kTermT2) F += exp2_dbl(f.cmT2 * rcpT);
             lF = log2_dbl(F);
         }
         const long long y0 = arrhenius_log2(f.k0, t), yi = f.flags & kKinfConst ? 0 : arrhenius_log2(k, t);
         // log2 Pr = log2 M + log2 k0 - log2 k_inf, and k = F A_inf k_inf Pr / (1 + Pr) by its logarithm, while
-        // neither coefficient is capped at f32::MAX and f32::MIN_POSITIVE vanishes next to k_inf and Pr, and one of them
-        // at least is an exponential
-        if ((f.flags & kTroeExact) || !(M > 1e-200 && M < 1e200) || y0 >= (127ll << kYq) || yi >= (127ll << kYq) || yi < -(60ll << kYq))
-            return troe_general(H, f, y0, yi, lF, M, t.T, t.rcpT);
+        // neither coefficient is capped at f32::MAX and f32::MIN_POSITIVE vanishes next to k_inf and Pr
+        // (nor k0 a constant: its y0 is above all others)
+        if (!(M > 1e-200 && M < 1e200) || y0 >= (127ll << kYq) || yi >= (127ll << kYq) || yi < -(60ll << kYq))
+            return troe_general(H, f, y0, yi, lF, M);
         const long long lPr = log2_fix(M) + y0 - yi;
-        if (lPr < -(60ll << kYq) || lPr > (1000ll << kYq)) return troe_general(H, f, y0, yi, lF, M, t.T, t.rcpT);
+        if (lPr < -(60ll << kYq) || lPr > (1000ll << kYq)) return troe_general(H, f, y0, yi, lF, M);
         const double Cc = fma(-0.67, lF, -H.l10_04);
         const double Nn = fma(-1.27, lF, H.l10_075);
         const double lPrC = fix_to_dbl(lPr, kYq) + Cc;
         const double f1 = div64(lPrC, fma(-0.14, lPrC, Nn));
         const double lFb = div64(lF, fma(f1, f1, 1.0));
-        if (!(lFb > -1000.0 && lFb < 1000.0)) return troe_general(H, f, y0, yi, lF, M, t.T, t.rcpT);
+        if (!(lFb > -1000.0 && lFb < 1000.0)) return troe_general(H, f, y0, yi, lF, M);
         return exp2_fix(dbl_to_fix(lFb, kYq) + f.lainf + yi + lPr - log2_fix(exp2_core(lPr) + 1.0));
     } else if constexpr (MODEL == 3) {  // Lindemann (reaction.rs:153-159)
         const double Ck0 = M * rate_constant(fo->k0, t);
@@ -192,7 +191,7 @@ __device__ __forceinline__ double forward_x(const RatesXHeader& H, const Arrheni
         const double Pr = div64(M * k0, ki + kF32MinPos);
         const double lP = log2_dbl(Pr + kF32MinPos) * 0.69314718055994530942;  // natural
         double base = exp2_dbl(f.smrC * t.T);
-        if (f.sri_flags & kSriA) base = fma(f.sA, exp2_dbl(f.smB * t.rcpT), base);
+        if (f.sri_flags & kSriA) base = fma(f.sA, exp2_dbl(f.smB * rcpT), base);
         double F = exp2_dbl(log2_dbl(base) * rcp64(fma(lP, lP, 1.0)));
         if (f.sri_flags & kSriD) F = f.sD * F;
         if (f.sri_flags & kSriE) F *= exp2_dbl(f.sE * log2_dbl(t.T));
@@ -304,7 +303,7 @@ __device__ __forceinline__ void reaction_x(const RatesXTables& tb, int r, const 
         }
         return;
     }
-    const double kf = forward(x.k);
+    const double kf = x.k.e.lo == kExactRate ? rate_exact(x.k.b.lo, __longlong_as_double(x.k.a), c.t.T) : forward(x.k);
     double Rf = 1.0, Pp = 1.0;
 #pragma unroll 1
     for (int q = 0; q < kMaxSide; q++) {

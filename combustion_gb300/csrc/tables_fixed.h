@@ -32,25 +32,32 @@ constexpr int kRq = 37;    // 1 / T, hi word (1/T <= 1/200)
 constexpr int kEq = 14;    // its factor, |.| < 2^17
 constexpr int kPq = 30;    // (T / 2^p)^i, hi word, p = 11 below 2048 K and 13 above
 constexpr int kGq = 18;    // its factor, |.| < 4096
-// Third-body sums: C_k / S (S a power of two above both totals) in 60 bits, efficiencies - 1 of a row in units of
-// 2^-(q + kThirdLo), q the largest (at most 29) that keeps the row's high words below 2^31 and their sum below 2^33: then
-// the cross products' sum stays below 2^63. The dropped products of low words are below 2^-(q + 32) S each; the sum's
-// error is below that of FP64 FMAs (an efficiency of 256 beside 52 of 0.5 to 3: largest 4.4e-16 of M, FP64 9.5e-16; with
-// one unit for the whole mechanism and 29-bit low words it was 2.1e-14).
+// Third-body sums: C_k / S (S a power of two above both totals) in 60 bits, efficiencies - 1 of four rows in units of
+// 2^-(q + kThirdLo), q the largest (at most 29) that keeps their high words below 2^31 and the sum of a row's below 2^33:
+// then the cross products' sum stays below 2^63. The dropped products of low words are below 2^-(q + 32) S each; the sum's
+// error is below that of FP64 FMAs for every efficiency that is accepted (of 61 beside 52 of 0.5 to 3 at most 1.9e-16 of
+// M, FP64 9.2e-16; with one unit for the whole mechanism and 29-bit low words 4e-15).
 constexpr int kThirdLo = 30;
+constexpr double kMaxEff = 128.0;  // of |efficiency - 1|
 
 struct Word2 {
     int32_t hi, lo;
 };
 
-// log2 of k = exp(beta ln T + mEa / T + ln A). A constant and a constant times a whole power of T keep their FP64 form
-// (exact, or two roundings, where a logarithm's last bit is 1.5e-16 of k): e.hi = kExactRate, b.hi the power (Factor) and
-// `a` the bits of A.
+// log2 of k = exp(beta ln T + mEa / T + ln A). Coefficients that FP64 holds exactly, or to a rounding or two, are not
+// taken through a logarithm (whose last bit is 1.5e-16 of k):
+//  - a constant is `a` = the bits of A + kConstRate with no factors. As a logarithm it lies above every other one's
+//    (A = 2^-500 .. 2^499 gives 2,046 .. 4,046, the others are below kMaxRate), where rate_slow finds it;
+//  - a constant times a whole power of T, of an elementary reaction, is the bits of A, the power (Factor) in b.lo and
+//    e.lo = kExactRate, in a reaction of general shape. (Where a third body multiplies it, its sum is the more exact for
+//    being in fixed point, and the logarithm's error is no more than that gains.)
 struct ArrheniusX {
     Word2 b, e;  // factors of log2 T and 1 / T
     int64_t a;   // Qy
 };
-constexpr int32_t kExactRate = INT32_MIN;  // beyond any factor of 1 / T
+constexpr int64_t kConstRate = 1000ll << kYq, kConstRateMin = 2046ll << kYq;
+constexpr double kMaxRate = 2000.0;  // of |log2 k|
+constexpr int32_t kExactRate = 1 << 29;  // no balanced low word
 
 // Shape flags of a reaction (ReactionX::shape).
 enum Shape : uint32_t {
@@ -73,18 +80,14 @@ struct ReactionX {  // 64 bytes
 };
 static_assert(sizeof(ReactionX) == 64, "four 16-byte loads");
 
-// One per reaction of models 2-5, in reaction order, padded to a multiple of 4 (of a three-body reaction the
-// efficiencies' unit only). Exponents and logarithms in base 2.
-constexpr int32_t kTroeExact = 1 << 16;  // beside the FP64 tables' flags
+// One per reaction of models 2-5, in reaction order (three-body entries unused). Exponents and
+// logarithms in base 2.
 struct FalloffX {
     ArrheniusX k0;
     double ainf, c1mA, cA, c3, c1, cmT2, l2_fcent;
     int64_t lainf;          // log2(ainf), Qy
     int32_t flags, sri_flags;
     double sA, smB, smrC, sD, sE;
-    double a0;                  // kTroeExact: both coefficients of a Troe reaction are constants times whole powers of T,
-    int32_t power0, power_inf;  // k0 = a0 T^.. and T^.. (1 with kKinfConst)
-    int32_t m_up, m_q;      // the third-body sum's unit is 2^-m_q S, 2^m_up below that of its high words' products
 };
 
 // Gibbs energy over RT in base-2 units: piece 0 for T <= split, else 1 below kFixTmid and 2 above (the
@@ -106,6 +109,7 @@ struct ThermoX {
 
 struct RatesXHeader {
     int32_t K, A, R, n_eff, total_bytes, off_species, off_thermo, off_reactions, off_falloff, off_eff;
+    int32_t off_eff_q;  // q of every four rows
     int32_t off_csr_start, off_csr;  // per species the reactions that change it, in order: [K + 1]; r << 8 | nu
     int32_t group_end[6];
     int64_t lM3, lcbrt, lC0;  // log2 of the Gibbs exponentials' caps and of P0 / R, Qy
