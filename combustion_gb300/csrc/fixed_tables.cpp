@@ -5,6 +5,7 @@
 #include <cstring>
 #include <vector>
 
+#include "kernels.h"
 #include "mechanism.hpp"
 #include "tables_fixed.h"
 
@@ -368,14 +369,24 @@ bool build_transport_fixed(HostMechanism& m) {
                 return false;
             largest = std::max(largest, A2[i]);
         }
-    const int bits = K <= 64 ? kMixAq<64> : kMixAq<256>;
+    const bool wide = kmax_for(K, m.n_eff) > 64;  // the kernels' words go by their capacity
+    const int bits = wide ? kMixAq<256> : kMixAq<64>, low = wide ? kMixLo<256> : kMixLo<64>;
+    const int sum_bits = 2 * low - (wide ? kMixXq<256> : kMixXq<64>);  // high words' products: a row of a^2 over 2^this
+    double row = 0.;
+    for (int k = 0; k < K; k++) {
+        double sum = 0.;
+        for (int j = 0; j < K; j++) sum += A2[(size_t)k * K + j];
+        row = std::max(row, sum);
+    }
     X.a_shift = bits;
     while (std::ldexp(largest, X.a_shift) >= std::ldexp(1.0, bits)) X.a_shift--;
     while (std::ldexp(largest, X.a_shift + 1) < std::ldexp(1.0, bits)) X.a_shift++;
+    while (std::ldexp(row, X.a_shift - sum_bits) >= 0.95 * std::ldexp(1.0, 62)) X.a_shift--;  // (the sums are doubled)
     std::vector<Word2> a2((size_t)K * K);
     for (int k = 0; k < K; k++)
         for (int j = 0; j < K; j++)
-            a2[(size_t)j * K + k] = words((int64_t)std::llround(std::ldexp((long double)A2[(size_t)k * K + j], X.a_shift)));
+            a2[(size_t)j * K + k] =
+                words((int64_t)std::llround(std::ldexp((long double)A2[(size_t)k * K + j], X.a_shift)), low);
 
     std::vector<uint8_t>& b = m.transport_fixed_blob;
     b.insert(b.end(), blob, blob + kMathBytes);

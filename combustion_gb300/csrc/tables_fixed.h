@@ -132,11 +132,15 @@ struct alignas(16) PolyX {  // three 16-byte loads
 static_assert(sizeof(PolyX) == 48, "three 16-byte loads");
 
 // Words of the Wilke sums: a^2 (column j: the rows k, so that rows in registers or lanes read consecutive words) times
-// a cell's X, X/v', X/v'^2 over their largest.
+// a cell's X, X/v', X/v'^2 over their largest. A product of low words is dropped: below 2^-57 of the largest term with 64
+// species. Sums over 256 leave fewer bits; with 27 low ones (54-bit words) it is below 2^-56, and coherent traces beside a
+// main species put viscosities at 250 species off by 6e-16, as FP64 sums (29 of 54 and 55 bits: 2^-53 and 1.4e-14).
+template <int KMAX>
+constexpr int kMixLo = KMAX <= 64 ? 29 : 27;
 template <int KMAX>
 constexpr int kMixAq = KMAX <= 64 ? 56 : 54;  // |a^2| 2^a_shift < 2^this
 template <int KMAX>
-constexpr int kMixXq = KMAX <= 64 ? 57 : 55;  // |X| over a power of two above the largest, < 2^this
+constexpr int kMixXq = KMAX <= 64 ? 57 : 54;  // |X| over a power of two above the largest, < 2^this
 
 struct TransportXHeader {
     int32_t K, n_pairs, total_bytes, pw;

@@ -18,7 +18,7 @@
 namespace cbg {
 
 // Rows k0 .. k0 + Q - 1 of Wilke's sums and their terms of mu (rows k0, k0 + 2 in mu0, the others in mu1).
-template <int Q>
+template <int Q, int LO>
 __device__ __forceinline__ void wilke_rows_x(const TransportXTables& tb, int K, int k0, const double* X, const double* r,
                                                const double* Xw, const double* Yw, const double* Zw, int q1, int q2,
                                                int q3, double& mu0, double& mu1) {
@@ -50,8 +50,8 @@ __device__ __forceinline__ void wilke_rows_x(const TransportXTables& tb, int K, 
 #pragma unroll
     for (int q = 0; q < Q; q++) {
         const double w = wilke_factor(X[k0 + q], tb.W4[k0 + q]),
-                     d = wilke_rcp(mix_value(s[q][0], t[q][0]), mix_value(s[q][1], t[q][1]), mix_value(s[q][2], t[q][2]), q1,
-                                   q2, q3, r[k0 + q]);
+                     d = wilke_rcp(mix_value<LO>(s[q][0], t[q][0]), mix_value<LO>(s[q][1], t[q][1]), mix_value<LO>(s[q][2], t[q][2]),
+                                   q1, q2, q3, r[k0 + q]);
         if (q & 1) mu1 = fma(w, d, mu1);
         else mu0 = fma(w, d, mu0);
     }
@@ -107,6 +107,7 @@ __device__ __forceinline__ void diffusion_rows(const TransportXTables& tb, int k
 
 template <int KMAX>
 __device__ __forceinline__ bool transport_cell_x(const TransportXTables& tb, const TransportArgs<KMAX>& io, size_t i, size_t o) {
+    constexpr int LO = kMixLo<KMAX>;
     const TransportXHeader& H = *tb.H;
     const int K = H.K;
     double N, Tn;
@@ -165,13 +166,13 @@ __device__ __forceinline__ bool transport_cell_x(const TransportXTables& tb, con
     const int qx = kMixXq<KMAX> - exponent_above(mx), qy = kMixXq<KMAX> - exponent_above(my),
               qz = kMixXq<KMAX> - exponent_above(mz);
     for (int k = 0; k < K; k++) {
-        const Word2 x = split_word(dbl_to_fix(X[k], qx)), y = split_word(dbl_to_fix(Y[k], qy)),
-                    z = split_word(dbl_to_fix(Z[k], qz));
+        const Word2 x = split_word<LO>(dbl_to_fix(X[k], qx)), y = split_word<LO>(dbl_to_fix(Y[k], qy)),
+                    z = split_word<LO>(dbl_to_fix(Z[k], qz));
         Xw[k] = __hiloint2double(x.hi, x.lo);
         Y[k] = __hiloint2double(y.hi, y.lo);
         Z[k] = __hiloint2double(z.hi, z.lo);
     }
-    const int unit = H.a_shift + 1 - 2 * kLo;  // of the sums, with the words' positions
+    const int unit = H.a_shift + 1 - 2 * LO;  // of the sums, with the words' positions
     // Two independent parts, the mixing rule on the integer pipe alone and the diffusion on both: half of each
     // sub-partition's warps take them in the other order, so that both pipes have work at any time (131,072 cells at 250
     // species 54.0 -> 44.3 ms; at 10 species the loops are too short to gain).
@@ -182,10 +183,10 @@ __device__ __forceinline__ bool transport_cell_x(const TransportXTables& tb, con
         if ((part == 0) != swap) {  // viscosity (transport.rs:148-158)
             double mu0 = 0.0, mu1 = 0.0;  // even and odd species
 #pragma unroll 1
-            for (; k + 4 <= K; k += 4) wilke_rows_x<4>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu0, mu1);
+            for (; k + 4 <= K; k += 4) wilke_rows_x<4, LO>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu0, mu1);
 #pragma unroll 1
-            for (; k + 2 <= K; k += 2) wilke_rows_x<2>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu0, mu1);
-            if (k < K) wilke_rows_x<1>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu0, mu1);
+            for (; k + 2 <= K; k += 2) wilke_rows_x<2, LO>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu0, mu1);
+            if (k < K) wilke_rows_x<1, LO>(tb, K, k, X, r, Xw, Y, Z, unit + qx, unit + qy, unit + qz, mu0, mu1);
             io.out[1][o] = VT * (mu0 + mu1);
         } else {  // mixture-averaged diffusion (transport.rs:162-177)
 #pragma unroll 1
@@ -236,6 +237,7 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
                                                       size_t o, double* sh, bool second) {
     constexpr int kStep = 32 * TEAM;
     const int lane = TEAM == 1 ? threadIdx.x & 31 : threadIdx.x, lane32 = threadIdx.x & 31;
+    constexpr int LO = kMixLo<KMAX>;
     const TransportXHeader& H = *tb.H;
     const int K = H.K;
     double N, Tn;
@@ -311,14 +313,14 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
     double* Xw = T;  // the tile holds X's words and the viscosity terms until the diffusion
     double* U = T + KMAX;
     for (int k = lane; k < K; k += kStep) {
-        const Word2 x = split_word(dbl_to_fix(X[k], qx)), y = split_word(dbl_to_fix(Y[k], qy)),
-                    z = split_word(dbl_to_fix(Z[k], qz));
+        const Word2 x = split_word<LO>(dbl_to_fix(X[k], qx)), y = split_word<LO>(dbl_to_fix(Y[k], qy)),
+                    z = split_word<LO>(dbl_to_fix(Z[k], qz));
         Xw[k] = __hiloint2double(x.hi, x.lo);
         Y[k] = __hiloint2double(y.hi, y.lo);
         Z[k] = __hiloint2double(z.hi, z.lo);
     }
     team_sync<TEAM>();
-    const int unit = H.a_shift + 1 - 2 * kLo;
+    const int unit = H.a_shift + 1 - 2 * LO;
 #pragma unroll 1
     for (int k = lane; k < K; k += kStep) {
         const Word2* a = tb.A2 + k;
@@ -331,8 +333,8 @@ __device__ __forceinline__ bool transport_cell_x_warp(const TransportXTables& tb
             dot_term(w, Word2{__double2hiint(Z[j]), __double2loint(Z[j])}, s[2], t[2]);
         }
         U[2 * k] = wilke_factor(X[k], tb.W4[k]);
-        U[2 * k + 1] = wilke_rcp(mix_value(s[0], t[0]), mix_value(s[1], t[1]), mix_value(s[2], t[2]), unit + qx, unit + qy,
-                                 unit + qz, v[k]);
+        U[2 * k + 1] = wilke_rcp(mix_value<LO>(s[0], t[0]), mix_value<LO>(s[1], t[1]), mix_value<LO>(s[2], t[2]), unit + qx,
+                                 unit + qy, unit + qz, v[k]);
     }
     team_sync<TEAM>();
     double mu = 0.0;

@@ -61,8 +61,9 @@ __device__ __forceinline__ double diffusion_x(double MN, double VT, double W, do
     return __dmul_rn(__dmul_rn(fma(-W, X, MN), VT), rcp64(S));
 }
 // The three sums' accumulators to values in one unit (one bit finer than the hi-hi products').
+template <int LO>
 __device__ __forceinline__ long long mix_value(long long s1, long long s2) {
-    return (s1 << 1) + ((s2 + (1ll << (kLo - 2))) >> (kLo - 1));
+    return (s1 << 1) + ((s2 + (1ll << (LO - 2))) >> (LO - 1));
 }
 
 }  // namespace cbg

@@ -347,3 +347,52 @@ def test_exact_rate_constants(config):
             err = np.abs((out[r] - ref) / ref).astype(np.float64).max()
             print(f"{config} Troe, T^{b}: max error {err:.2e}")
             assert err <= 4e-15
+
+
+def test_coherent_traces():
+    """Viscosity at 250 species of a main species and traces whose words' low halves all have the sign of their matrix
+    words' (in words of 29 low bits, the worst case of what the integer sums drop): as close to long double as FP64 sums,
+    6e-16 and the roundings of a dozen operations beside them."""
+    import torch
+    import combustion_gb300 as cb
+    LD = np.longdouble
+    m = util.mechanism("k250")
+    K, W = m.K, m.molar_mass.astype(LD)
+    mech = cb.Mechanism(m)
+    T0, mu0, l0 = synthetic.transport_scales(m)
+    mech.transport_setup(T0, mu0, l0)
+    visc = mech.transport_coefficients()[1].astype(LD) * (np.sqrt(np.sqrt(LD(T0))) / np.sqrt(LD(mu0)))
+    va = np.sqrt(1 / np.sqrt(LD(8)) / np.sqrt(1 + W[:, None] / W))
+    b = va * (W / W[:, None]) ** LD(0.25)
+    word = np.rint(np.ldexp(va * va, 55)).astype(np.int64)  # the largest below 2^54
+    assert 2 ** 53 <= word.max() < 2 ** 54
+    low = word - ((word + (1 << 28) >> 29) << 29)
+    mains = [K - 1, 0, 100, 17]
+    x = np.zeros((K + 1, len(mains) * 3))  # sum n, T/T0, n_0 ..
+    for i, k in enumerate(mains):
+        for j, trace in enumerate((2.0 ** -27, 2.0 ** -28, 2.0 ** -26 * 0.999)):
+            X = np.where(low[k] > 0, trace, 0.0)
+            X[k] = 1.0
+            x[2:, 3 * i + j] = X[:-1]
+            s = 0.0
+            for v in X[:-1]:
+                s = s + v
+            x[0, 3 * i + j] = s + X[-1]
+    x[1] = 1500.0 / T0
+    for reps in (1, 40, 152 * 260 // x.shape[1] + 1):
+        large = torch.empty((K + 2, x.shape[1] * reps), dtype=torch.float64, device="cuda")
+        mech.transport(dev(np.tile(x, (1, reps))), large)
+        mech.synchronize()
+        out = large[1, -x.shape[1]:].cpu().numpy()
+        for c in range(x.shape[1]):
+            n = x[2:, c]
+            s = 0.0
+            for v in n:
+                s = s + v
+            X = np.append(n, x[0, c] - s).astype(LD)
+            L = np.log(LD(x[1, c]))
+            v = (visc * np.array([L ** i for i in range(5)])).sum(1)
+            mu = sum(X[k] * v[k] ** 2 / (X * (va[k] + b[k] * v[k] / v) ** 2).sum() for k in range(K) if X[k] > 0)
+            err = float(abs((out[c] - np.sqrt(LD(x[1, c])) * mu) / (np.sqrt(LD(x[1, c])) * mu)))
+            print(f"main species {mains[c // 3]}, {x.shape[1] * reps} cells: {err:.2e}")
+            assert err <= 2e-15
