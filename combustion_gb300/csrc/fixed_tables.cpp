@@ -3,6 +3,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
 #include <vector>
 
 #include "kernels.h"
@@ -34,7 +35,7 @@ bool to_words(long double x, int q_hi, long double limit, Word2& w, int lo = kLo
 
 // k = exp(x) or A times a power of T, as log2 k; `bound` receives the largest |log2 k| over the fixed-point temperature
 // range. `constant`: a constant as itself (kConstRate).
-bool arrhenius_fix(const Arrhenius& a, ArrheniusX& f, long double& bound, bool constant) {
+bool arrhenius_fix(const Arrhenius& a, double Tmin, ArrheniusX& f, long double& bound, bool constant) {
     static const int power[] = {0, -2, -1, 4, 3, 2, 1};  // Factor
     const long double beta = a.has_x ? (long double)a.beta : (long double)power[a.factor];
     const long double e = a.has_x ? (long double)a.mEa * kLog2e : 0.0L;
@@ -46,7 +47,7 @@ bool arrhenius_fix(const Arrhenius& a, ArrheniusX& f, long double& bound, bool c
         return true;
     }
     const long double l = a.has_x ? (long double)a.lnA * kLog2e : std::log2((long double)a.A);
-    bound = std::fabs(l) + std::fabs(beta) * 13.0L + std::fabs(e) / (long double)kFixTmin;
+    bound = std::fabs(l) + std::fabs(beta) * 13.0L + std::fabs(e) / (long double)Tmin;
     return to_words(beta, kBq, 64.0L, f.b) && to_words(e, kEq, 131000.0L, f.e) && to_fix(l, kYq, 4000.0L, f.a) &&
            bound < (long double)kMaxRate;
 }
@@ -75,7 +76,8 @@ FixMath make_fix_math() {
     return t;
 }
 
-bool build_rates_fixed(HostMechanism& m) {
+namespace {
+bool build_rates(HostMechanism& m, double Tmin) {
     m.rates_fixed_blob.clear();
     const uint8_t* blob = m.rates_blob.data();
     RatesHeader H;
@@ -90,6 +92,7 @@ bool build_rates_fixed(HostMechanism& m) {
     X.R = R;
     X.n_eff = H.n_eff;
     std::memcpy(X.group_end, H.group_end, sizeof X.group_end);
+    X.Tmin = Tmin;
     X.l10_04 = (double)(0.4L * std::log2(10.0L));
     X.l10_075 = (double)(0.75L * std::log2(10.0L));
     if (!to_fix(std::log2((long double)H.M3), kYq, 4000.0L, X.lM3) ||
@@ -115,7 +118,7 @@ bool build_rates_fixed(HostMechanism& m) {
             const double* g = s.g[std::isnan(s.split) ? 0 : set == 0 ? 0 : 1];
             const int p = set == 2 ? 13 : 11;
             long double b = std::fabs((long double)g[0]) * kLog2e + std::fabs((long double)g[1]) * 13.0L +
-                            std::fabs((long double)g[6]) * kLog2e / (long double)kFixTmin;
+                            std::fabs((long double)g[6]) * kLog2e / (long double)Tmin;
             bool ok = to_fix((long double)g[0] * kLog2e, kYq, 2000.0L, f.g0[set]) &&
                       to_words((long double)g[1], kBq, 64.0L, f.g[set][0]) &&
                       to_words((long double)g[6] * kLog2e, kEq, 131000.0L, f.g[set][1]);
@@ -203,7 +206,7 @@ bool build_rates_fixed(HostMechanism& m) {
         Falloff fo;
         if (x.falloff >= 0) at(H.off_falloff, x.falloff, sizeof fo, &fo);
         const bool const_k = x.model == 4 && (fo.flags & kKinfConst);
-        if (!const_k && !arrhenius_fix(x.k, f.k, bound, true)) return false;
+        if (!const_k && !arrhenius_fix(x.k, Tmin, f.k, bound, true)) return false;
         if (power) {
             f.k.b = {0, x.k.factor};
             f.k.e = {0, kExactRate};
@@ -219,7 +222,7 @@ bool build_rates_fixed(HostMechanism& m) {
             std::memset(&g, 0, sizeof g);
             if (x.falloff >= 0) {
                 // (of a Troe reaction when k_inf is a constant too: otherwise their logarithms are added)
-                if (!arrhenius_fix(fo.k0, g.k0, bound, x.model != 4 || const_k)) return false;
+                if (!arrhenius_fix(fo.k0, Tmin, g.k0, bound, x.model != 4 || const_k)) return false;
                 g.ainf = fo.ainf;
                 if (x.model == 4 && (!(fo.ainf > 0.) || !to_fix(std::log2((long double)fo.ainf), kYq, 1000.0L, g.lainf)))
                     return false;
@@ -291,13 +294,20 @@ bool build_rates_fixed(HostMechanism& m) {
     std::memcpy(b.data() + off_header, &X, sizeof X);
     return true;
 }
+}  // namespace
+
+bool build_rates_fixed(HostMechanism& m) {
+    for (double Tmin : kFixTmin)
+        if (build_rates(m, Tmin)) return true;
+    return false;
+}
 
 namespace {
 
 // A polynomial over the fixed-point temperature range: positive, within a factor of 2^5, coefficients that fit.
-bool poly_fix(const double* P, double T0, int pw, long double scale, PolyX& f) {
+bool poly_fix(const double* P, double Tn_lo, double Tn_hi, int pw, long double scale, PolyX& f) {
     long double lo = 1e300L, hi = 0.0L;
-    const long double a = std::log((long double)kFixTransportTmin / T0), b = std::log((long double)kFixTransportTmax / T0);
+    const long double a = std::log((long double)Tn_lo), b = std::log((long double)Tn_hi);
     for (int i = 0; i <= 256; i++) {
         const long double L = a + (b - a) * i / 256.0L;
         const long double D = scale * (P[0] + L * (P[1] + L * (P[2] + L * (P[3] + L * (long double)P[4]))));
@@ -316,9 +326,15 @@ bool poly_fix(const double* P, double T0, int pw, long double scale, PolyX& f) {
     return true;
 }
 
-}  // namespace
+// Bits of 2^pw above |ln(T/T0)|.
+int log_power(double Tn_lo, double Tn_hi) {
+    const double Lmax = std::max(std::fabs(std::log(Tn_lo)), std::fabs(std::log(Tn_hi)));
+    int pw = 0;
+    while (std::ldexp(1.0, pw) <= Lmax) pw++;
+    return pw;
+}
 
-bool build_transport_fixed(HostMechanism& m) {
+bool build_transport(HostMechanism& m, double Tmin, double Tmax) {
     m.transport_fixed_blob.clear();
     const uint8_t* blob = m.transport_blob.data();
     TransportHeader H;
@@ -339,11 +355,11 @@ bool build_transport_fixed(HostMechanism& m) {
     X.K = K;
     X.n_pairs = H.n_pairs;
     X.T0 = H.T0;
-    X.Tn_lo = kFixTransportTmin / H.T0;
-    X.Tn_hi = kFixTransportTmax / H.T0;
-    const double Lmax = std::max(std::fabs(std::log(X.Tn_lo)), std::fabs(std::log(X.Tn_hi)));
-    while (std::ldexp(1.0, X.pw) <= Lmax) X.pw++;
-    if (X.pw > 4) return false;
+    X.Tn_lo = Tmin / H.T0;
+    X.Tn_hi = Tmax / H.T0;
+    X.pw = log_power(X.Tn_lo, X.Tn_hi);
+    const double* narrowest = std::end(kFixTransportT)[-1];
+    if (X.pw > 4 || X.pw != log_power(narrowest[0] / H.T0, narrowest[1] / H.T0)) return false;
     std::vector<PolyX> pc(K), pv(K), pd(std::max(H.n_pairs, 1));
     std::memset(pc.data(), 0, pc.size() * sizeof(PolyX));
     std::memset(pv.data(), 0, pv.size() * sizeof(PolyX));
@@ -353,11 +369,11 @@ bool build_transport_fixed(HostMechanism& m) {
     for (int k = 0; k < K; k++) {
         w4[k] = std::sqrt(std::sqrt((long double)m.W[k]));
         W4[k] = (double)std::sqrt((long double)m.W[k]);
-        if (!poly_fix(&cond[(size_t)k * 5], H.T0, X.pw, 1.0, pc[k])) return false;
-        if (!poly_fix(&visc[(size_t)k * 5], H.T0, X.pw, 1.0L / w4[k], pv[k])) return false;
+        if (!poly_fix(&cond[(size_t)k * 5], X.Tn_lo, X.Tn_hi, X.pw, 1.0, pc[k])) return false;
+        if (!poly_fix(&visc[(size_t)k * 5], X.Tn_lo, X.Tn_hi, X.pw, 1.0L / w4[k], pv[k])) return false;
     }
     for (int p = 0; p < H.n_pairs; p++)
-        if (!poly_fix(&diff[(size_t)p * 5], H.T0, X.pw, 1.0, pd[p])) return false;
+        if (!poly_fix(&diff[(size_t)p * 5], X.Tn_lo, X.Tn_hi, X.pw, 1.0, pd[p])) return false;
     // b_kj = a_kj (W_j / W_k)^(1/4) to FP64 rounding (a constant that the reference's builder folds to 0 or 1 is
     // not); |a^2| to the words' position
     double largest = 0.;
@@ -402,6 +418,13 @@ bool build_transport_fixed(HostMechanism& m) {
     X.total_bytes = (int32_t)b.size();
     std::memcpy(b.data() + off_header, &X, sizeof X);
     return true;
+}
+}  // namespace
+
+bool build_transport_fixed(HostMechanism& m) {
+    for (const double* T : kFixTransportT)
+        if (build_transport(m, T[0], T[1])) return true;
+    return false;
 }
 
 }  // namespace cbg

@@ -6,7 +6,8 @@
 // logarithms and divisions and 0.7 k exponents. Here the exponents, exponentials, logarithms, equilibrium
 // constants and third-body sums run on the integer pipe next to it.
 // Cells outside the fixed-point range (T, non-finite or non-positive state) take the FP64 form, with its
-// tables read from global memory.
+// tables read from global memory: 2^19 cells of 53 species above 8,192 K 17.5 ms (5.5 in range, 16.2 in the FP64 kernel,
+// whose tables are in shared memory), in a mixed field up to the sum of both forms; one of them alone 0.94 ms (0.83).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -44,7 +45,7 @@ __device__ __forceinline__ bool cell_setup_x(const RatesXTables& tb, double pres
                                              const double* const* amounts, size_t i, CellX<KMAX>& c) {
     const RatesXHeader& H = *tb.H;
     const int K = H.K, A = H.A;
-    if (!(T >= kFixTmin && T < kFixTmax)) return false;
+    if (!(T >= H.Tmin && T < kFixTmax)) return false;
     // both reciprocals and the products rounded as the reference's: the bulk concentration is a difference of
     // totals, whose last bits it magnifies
     const double md = __drcp_rn(V);
@@ -168,12 +169,25 @@ __device__ __forceinline__ bool reaction_rates_cell_x(const RatesXTables& tb, co
 
 // The FP64 form of one cell, out of line: it is rarely taken.
 template <int KMAX>
-__device__ __noinline__ void rates_cell_f64(const RatesArgs<KMAX>& io, size_t i) {
-    rates_cell<KMAX>(RatesTables(io.f64_tab), io, i);
+__device__ __noinline__ void rates_cell_f64(const uint8_t* f64_tab, const RatesArgs<KMAX>& io, size_t i) {
+    rates_cell<KMAX>(RatesTables(f64_tab), io, i);
 }
 template <int KMAX>
-__device__ __noinline__ void reaction_rates_cell_f64(const ReactionRatesArgs<KMAX>& io, size_t i) {
-    reaction_rates_cell<KMAX>(RatesTables(io.f64_tab), io, i);
+__device__ __noinline__ void reaction_rates_cell_f64(const uint8_t* f64_tab, const ReactionRatesArgs<KMAX>& io, size_t i) {
+    reaction_rates_cell<KMAX>(RatesTables(f64_tab), io, i);
+}
+// The FP64 tables in place of the others in the block's shared memory, or where they are when they do not fit: one thread
+// reads them, one entry after the other (a state of 53 species above 8,192 K 940 us, from global memory 1,330).
+__device__ __forceinline__ const uint8_t* stage_f64(const uint8_t* f64_tab) {
+    const uint32_t bytes = (uint32_t)reinterpret_cast<const RatesHeader*>(f64_tab + kMathBytes)->total_bytes;
+    uint32_t room;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(room));
+    if (bytes > room) return f64_tab;
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < bytes / 16; q += blockDim.x)
+        reinterpret_cast<uint4*>(cb_dsmem)[q] = reinterpret_cast<const uint4*>(f64_tab)[q];
+    __syncthreads();
+    return cb_dsmem;
 }
 
 // The tables into shared memory, or only the functions' tables (the rest is then read through L1).
@@ -200,7 +214,7 @@ __global__ void __launch_bounds__(kRatesXBlock) rates_x_kernel(const uint8_t* __
     for (size_t b = (size_t)blockIdx.x * blockDim.x; b < n; b += (size_t)gridDim.x * blockDim.x) {
         __syncthreads();
         const size_t i = b + threadIdx.x;
-        if (i < n && !rates_cell_x<KMAX>(tb, io, i)) rates_cell_f64<KMAX>(io, i);
+        if (i < n && !rates_cell_x<KMAX>(tb, io, i)) rates_cell_f64<KMAX>(io.f64_tab, io, i);
     }
 }
 
@@ -214,7 +228,7 @@ __global__ void __launch_bounds__(kRatesXBlock) reaction_rates_x_kernel(const ui
     for (size_t b = (size_t)blockIdx.x * blockDim.x; b < n; b += (size_t)gridDim.x * blockDim.x) {
         __syncthreads();
         const size_t i = b + threadIdx.x;
-        if (i < n && !reaction_rates_cell_x<KMAX>(tb, io, i)) reaction_rates_cell_f64<KMAX>(io, i);
+        if (i < n && !reaction_rates_cell_x<KMAX>(tb, io, i)) reaction_rates_cell_f64<KMAX>(io.f64_tab, io, i);
     }
 }
 
@@ -245,7 +259,7 @@ __device__ __forceinline__ bool cell_progress_warp(const RatesXTables& tb, doubl
     constexpr int kStep = 32 * TEAM;
     const RatesXHeader& H = *tb.H;
     const int K = H.K, A = H.A;
-    if (!(T >= kFixTmin && T < kFixTmax)) return false;
+    if (!(T >= H.Tmin && T < kFixTmax)) return false;
     double* C = sh;
     double* cw = sh + K;
     long long* g = reinterpret_cast<long long*>(sh + 2 * K);
@@ -376,15 +390,17 @@ __device__ __forceinline__ bool reaction_rates_cell_warp(const RatesXTables& tb,
 
 // The warp's cells; those that need the FP64 form are put off until there are 32, one per lane.
 template <bool SMEM, int TEAM, class Cell, class F64>
-__device__ __forceinline__ void warp_cells(const uint8_t* gtab, uint32_t tab_bytes, size_t n, int* status, Cell cell, F64 f64) {
+__device__ __forceinline__ void warp_cells(const uint8_t* gtab, uint32_t tab_bytes, const uint8_t* f64_tab, size_t n, int* status,
+                                           Cell cell, F64 f64) {
     __shared__ uint64_t bar;
     if (!stage_x<SMEM>(gtab, tab_bytes, &bar, status)) return;
     const RatesXTables tb(SMEM ? cb_dsmem : gtab);
     const uint32_t tables = SMEM ? tab_bytes : (uint32_t)(kMathBytes + kFixMathBytes);
     if (TEAM > 1) {
-        for (size_t i = blockIdx.x; i < n; i += gridDim.x) {
-            if (!cell(tb, i, reinterpret_cast<double*>(cb_dsmem + tables), (int)threadIdx.x) && threadIdx.x == 0) f64(i);
-            __syncthreads();
+        const size_t i = blockIdx.x;  // the block's only cell (launch_team_kernel)
+        if (i < n && !cell(tb, i, reinterpret_cast<double*>(cb_dsmem + tables), (int)threadIdx.x)) {
+            f64_tab = stage_f64(f64_tab);
+            if (threadIdx.x == 0) f64(f64_tab, i);
         }
         return;
     }
@@ -398,12 +414,12 @@ __device__ __forceinline__ void warp_cells(const uint8_t* gtab, uint32_t tab_byt
         __syncwarp();
         if (lane == put_off) later = i;
         if (++put_off == 32) {
-            f64(later);
+            f64(f64_tab, later);
             __syncwarp();
             put_off = 0;
         }
     }
-    if (lane < put_off) f64(later);
+    if (lane < put_off) f64(f64_tab, later);
 }
 
 template <int KMAX, bool SMEM, int TEAM>
@@ -412,20 +428,20 @@ __global__ void __launch_bounds__(32 * (TEAM > 1 ? TEAM : kRatesWarps)) rates_x_
                                                                       int* status) {
     let_next_start();
     warp_cells<SMEM, TEAM>(
-        gtab, tab_bytes, n, status,
+        gtab, tab_bytes, io.f64_tab, n, status,
         [&](const RatesXTables& tb, size_t i, double* sh, int lane) { return rates_cell_warp<TEAM, KMAX>(tb, io, i, sh, lane); },
-        [&](size_t i) { rates_cell_f64<KMAX>(io, i); });
+        [&](const uint8_t* tab, size_t i) { rates_cell_f64<KMAX>(tab, io, i); });
 }
 template <int KMAX, bool SMEM, int TEAM>
 __global__ void __launch_bounds__(32 * (TEAM > 1 ? TEAM : kRatesWarps))
     reaction_rates_x_warp_kernel(const uint8_t* __restrict__ gtab, uint32_t tab_bytes,
                                  const __grid_constant__ ReactionRatesArgs<KMAX> io, size_t n, int* status) {
     warp_cells<SMEM, TEAM>(
-        gtab, tab_bytes, n, status,
+        gtab, tab_bytes, io.f64_tab, n, status,
         [&](const RatesXTables& tb, size_t i, double* sh, int lane) {
             return reaction_rates_cell_warp<TEAM, KMAX>(tb, io, i, sh, lane);
         },
-        [&](size_t i) { reaction_rates_cell_f64<KMAX>(io, i); });
+        [&](const uint8_t* tab, size_t i) { reaction_rates_cell_f64<KMAX>(tab, io, i); });
 }
 
 namespace {

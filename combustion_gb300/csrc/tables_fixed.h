@@ -21,14 +21,15 @@ struct FixMath {
 constexpr int kFixMathBytes = (int)sizeof(FixMath);
 static_assert(kFixMathBytes % kAlign == 0, "fixed-point tables must keep the blob sections aligned");
 
-// Bounds of the fixed-point form. A cell takes it for T in [kFixTmin, kFixTmax); a mechanism when every
-// constant fits its word over that range (fixed_tables.cpp checks; otherwise the FP64 form runs).
-constexpr double kFixTmin = 200.0, kFixTmax = 8192.0, kFixTmid = 2048.0;
+// Bounds of the fixed-point form. A cell takes it for T in [Tmin, kFixTmax), Tmin the lowest of kFixTmin over which every
+// constant of the mechanism fits its word (fixed_tables.cpp checks; without one the FP64 form runs). The words of 1 / T
+// hold 65 K; large exponents over T may not.
+constexpr double kFixTmin[] = {65.0, 100.0, 200.0}, kFixTmax = 8192.0, kFixTmid = 2048.0;
 constexpr int kYq = 51;    // base-2 logarithms: |y| < 2^12
 constexpr int kLo = 29;    // bits of a low word
 constexpr int kLq = 27;    // log2 T, hi word (log2 T < 13)
 constexpr int kBq = 24;    // its factor, |.| < 64
-constexpr int kRq = 37;    // 1 / T, hi word (1/T <= 1/200)
+constexpr int kRq = 37;    // 1 / T, hi word (1/T <= 1/65)
 constexpr int kEq = 14;    // its factor, |.| < 2^17
 constexpr int kPq = 30;    // (T / 2^p)^i, hi word, p = 11 below 2048 K and 13 above
 constexpr int kGq = 18;    // its factor, |.| < 4096
@@ -114,12 +115,14 @@ struct RatesXHeader {
     int32_t group_end[6];
     int64_t lM3, lcbrt, lC0;  // log2 of the Gibbs exponentials' caps and of P0 / R, Qy
     double l10_04, l10_075;   // 0.4 and 0.75 log2(10)
+    double Tmin;
 };
 
 // ---- transport --------------------------------------------------------------------------------------
 // A fitted polynomial D = P0 + P1 L + .. + P4 L^4 in L = ln(T/T0), over 2^sp so that it lies in (2^-6, 1) over
-// the fixed-point temperature range.
-constexpr int kFixTransportTmin = 200, kFixTransportTmax = 4000;
+// the fixed-point temperature range: the widest of these that its mechanism's polynomials allow and whose L need no larger
+// 2^pw than the narrowest's (at T0 = 1,000 K 136 to 7,380 K, |L| < 2).
+constexpr double kFixTransportT[][2] = {{136.0, 7380.0}, {160.0, 6000.0}, {200.0, 5000.0}, {200.0, 4000.0}};
 constexpr int kLpq = 29;  // (L / 2^pw)^m, hi word
 constexpr int kPpq = 28;  // its coefficient, |.| < 4
 constexpr int kPlo = 30;  // bits of their low words

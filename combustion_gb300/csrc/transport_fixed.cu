@@ -6,7 +6,8 @@
 // cell at 53 species, 64 cycles each). Here the fits, their reciprocals and Wilke's sums are integer sums of three
 // 4-cycle mad.wide per term; the FP64 pipe keeps the mixing sums over reciprocals (2 per pair).
 // Cells outside the range of temperatures or with non-finite amounts take the FP64 form, tables read from global
-// memory.
+// memory: 2^19 cells of 53 species above 7,380 K 20.5 ms (5.7 in range, 20.5 in the FP64 kernel), in a mixed field up to
+// the sum of both forms.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -218,7 +219,6 @@ __global__ void __launch_bounds__(kTransportXBlock<KMAX>) transport_x_kernel(con
     const TransportXTables tb(SMEM ? cb_dsmem : gtab);
     if (io.count) n = min(n, (size_t)*io.count);
     for (size_t b = (size_t)blockIdx.x * blockDim.x; b < n; b += (size_t)gridDim.x * blockDim.x) {
-
         const size_t j = b + threadIdx.x;
         if (j >= n) continue;
         const size_t i = io.index ? (size_t)(io.index[j] & kIndexMask) : j, o = (io.flags & kCompactOut) ? j : i;

@@ -396,3 +396,90 @@ def test_coherent_traces():
             err = float(abs((out[c] - np.sqrt(LD(x[1, c])) * mu) / (np.sqrt(LD(x[1, c])) * mu)))
             print(f"main species {mains[c // 3]}, {x.shape[1] * reps} cells: {err:.2e}")
             assert err <= 2e-15
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+def test_ends_of_the_temperatures(config):
+    """Rates from 60 to 9,000 K and transport from 100 to 9,000 K, across the ends of the fixed-point form's
+    temperatures, in calls of one cell per block, per warp and per thread: against the oracle, one cell having the same
+    bits in each."""
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = util.mechanism(config)
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    scales = synthetic.transport_scales(m)
+    mech.transport_setup(*scales)
+    o.set_transport(*scales, *mech.transport_coefficients())
+    up, T0 = np.nextafter, scales[0]
+    ends = [60.0, up(65.0, 0), 65.0, 80.0, up(100.0, 0), 100.0, 136.0, 150.0, up(200.0, 0), 200.0, 3999.0, 4000.0, 5500.0, 7379.0,
+            7381.0, up(8192.0, 0), 8192.0, 9000.0]
+    ends += [136.0 * (1 - 1e-12), 136.0 * (1 + 1e-12), 7380.0 * (1 - 1e-12), 7380.0 * (1 + 1e-12)]
+    n = 48
+    cells = synthetic.generate_cells(m.K, n, config, seed=53)
+    scale = cells.temperature.copy()
+    cells.temperature[:len(ends)] = ends
+    cells.temperature[len(ends):] = np.geomspace(61.0, 8900.0, n - len(ends))
+    scale /= cells.temperature
+    cells.total_amount *= scale
+    cells.amounts *= scale
+    rin, pin, tin = o.rates_inputs(cells), o.reaction_rates_inputs(cells), o.transport_inputs(cells)
+    hot = np.asarray(cells.temperature) >= 100.0  # (the conductivity polynomials have zeros below)
+    calls = (("rates", rin, m.active() + 2, o.rates(rin, scale=True), hot | True),
+             ("reaction_rates", pin, m.R, o.reaction_rates(pin, scale=True), hot | True),
+             ("transport", tin, m.K + 2, o.transport(tin, scale=True), hot))
+    reps = {"k10": 64, "k53": 400, "k250": 400}[config] * 152 // n + 1
+    for name, x, rows, (ref, sc), cols in calls:
+        first = None
+        for r in (1, 40, reps):
+            t = torch.full((rows, n * r), float("nan"), dtype=torch.float64, device="cuda")
+            getattr(mech, name)(dev(np.tile(np.array(x), (1, r))), t)
+            mech.synchronize()
+            t = t[:, -n:].cpu().numpy()
+            first = t if first is None else first
+            assert np.array_equal(t, first, equal_nan=True), (name, r)
+        e = util.cond_err(first, ref, sc)[:, cols]
+        print(f"{config} {name}: max cond err {np.nanmax(e):.2e} (T = {cells.temperature[cols][np.nanargmax(np.nanmax(e, 0))]:g})")
+        assert np.array_equal(np.isfinite(first[:, cols]), np.isfinite(ref[:, cols]))
+        assert np.nanmax(e) <= util.PLAIN_TOL
+
+
+def test_hot_and_cold_cells_take_no_longer():
+    """Transport of cells at 3,500 to 7,300 K and rates at 70 to 250 K take as long as at ordinary temperatures."""
+    import torch
+    import combustion_gb300 as cb
+    from combustion_gb300 import surrogate as S
+    m = util.mechanism("k53")
+    mech = cb.Mechanism(m)
+    mech.transport_setup(*synthetic.transport_scales(m))
+    n = 1 << 18
+    x = S.generate_cells(mech, n, S.distribution("k53", seed=5))
+    rates = torch.empty((mech.A + 2, n), dtype=torch.float64, device="cuda")
+    transport = torch.empty((mech.K + 2, n), dtype=torch.float64, device="cuda")
+
+    def at(lo, hi):
+        y = x.clone()
+        y[2] = torch.linspace(lo, hi, n, dtype=torch.float64, device="cuda")[torch.randperm(n, device="cuda")]
+        y[4:] *= x[2] / y[2]
+        return y
+
+    def timed(call):
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            call()
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return float(np.median(times))
+
+    inputs = {name: at(*T) for name, T in (("ordinary", (800, 2800)), ("hot", (3500, 7300)), ("cold", (70, 250)))}
+    for call, other in (("transport", "hot"), ("rates", "cold")):
+        t = {}
+        for name in ("ordinary", other):
+            c = inputs[name]
+            given = torch.cat([(c[0] * c[3] / c[2])[None], (c[2] / 1000.0)[None], c[4:]])
+            t[name] = timed((lambda: mech.rates(c, rates)) if call == "rates" else (lambda: mech.transport(given, transport)))
+        print(call, {k: round(v, 2) for k, v in t.items()})
+        assert t[other] < 1.25 * t["ordinary"]
