@@ -94,7 +94,10 @@ __device__ __forceinline__ double exp2_core(long long y) {
     return __longlong_as_double(((long long)(((int)yh >> 19) + 1022) << 52) + (long long)((m + 512) >> 10));
 }
 static __device__ __noinline__ double exp2_slow(double y) { return exp2(y); }
-static __device__ __noinline__ double exp2_slow_fix(long long y) { return exp2((double)y * 0x1p-51); }
+static __device__ __noinline__ double exp2_slow_fix(long long y) {
+    if (y < -(1076ll << kYq)) return 0.0;  // (no FP64 instructions: at low temperatures many)
+    return exp2((double)y * 0x1p-51);
+}
 __device__ __forceinline__ double exp2_fix(long long y) {
     // -1021 <= y < 1023 by the high word
     if ((unsigned)((int)(y >> 32) + (1021 << 19)) >= (2044u << 19)) return exp2_slow_fix(y);
@@ -104,6 +107,7 @@ __device__ __forceinline__ double exp2_fix(long long y) {
 static __device__ __noinline__ double rate_slow(long long y) {
     if (y >= kConstRateMin) return min_pos(kF32Max, __longlong_as_double(y - kConstRate));
     if (y >= (128ll << kYq)) return kF32Max;
+    if (y < -(1076ll << kYq)) return 0.0;
     return min_pos(kF32Max, exp2((double)y * 0x1p-51));
 }
 __device__ __forceinline__ double rate_fix(long long y) {

@@ -445,7 +445,7 @@ def test_ends_of_the_temperatures(config):
 
 
 def test_hot_and_cold_cells_take_no_longer():
-    """Transport of cells at 3,500 to 7,300 K and rates at 70 to 250 K take as long as at ordinary temperatures."""
+    """Transport of cells at 3,500 to 7,300 K and rates at 105 to 250 K take as long as at ordinary temperatures."""
     import torch
     import combustion_gb300 as cb
     from combustion_gb300 import surrogate as S
@@ -474,7 +474,7 @@ def test_hot_and_cold_cells_take_no_longer():
             times.append(a.elapsed_time(b))
         return float(np.median(times))
 
-    inputs = {name: at(*T) for name, T in (("ordinary", (800, 2800)), ("hot", (3500, 7300)), ("cold", (70, 250)))}
+    inputs = {name: at(*T) for name, T in (("ordinary", (800, 2800)), ("hot", (3500, 7300)), ("cold", (105, 250)))}
     for call, other in (("transport", "hot"), ("rates", "cold")):
         t = {}
         for name in ("ordinary", other):
