@@ -41,6 +41,7 @@ EXPORTS = ["cb_mech_create", "cb_mech_validate", "cb_mech_destroy", "cb_mech_que
            "cb_surrogate_evaluate", "cb_reactors_create", "cb_reactors_destroy", "cb_reactors_set_state",
            "cb_reactors_autotune", "cb_reactors_integrate", "cb_reactors_results", "cb_reactors_eval",
            "cb_reactors_eval_noalloc", "cb_yaml_load", "cb_yaml_desc", "cb_yaml_free", "cb_debug_stage_wait_polls",
+           "cb_debug_fixed_math",
            "cb_surrogate_transport_pair"]
 
 
@@ -101,6 +102,7 @@ def lib():
         L.cb_version.restype = C.c_char_p
         L.cb_device_fp64_peak.argtypes = [C.POINTER(C.c_double)]
         L.cb_fp64_math.argtypes = [C.c_int, vp, vp, sz, vp]
+        L.cb_debug_fixed_math.argtypes = [C.c_int, vp, vp, sz, vp]
         L.cb_debug_stage_wait_polls.argtypes = [C.c_int64]
         _lib = L
     return _lib
@@ -321,6 +323,17 @@ def fp64_math(which: str, x):
     x = x.contiguous()
     y = torch.empty_like(x)
     _check(lib().cb_fp64_math(code, x.data_ptr(), y.data_ptr(), x.numel(), torch.cuda.current_stream().cuda_stream))
+    return y
+
+
+def debug_fixed_math(which: str, x):
+    """Test hook: the plain kernels' fixed-point functions on a CUDA float64 tensor (which: "exp2", "log2", "rcp" of 1/32 to
+    1, "fix" to a multiple of 2^-51 and back)."""
+    import torch
+    code = {"exp2": 0, "log2": 1, "rcp": 2, "fix": 3}[which]
+    x = x.contiguous()
+    y = torch.empty_like(x)
+    _check(lib().cb_debug_fixed_math(code, x.data_ptr(), y.data_ptr(), x.numel(), torch.cuda.current_stream().cuda_stream))
     return y
 
 

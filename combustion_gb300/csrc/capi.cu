@@ -15,6 +15,7 @@
 #include "launch.cuh"
 #include "mechanism.hpp"
 #include "tables.h"
+#include "tables_fixed.h"
 
 struct cb_mech {
     cbg::HostMechanism host;
@@ -719,6 +720,21 @@ int cb_fp64_math(int which, const double* x, double* y, size_t n, void* stream) 
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cudaFree(d);
     return e == cudaSuccess ? CB_OK : cuda_fail(e, "math check");
+}
+
+int cb_debug_fixed_math(int which, const double* x, double* y, size_t n, void* stream) {
+    if (which < 0 || which > 3 || (n && (!x || !y))) return fail(CB_ERR_INVALID, "bad arguments");
+    const cbg::MathTables t = cbg::make_math_tables();
+    const cbg::FixMath f = cbg::make_fix_math();
+    uint8_t* d = nullptr;
+    CB_CUDA(cudaMalloc(&d, sizeof t + sizeof f));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    cudaError_t e = cudaMemcpyAsync(d, &t, sizeof t, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d + sizeof t, &f, sizeof f, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cbg::launch_fixed_math_check(d, which, x, y, n, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d);
+    return e == cudaSuccess ? CB_OK : cuda_fail(e, "fixed-point math check");
 }
 
 int cb_debug_stage_wait_polls(int64_t polls) {

@@ -154,8 +154,8 @@ int max_table_smem() {
     return v;
 }
 
-CB_DISPATCH(launch_rates, rates_kernel, RatesArgs, kBlock, kMathBytes, true)
-CB_DISPATCH(launch_reaction_rates, reaction_rates_kernel, ReactionRatesArgs, kBlock, kMathBytes, true)
+CB_DISPATCH(launch_rates, rates_kernel, RatesArgs, kBlock, kMathBytes, false)
+CB_DISPATCH(launch_reaction_rates, reaction_rates_kernel, ReactionRatesArgs, kBlock, kMathBytes, false)
 
 CB_WAVE(wave_rates, rates_kernel, kBlock, kMathBytes)
 CB_WAVE(wave_reaction_rates, reaction_rates_kernel, kBlock, kMathBytes)

@@ -144,6 +144,8 @@ cudaError_t launch_rates(int kmax, const uint8_t* tab, uint32_t tab_bytes, const
                          cudaStream_t st, int* status);
 cudaError_t launch_reaction_rates(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n,
                                   cudaStream_t st, int* status);
+// The fixed-point functions on doubles: `tab` [MathTables][FixMath].
+cudaError_t launch_fixed_math_check(const uint8_t* tab, int which, const double* x, double* y, size_t n, cudaStream_t st);
 // The fixed-point forms (kernels_fixed.cu); `args` carries the FP64 tables as well.
 // warp_bytes: a warp's scratch in the form of one cell per warp (rates_warp_bytes).
 cudaError_t launch_rates_x(int kmax, const uint8_t* tab, uint32_t tab_bytes, const void* args, size_t n, size_t warp_bytes,

@@ -464,7 +464,7 @@ cudaError_t launch_rates_xk(const uint8_t* tab, uint32_t tab_bytes, const RatesA
         return launch_warp_kernel<kRatesWarps>(rates_x_warp_kernel<KMAX, true, 1>, rates_x_warp_kernel<KMAX, false, 1>, tab, tab_bytes, io, n,
                                                kMathBytes + kFixMathBytes, warp_bytes, st, status);
     return launch_table_kernel<kRatesXBlock>(rates_x_kernel<KMAX, true>, rates_x_kernel<KMAX, false>, tab, tab_bytes, io, n,
-                                             kMathBytes + kFixMathBytes, true, st, status);
+                                             kMathBytes + kFixMathBytes, false, st, status);
 }
 template <int KMAX>
 cudaError_t launch_reaction_rates_xk(const uint8_t* tab, uint32_t tab_bytes, const ReactionRatesArgs<KMAX>& io, size_t n,
@@ -478,7 +478,7 @@ cudaError_t launch_reaction_rates_xk(const uint8_t* tab, uint32_t tab_bytes, con
         return launch_warp_kernel<kRatesWarps>(reaction_rates_x_warp_kernel<KMAX, true, 1>, reaction_rates_x_warp_kernel<KMAX, false, 1>, tab,
                                                tab_bytes, io, n, kMathBytes + kFixMathBytes, warp_bytes, st, status);
     return launch_table_kernel<kRatesXBlock>(reaction_rates_x_kernel<KMAX, true>, reaction_rates_x_kernel<KMAX, false>, tab,
-                                             tab_bytes, io, n, kMathBytes + kFixMathBytes, true, st, status);
+                                             tab_bytes, io, n, kMathBytes + kFixMathBytes, false, st, status);
 }
 }  // namespace
 
@@ -509,6 +509,23 @@ cudaError_t launch_reaction_rates_x(int kmax, const uint8_t* tab, uint32_t tab_b
 }
 CB_WAVE(wave_rates_x, rates_x_kernel, kRatesXBlock, kMathBytes + kFixMathBytes)
 CB_WAVE(wave_reaction_rates_x, reaction_rates_x_kernel, kRatesXBlock, kMathBytes + kFixMathBytes)
+
+// Test hook: the fixed-point functions one by one (cb_debug_fixed_math).
+__global__ void fixed_math_check_kernel(const uint8_t* tab, int which, const double* x, double* y, size_t n) {
+    stage_x<false>(tab, 0, nullptr, nullptr);
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const double v = x[i];
+        y[i] = which == 0   ? exp2_dbl(v)
+               : which == 1 ? log2_dbl(v)
+               : which == 2 ? rcp_fixed(dbl_to_fix(v, kDq), 1022 + 63 - 56)
+                            : fix_to_dbl(dbl_to_fix(v, kYq), kYq);
+    }
+}
+cudaError_t launch_fixed_math_check(const uint8_t* tab, int which, const double* x, double* y, size_t n, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    fixed_math_check_kernel<<<(unsigned)(n < 256 * 4096 ? (n + 255) / 256 : 4096), 256, kMathBytes + kFixMathBytes, st>>>(tab, which, x, y, n);
+    return cudaGetLastError();
+}
 
 cudaError_t set_stage_wait_polls_x(long long polls) { return cudaMemcpyToSymbol(g_stage_wait_polls, &polls, sizeof polls); }
 

@@ -50,6 +50,8 @@ bool build_transport_fixed(HostMechanism& m);
 
 struct MathTables;
 MathTables make_math_tables();
+struct FixMath;
+FixMath make_fix_math();
 
 // Transport physics of one species or pair at temperature T (SI), used by the fits.
 double species_viscosity(const HostMechanism& m, int k, double T);

@@ -76,8 +76,8 @@ __device__ __forceinline__ double small_int_to_double(int v) {
 // (kMaxSide slots, absent ones skipped) are issued together before the first multiply, so that the reads
 // overlap instead of each waiting for the previous factor. Otherwise (a warp's cell in shared memory,
 // one reaction per lane) one load per factor, fewer registers. The multiplication order is the same.
-template <bool BATCH, class Index>
-__device__ __forceinline__ double conc_product(const double* C, const Index* ks, const int8_t* ns, int n) {
+template <bool BATCH>
+__device__ __forceinline__ double conc_product(const double* C, const uint16_t* ks, const int8_t* ns, int n) {
     if constexpr (BATCH) {
         double v[kMaxSide];
 #pragma unroll

@@ -23,7 +23,7 @@ static_assert(kFixMathBytes % kAlign == 0, "fixed-point tables must keep the blo
 
 // Bounds of the fixed-point form. A cell takes it for T in [Tmin, kFixTmax), Tmin the lowest of kFixTmin over which every
 // constant of the mechanism fits its word (fixed_tables.cpp checks; without one the FP64 form runs). The words of 1 / T
-// hold 65 K; large exponents over T may not.
+// hold 65 K; large exponents over T may not (100 K at 53 and 250 species of the generator).
 constexpr double kFixTmin[] = {65.0, 100.0, 200.0}, kFixTmax = 8192.0, kFixTmid = 2048.0;
 constexpr int kYq = 51;    // base-2 logarithms: |y| < 2^12
 constexpr int kLo = 29;    // bits of a low word

@@ -178,6 +178,11 @@ int cb_synchronize(cb_mech* mech, void* stream);
  * synchronising call reports CB_ERR_DEVICE (and clears the status). For tests of that error path. */
 int cb_debug_stage_wait_polls(int64_t polls);
 
+/* Test hook, no reference counterpart: the plain kernels' fixed-point functions on n device doubles, synchronously on
+ * `stream`. which: 0 2^x (x to a multiple of 2^-51), 1 log2 (to a multiple of 2^-51), 2 the reciprocal of x in (1/32, 1)
+ * (to a multiple of 2^-60), 3 x as a multiple of 2^-51 (|x| < 2^9). */
+int cb_debug_fixed_math(int which, const double* x, double* y, size_t n, void* stream);
+
 /* ---- Seeded synthetic cells on the device ----------------------------------------------------------
  * No reference counterpart (the reference reads states from Cantera or its own reactor). T uniform on
  * [T_min, T_max] K, P log-uniform on [P_min, P_max] atm (fixed when equal), V = 1 m^3, mole fractions
