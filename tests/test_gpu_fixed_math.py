@@ -75,3 +75,41 @@ def test_conversions():
     assert (err <= LD(2) ** -52).all()  # (a value of 2 or more has no bits below, and is itself)
     assert (y.astype(LD) * LD(2) ** 51 == np.rint(y.astype(LD) * LD(2) ** 51)).all()
     assert np.array_equal(y[np.abs(x) >= 2], x[np.abs(x) >= 2])
+
+
+@pytest.mark.parametrize("config, n", [("k10", 2048), ("k53", 1024), ("k250", 128)])
+def test_errors_against_long_double(config, n):
+    """Rates and transport of seeded cells against long double: the condition-scaled rms error of every output group is
+    below that of the same program in FP64 (the oracle)."""
+    import torch
+    import combustion_gb300 as cb
+    import numpy_restatement
+    import oracle
+    import util
+    from combustion_gb300 import synthetic
+    m = util.mechanism(config)
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    scales = synthetic.transport_scales(m)
+    mech.transport_setup(*scales)
+    coefs = mech.transport_coefficients()
+    o.set_transport(*scales, *coefs)
+    cells = synthetic.generate_cells(m.K, n, config, seed=77)
+    rin, tin = o.rates_inputs(cells), o.transport_inputs(cells)
+    wide = [x.astype(LD) for x in rin]
+    wide[1] = 1 / wide[0]
+    dev = lambda x: torch.tensor(np.array(x), dtype=torch.float64, device="cuda")  # noqa: E731
+    rates = torch.empty((mech.A + 2, n), dtype=torch.float64, device="cuda")
+    transport = torch.empty((mech.K + 2, n), dtype=torch.float64, device="cuda")
+    mech.rates(dev(rin), rates)
+    mech.transport(dev(tin), transport)
+    mech.synchronize()
+    cases = (("rates", rates, o.rates(rin, scale=True), util.RATES_GROUPS,
+              numpy_restatement.rates(m, wide[0], wide[1], wide[2], wide[3], wide[4:])),
+             ("transport", transport, o.transport(tin, scale=True), util.TRANSPORT_GROUPS,
+              numpy_restatement.transport(m, scales, coefs, tin[0].astype(LD), tin[1].astype(LD), [x.astype(LD) for x in tin[2:]])))
+    for name, out, (fp64, scale), groups, ref in cases:
+        ours, theirs = (np.abs((x.astype(LD) - ref) / scale).astype(float) for x in (out.cpu().numpy(), fp64))
+        for group, rows in groups:
+            a, b = (np.sqrt((e[rows] ** 2).mean()) for e in (ours, theirs))
+            print(f"{config} {name} {group}: rms {a:.2e} (FP64 {b:.2e}), max {ours[rows].max():.2e} ({theirs[rows].max():.2e})")
+            assert a <= b
