@@ -397,10 +397,14 @@ __device__ __forceinline__ void warp_cells(const uint8_t* gtab, uint32_t tab_byt
     const RatesXTables tb(SMEM ? cb_dsmem : gtab);
     const uint32_t tables = SMEM ? tab_bytes : (uint32_t)(kMathBytes + kFixMathBytes);
     if (TEAM > 1) {
-        const size_t i = blockIdx.x;  // the block's only cell (launch_team_kernel)
-        if (i < n && !cell(tb, i, reinterpret_cast<double*>(cb_dsmem + tables), (int)threadIdx.x)) {
-            f64_tab = stage_f64(f64_tab);
-            if (threadIdx.x == 0) f64(f64_tab, i);
+        // The block's only cell (launch_team_kernel), so that the FP64 tables may take the place of the others. In a loop
+        // all the same: without one the compiler takes 80 registers for 128 and spills (250 species 107 -> 110 us).
+        for (size_t i = blockIdx.x; i < n; i += gridDim.x) {
+            if (!cell(tb, i, reinterpret_cast<double*>(cb_dsmem + tables), (int)threadIdx.x)) {
+                const uint8_t* staged = gridDim.x < n ? f64_tab : stage_f64(f64_tab);
+                if (threadIdx.x == 0) f64(staged, i);
+            }
+            __syncthreads();
         }
         return;
     }
