@@ -483,3 +483,36 @@ def test_hot_and_cold_cells_take_no_longer():
             t[name] = timed((lambda: mech.rates(c, rates)) if call == "rates" else (lambda: mech.transport(given, transport)))
         print(call, {k: round(v, 2) for k, v in t.items()})
         assert t[other] < 1.25 * t["ordinary"]
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+def test_transport_states(config):
+    """Transport of non-finite, zero and negative states: NaN where the oracle has NaN, infinity where it has infinity, the
+    rest at the plain bar, in calls of every form."""
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = util.mechanism(config)
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    scales = synthetic.transport_scales(m)
+    mech.transport_setup(*scales)
+    o.set_transport(*scales, *mech.transport_coefficients())
+    n, K = 48, m.K
+    x = np.array(o.transport_inputs(synthetic.generate_cells(K, n, config, seed=59)))  # sum n, T/T0, n_0 ..
+    states = [(row, v) for row in (0, 1, 2, 2 + K // 2, K) for v in (np.nan, np.inf, -np.inf)]
+    states += [(1, -1.0), (1, 0.0), (0, 0.0), (2, -1e-3 * x[0, 0]), (2 + K // 2, 1e200), (0, 1e200)]
+    for c, (row, v) in enumerate(states):
+        x[row, c] = v
+    with np.errstate(all="ignore"):
+        ref, sc = o.transport(list(x), scale=True)
+    for r in (1, 40, {"k10": 64, "k53": 192, "k250": 520}[config] * 152 // n + 1):
+        t = torch.full((K + 2, n * r), 7.0, dtype=torch.float64, device="cuda")
+        mech.transport(dev(np.tile(x, (1, r))), t)
+        mech.synchronize()
+        t = t[:, -n:].cpu().numpy()
+        for c in range(n):
+            what = f"{n * r} cells, state {states[c] if c < len(states) else 'ordinary'}"
+            assert np.array_equal(np.isnan(t[:, c]), np.isnan(ref[:, c])), what
+            assert np.array_equal(np.isinf(t[:, c]), np.isinf(ref[:, c])), what
+        both = np.isfinite(ref) & np.isfinite(sc)
+        assert (util.cond_err(t, ref, sc)[both] <= util.PLAIN_TOL).all()
