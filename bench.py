@@ -685,11 +685,12 @@ def run_ours(args):
     # the same kernel with every division, exponential, logarithm and square root counted as one flop
     unit_flops = work["flops"] + sum(work[k] for k in SLOT_COST)
     achieved_unit = unit_flops * n / (ms * 1e-3) / 1e12
-    traffic = fp64_left = None
+    traffic = fp64_left = int_mad = None
     tpath = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     if os.path.exists(tpath):
         ncu = json.load(open(tpath)).get(dom, {})
         traffic = ncu["dram_bytes_per_cell"] * n if "dram_bytes_per_cell" in ncu else None
+        int_mad = ncu.get("int_mad_pipe_active")  # ncu: the pipe of mad.wide, IMAD and FP32 multiplies
         # what the FP64 pipe still executes (ncu count) over its measured issue rate
         fp64_left = ncu["fp64_inst_per_cell"] * n / (ms * 1e-3) / (peak * 1e12 / 2) if "fp64_inst_per_cell" in ncu else None
 
@@ -797,9 +798,10 @@ def run_ours(args):
                          "flop_model": "reference program ops (+-x min max = 1) plus exp/log/div/sqrt at "
                                        "2 x {10,12,4,4} FMA slots",
                          "note": "most of this arithmetic runs in 64-bit fixed point on the integer pipe, beside the FP64 "
-                                 "pipe: frac, of the FP64 rate alone, is above 1; fp64_pipe_frac counts the FP64 "
+                                 "pipe: frac, of the FP64 rate alone, is above 1 and bounds nothing; fp64_pipe_frac counts the FP64 "
                                  "instructions that are left",
                          "fp64_pipe_frac": fp64_left,
+                         "int_mad_pipe_frac": int_mad,
                          "unit_weight": {"flops_per_cell": unit_flops, "achieved": achieved_unit,
                                          "frac": achieved_unit / peak,
                                          "flop_model": "every op, exp, log, div and sqrt = 1 flop"}},
