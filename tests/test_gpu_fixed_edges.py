@@ -516,3 +516,38 @@ def test_transport_states(config):
             assert np.array_equal(np.isinf(t[:, c]), np.isinf(ref[:, c])), what
         both = np.isfinite(ref) & np.isfinite(sc)
         assert (util.cond_err(t, ref, sc)[both] <= util.PLAIN_TOL).all()
+
+
+@pytest.mark.parametrize("config", ["k10", "k53", "k250"])
+@pytest.mark.parametrize("T0", [250.0, 298.15, 3000.0])
+def test_other_reference_temperatures(config, T0):
+    """Transport with polynomials in ln(T / T0) of other reference temperatures, whose fixed-point range and words differ:
+    from 140 to 7,300 K at the plain bar, one cell having the same bits in calls of every form."""
+    import torch
+    import combustion_gb300 as cb
+    import oracle
+    m = util.mechanism(config)
+    mech, o = cb.Mechanism(m), oracle.Oracle(m)
+    scales = synthetic.transport_scales(m, T0=T0)
+    mech.transport_setup(*scales)
+    o.set_transport(*scales, *mech.transport_coefficients())
+    n = 48
+    cells = synthetic.generate_cells(m.K, n, config, seed=61)
+    scale = cells.temperature.copy()
+    cells.temperature[:] = np.geomspace(140.0, 7300.0, n)
+    scale /= cells.temperature
+    cells.total_amount *= scale
+    cells.amounts *= scale
+    x = np.array(o.transport_inputs(cells))
+    ref, sc = o.transport(list(x), scale=True)
+    first = None
+    for r in (1, 40, {"k10": 64, "k53": 192, "k250": 520}[config] * 152 // n + 1):
+        t = torch.full((m.K + 2, n * r), float("nan"), dtype=torch.float64, device="cuda")
+        mech.transport(dev(np.tile(x, (1, r))), t)
+        mech.synchronize()
+        t = t[:, -n:].cpu().numpy()
+        first = t if first is None else first
+        assert np.array_equal(t, first)
+    e = util.cond_err(first, ref, sc)
+    print(f"{config}, T0 = {T0}: max cond err {e.max():.2e} (T = {cells.temperature[e.max(0).argmax()]:.0f})")
+    assert e.max() <= util.PLAIN_TOL
